@@ -20,6 +20,14 @@ constexpr float kDefaultCondMax = 1000.0f;  // |C| inverted in FP32 up to this i
 constexpr float kDefaultShift = 0.999f;     // inverse-iteration shift, in units of min(1, rho)
 constexpr float kDefaultShiftBackoff = 0.97f;   // second shift when M - sigma I is not definite
 
+// decision boundary of the Anderson-Darling test (nmap.cu) for one stack
+// depth and threshold
+struct NmapAdPlan {
+    int n = 0, mode = 0;
+    double prob = 0.0, star = 0.0;
+    float lo = 0.f, hi = 0.f, w[2 * FPL_MAX_BANDS] = {};
+};
+
 struct fpl_ctx {
     int device = 0;
     int num_sms = 0;
@@ -44,6 +52,7 @@ struct fpl_ctx {
     // nmap: sorted amplitudes, validity and staging of host jobs
     void *d_nm = nullptr;
     size_t cap_nm = 0;
+    NmapAdPlan nmap_ad;
     // host-memory runs: outputs of the FP64-settled pixels, packed for the
     // copy back (device) and received (host)
     void *d_pack = nullptr;

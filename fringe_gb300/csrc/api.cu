@@ -309,7 +309,8 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
         const int rows_per_chunk = (int)std::max<long long>(1, chunk_px_max / P.cols);
         const long long chunk_px = (long long)std::min(rows_per_chunk, r1 - r0) * P.cols;
         if ((rc = grow(ctx, &ctx->d_cbuf, &ctx->cap_cbuf, sizeof(float) * (size_t)rec * chunk_px))) return rc;
-        if ((rc = grow(ctx, &ctx->d_cinfo, &ctx->cap_cinfo, sizeof(int) * (size_t)chunk_px))) return rc;
+        // tile information and rest list
+        if ((rc = grow(ctx, &ctx->d_cinfo, &ctx->cap_cinfo, 2 * sizeof(int) * (size_t)chunk_px))) return rc;
         for (int ra = r0; ra < r1; ra += rows_per_chunk) {
             const int rb = std::min(r1, ra + rows_per_chunk);
             KParams Q = P;
@@ -317,6 +318,7 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
             Q.npix = (long long)(rb - ra) * P.cols;
             Q.cbuf = static_cast<float2 *>(ctx->d_cbuf);
             Q.cinfo = static_cast<int *>(ctx->d_cinfo);
+            Q.rest = Q.cinfo + chunk_px;
             Q.cbase = Q.pix_begin;
             Q.cstride = rec;
             FPL_CUDA(ctx, timed(FPL_KTAG_GRAM, [&] { return fpl::launch_gram_box(Q, ctx->num_sms, st); }));

@@ -288,7 +288,7 @@ struct fpl_batch {
     fpl::BatchEntry *d_m64 = nullptr;     // mixed: every piece, by padded depth (FP64 settle)
     int m64_first[3] = {0, 0, 0}, m64_count[3] = {0, 0, 0};
     int mixed_warps[3] = {0, 0, 0};  // warps per CTA of the mixed solve launches (0: the most that fit)
-    void *d_rec = nullptr;           // mixed: Gamma records and tile infos of one wave
+    void *d_rec = nullptr;           // mixed: Gamma records, tile infos and rest lists of one wave
     std::vector<BatchClass> classes;
     fpl::BatchEntry *d_table = nullptr;
     void *d_scratch = nullptr;       // per-job counters, work counters, FP64 lists
@@ -461,7 +461,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 b->waves.resize(w + 1);
             }
             const size_t rec_bytes = (sizeof(float) * rec_max + 255) & ~size_t(255);
-            if (cudaMalloc(&b->d_rec, rec_bytes + sizeof(int) * std::max<size_t>(info_max, 1)) != cudaSuccess) {
+            if (cudaMalloc(&b->d_rec, rec_bytes + 2 * sizeof(int) * std::max<size_t>(info_max, 1)) != cudaSuccess) {
                 fpl_batch_destroy(b);
                 return FPL_ERR_NOMEM;
             }
@@ -477,6 +477,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 set_counters(P, nf + i);
                 P.cbuf = reinterpret_cast<float2 *>(recs + rec_off[i]);
                 P.cinfo = infos + info_off[i];
+                P.rest = P.cinfo + info_max;
                 P.cbase = P.pix_begin;
                 P.cstride = fpl::gram_box_record(jb.nbands);
                 b->job_of_entry.push_back(pc.job);

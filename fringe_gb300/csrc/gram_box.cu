@@ -272,6 +272,11 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
         }
         st.blk_dp = dp;
     }
+    // the chunk's rest list starts empty (the solve kernels run after this one)
+    if (t == 0 && tid == 0) {
+        P.fb_count[1] = 0;
+        P.fb_count[13] = 0;
+    }
     // ---- per-pixel SHP masks over the union samples ----------------
     for (int e = tid; e < BX_M * W; e += BX_THREADS) umask[e] = 0;
     for (int e = tid; e < W; e += BX_THREADS) tbad[e] = 0;

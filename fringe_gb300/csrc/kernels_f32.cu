@@ -25,11 +25,13 @@ cudaError_t launch_fp32(const KParams &P, int num_sms, cudaStream_t st)
 
 cudaError_t launch_solve(const KParams &P, int num_sms, cudaStream_t st)
 {
-    switch (pick_np(P.nb)) {
-    case 16: return launch_solve_t<16, true>(P, num_sms, st);
-    case 32: return launch_solve_t<32, true>(P, num_sms, st);
-    case 64: return launch_solve_t<64, true>(P, num_sms, st);
-    }
+    // the smallest grid that holds the dates: its blocks per lane (3, 6, 10; 12,
+    // 20) set the work of a step and the registers, so the warps per SM
+    if (P.nb <= 16) return launch_solve_t<16, 2>(P, num_sms, st);
+    if (P.nb <= 24) return launch_solve_t<16, 3>(P, num_sms, st);
+    if (P.nb <= 32) return launch_solve_t<16, 4>(P, num_sms, st);
+    if (P.nb <= 48) return launch_solve_t<32, 3>(P, num_sms, st);
+    if (P.nb <= 64) return launch_solve_t<32, 4>(P, num_sms, st);
     return cudaErrorInvalidValue;
 }
 
@@ -38,9 +40,9 @@ cudaError_t prepare_mixed_batch(int np)
     cudaError_t e = prepare_gram_batch();
     if (e != cudaSuccess) return e;
     switch (np) {
-    case 16: return configure_solve_batch<16, true>();
-    case 32: return configure_solve_batch<32, true>();
-    case 64: return configure_solve_batch<64, true>();
+    case 16: return configure_solve_batch<16, 2>();
+    case 32: return configure_solve_batch<16, 4>();
+    case 64: return configure_solve_batch<32, 4>();
     }
     return cudaErrorInvalidValue;
 }
@@ -48,9 +50,9 @@ cudaError_t prepare_mixed_batch(int np)
 int solve_max_warps(int np)
 {
     switch (np) {
-    case 16: return std::min(20, int((224 * 1024) / SolveWarp<16, true>::bytes));
-    case 32: return std::min(32, int((224 * 1024) / Lay<float, 32>::bytes_noc));
-    case 64: return std::min(8, int((224 * 1024) / Lay<float, 64>::bytes_noc));
+    case 16: return solve_warps<16, 2>();
+    case 32: return solve_warps<16, 4>();
+    case 64: return solve_warps<32, 4>();
     }
     return 1;
 }
@@ -60,9 +62,9 @@ cudaError_t launch_solve_batch(int np, const BatchEntry *ents, int nent, long lo
 {
     if (nent <= 0 || total <= 0) return cudaSuccess;
     switch (np) {
-    case 16: return launch_solve_batch_t<16, true>(ents, nent, total, num_sms, st, warps);
-    case 32: return launch_solve_batch_t<32, true>(ents, nent, total, num_sms, st, warps);
-    case 64: return launch_solve_batch_t<64, true>(ents, nent, total, num_sms, st, warps);
+    case 16: return launch_solve_batch_t<16, 2>(ents, nent, total, num_sms, st, warps);
+    case 32: return launch_solve_batch_t<16, 4>(ents, nent, total, num_sms, st, warps);
+    case 64: return launch_solve_batch_t<32, 4>(ents, nent, total, num_sms, st, warps);
     }
     return cudaErrorInvalidValue;
 }

@@ -13,7 +13,7 @@
 #include <type_traits>
 #include "kernels.h"
 #include "pixel.cuh"
-#include "solve_pair.cuh"
+#include "solve_tile.cuh"
 
 namespace fpl {
 
@@ -51,151 +51,78 @@ __global__ void k_pixels(KParams P)
     if constexpr (CInTmem<T, NP>::value || CRowsTmemF<T, NP>::value) tmem_free_cta(tbase, warp, (uint32_t)tcols);
 }
 
-// mixed form, second half: eigen-solves from the tensor-core Gamma records.
-// TM: each warp keeps its pixel's coherence rows in tensor memory (2*NP
-// columns of its 32-lane quadrant) instead of shared memory, so a CTA holds
-// about twice as many warps; the kernel issues no MMA.  At padded order 16 a
-// warp solves two pixels, one per 16-lane half (solve_pair.cuh): two slabs
-// per warp, the rows of both in the warp's 2*NP columns.
-template <int NP, bool TM> struct PairSolve {
-    static constexpr bool value = TM && NP == 16;
-};
-template <int NP, bool TM> struct SolveWarp {
-    static constexpr bool pair = PairSolve<NP, TM>::value;
-    static constexpr size_t bytes =
-        pair ? 2 * Lay<float, NP>::bytes_noc : (TM ? Lay<float, NP>::bytes_noc : Lay<float, NP>::bytes);
-    // warp work items: pixel pairs or pixels
-    static __host__ __device__ long long items(long long px) { return pair ? (px + 1) / 2 : px; }
-};
+// ---- eigen-solves from the Gamma records ---------------------------------
+// MLE pixels (and phase_link's) are solved in registers by k_solve, G lanes per
+// pixel (solve_tile.cuh); those it hands back, and the pixels of the other
+// methods, by k_rest, a warp per pixel with its coherence rows in tensor memory
+// (pixel_solve).  Neither issues an MMA.
+__device__ __forceinline__ bool tile_solved(const KParams &P) { return P.method == M_MLE || P.semantics == SEM_PL; }
 
-// pixel pp of the launch P: record -> coherence rows -> solve and outputs
-template <int NP, typename CP>
-__device__ __forceinline__ void solve_pixel(const KParams &P, long long pp, unsigned char *sm, int lane, const CP &cp,
-                                            C2<float> *A)
-{
-    if constexpr (NP <= 32) {
-        const int npix = pixel_load_gamma<NP, false>(P, pp, sm, lane, A);
-        float cfro = -1.f;
-        if (npix >= 0 && rows_coherence<NP>(P, pp, A, sm, cp, lane, &cfro))
-            pixel_solve<float, NP>(P, pp, sm, lane, npix, cp, cfro);
-    } else if constexpr (std::is_same<CP, CRowsTmem<NP>>::value) {
-        // two rows per lane: normalise in the slab, then copy the rows over
-        const int npix = pixel_load_gamma<NP>(P, pp, sm, lane, A);
-        if (npix >= 0) {
-            rows_from_smem<NP>(cp, A, lane);
-            pixel_solve<float, NP>(P, pp, sm, lane, npix, cp);
-        }
-    } else {
-        const int npix = pixel_load_gamma<NP>(P, pp, sm, lane, A);
-        if (npix >= 0) pixel_solve<float, NP>(P, pp, sm, lane, npix, cp);
-    }
-}
+template <int G, int NL> struct SolveShape {
+    using M = Tile<G, NL>;
+    static constexpr int PX = 32 / G;                       // pixels per warp
+    static constexpr size_t bytes = PX * M::bytes;          // shared memory per warp
+    static constexpr int cols = 8 * M::NB;                  // tensor-memory columns per warp
+    // warps per CTA (one CTA per SM) that the registers allow: NB 8-register blocks and the working set
+    static constexpr int max_warps = M::NB >= 20 ? 8 : (M::NB >= 12 ? 12 : (M::NB >= 10 ? 16 : (M::NB >= 6 ? 20 : 24)));
+    static __host__ __device__ long long items(long long px) { return (px + PX - 1) / PX; }
+};
 
 // Solve kernel over a pixel source: SRC(q) gives (launch, pixel) of item q
-// of [0, total).  TM: each warp keeps its pixel's coherence rows in tensor
-// memory (2*NP columns of its 32-lane quadrant) instead of shared memory,
-// so a CTA holds about twice as many warps; the kernel issues no MMA.
-template <int NP, bool TM, typename SRC>
+// of [0, total).
+template <int G, int NL, typename SRC>
 __device__ __forceinline__ void solve_loop(long long total, const SRC &src)
 {
+    using SH = SolveShape<G, NL>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr size_t per_warp = SolveWarp<NP, TM>::bytes;
-    unsigned char *sm = smem + (size_t)warp * per_warp;
     const long long gw = (long long)blockIdx.x * warps + warp;
     const long long nw = (long long)gridDim.x * warps;
-    if constexpr (TM) {
-        __shared__ uint32_t tslot;
-        const int tcols = tmem_cols_for(warps, NP);
-        if (warp == 0) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                         :: "r"((uint32_t)__cvta_generic_to_shared(&tslot)), "r"(tcols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    __shared__ uint32_t tslot;
+    uint32_t tcols = 32;
+    while ((int)tcols < (warps + 3) / 4 * SH::cols) tcols <<= 1;
+    const uint32_t tbase = tmem_alloc_cta(&tslot, warp, tcols);
+    const uint32_t taddr = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * (uint32_t)SH::cols;
+    const int g = lane & (G - 1), h = lane / G;
+    const TileLane L{g, g >> 2, g & 3,
+                     (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)(warp * SH::bytes + h * Tile<G, NL>::bytes)};
+    const long long items = SH::items(total);
+    for (long long k = gw; k < items; k += nw) {
+        const long long q0 = SH::PX * k;
+        const bool in = q0 + h < total;
+        long long pp;
+        const KParams &P = src(in ? q0 + h : q0, pp);
+        const bool valid = in && tile_solved(P);
+        if (k + nw < items && q0 + SH::PX * nw + h < total) {
+            long long pn;
+            const KParams &Pn = src(q0 + SH::PX * nw + h, pn);
+            tile_prefetch<G>(Pn, pn, g);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tbase = tslot;
-        const CRowsTmem<NP> cp{tbase + ((uint32_t)(32 * (warp & 3)) << 16) +
-                               (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp};
-        C2<float> *A = reinterpret_cast<C2<float> *>(sm + Lay<float, NP>::wm);
-        if constexpr (PairSolve<NP, TM>::value) {
-            // pixels 2k and 2k+1 on halves 0 and 1; MLE pixels with evd
-            // semantics are solved by the halves together, any other pixel by
-            // the whole warp on its half's slab
-            const int h = lane >> 4;
-            const PairHalf H{lane & 15, h, h ? 0xffff0000u : 0x0000ffffu};
-            const long long npair = (total + 1) >> 1;
-            for (long long k = gw; k < npair; k += nw) {
-                const long long q0 = 2 * k;
-                const bool valid = q0 + h < total;
-                long long pp;
-                const KParams &P = src(valid ? q0 + h : q0, pp);
-                const bool paired = valid && P.method == M_MLE && P.semantics != SEM_PL;
-                if (k + nw < npair && q0 + 2 * nw + h < total) {
-                    long long pn;
-                    const KParams &Pn = src(q0 + 2 * nw + h, pn);
-                    pair_prefetch(Pn, pn, H.hl);
-                }
-                pair_mle(P, pp, sm, cp, H, paired);
-                for (int hh = 0; hh < 2; ++hh) {
-                    if (!__shfl_sync(0xffffffffu, (int)(valid && !paired), 16 * hh)) continue;
-                    long long ph;
-                    const KParams &Ph = src(q0 + hh, ph);
-                    unsigned char *smh = sm + hh * Lay<float, NP>::bytes_noc;
-                    solve_pixel<NP>(Ph, ph, smh, lane, cp, reinterpret_cast<C2<float> *>(smh + Lay<float, NP>::wm));
-                }
-            }
-        } else {
-        for (long long q = gw; q < total; q += nw) {
-            long long pp;
-            const KParams &P = src(q, pp);
-            if (q + nw < total) {
-                long long pn;
-                const KParams &Pn = src(q + nw, pn);
-                prefetch_record(Pn, pn, lane);
-            }
-            solve_pixel<NP>(P, pp, sm, lane, cp, A);
-        }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (warp == 0) {
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(tcols) : "memory");
-        }
-    } else {
-        C2<float> *Cm = reinterpret_cast<C2<float> *>(sm + Lay<float, NP>::cm);
-        const CRowsSmem<float, NP> cp{Cm, lane};
-        for (long long q = gw; q < total; q += nw) {
-            long long pp;
-            const KParams &P = src(q, pp);
-            if (q + nw < total) {
-                long long pn;
-                const KParams &Pn = src(q + nw, pn);
-                prefetch_record(Pn, pn, lane);
-            }
-            solve_pixel<NP>(P, pp, sm, lane, cp, Cm);
-        }
+        if (!__any_sync(0xffffffffu, valid)) continue;
+        const int state = tile_mle<G, NL>(P, pp, L, taddr, valid);
+        if (valid && state == TILE_GENERAL && g == 0) rest_put(P, pp);
+        __syncwarp();
     }
+    tmem_free_cta(tbase, warp, tcols);
 }
 
-template <int NP, bool TM>
-__global__ void __launch_bounds__((TM && NP <= 32) ? 640 : (TM ? 256 : 512), 1) k_solve(KParams P)
+template <int G, int NL>
+__global__ void __launch_bounds__(32 * SolveShape<G, NL>::max_warps, 1) k_solve(const __grid_constant__ KParams P)
 {
-    solve_loop<NP, TM>(P.npix, [&](long long q, long long &pp) -> const KParams & {
-        pp = P.pix_begin + q;
-        return P;
+    const KParams *p = &P;
+    solve_loop<G, NL>(P.npix, [p](long long q, long long &pp) -> const KParams & {
+        pp = p->pix_begin + q;
+        return *p;
     });
 }
 
-// the mixed form over many launches of one padded depth
-template <int NP, bool TM>
-__global__ void __launch_bounds__((TM && NP <= 32) ? 640 : (TM ? 256 : 512), 1) k_solve_batch(const BatchEntry *__restrict__ ents, int nent,
-                                                                  long long total)
+// over many launches of one padded depth
+template <int G, int NL>
+__global__ void __launch_bounds__(32 * SolveShape<G, NL>::max_warps, 1) k_solve_batch(const BatchEntry *__restrict__ ents,
+                                                                                     int nent, long long total)
 {
-    solve_loop<NP, TM>(total, [&](long long q, long long &pp) -> const KParams & {
+    solve_loop<G, NL>(total, [&](long long q, long long &pp) -> const KParams & {
         int lo = 0, hi = nent - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -206,38 +133,74 @@ __global__ void __launch_bounds__((TM && NP <= 32) ? 640 : (TM ? 256 : 512), 1) 
     });
 }
 
-// CTA shape of the solve kernels: warps per CTA by shared memory (and
-// registers), one CTA per SM in the tensor-memory form
-template <int NP, bool TM, typename K>
-static cudaError_t solve_shape(K kern, int *warps_out, int *per_sm_out, size_t *smem_out, int warps_req = 0)
+// the pixels of entry P that k_solve left: every one, or those of its rest list
+template <int NP>
+__device__ __forceinline__ void rest_loop(const KParams &P, unsigned char *sm, int lane, const CRowsTmem<NP> &cp)
 {
-    const size_t per_warp = SolveWarp<NP, TM>::bytes;
-    const size_t budget = 224 * 1024;
-    // tensor memory: 512 columns per lane quadrant, CRowsTmem<NP>::kColsPerWarp per warp
-    const int cap = TM ? int(4 * (512 / CRowsTmem<NP>::kColsPerWarp)) : 16;
-    int warps = int(budget / per_warp);
-    if (warps > cap) warps = cap;
-    if (warps_req > 0 && warps > warps_req) warps = warps_req;
-    if (warps < 1) warps = 1;
-    int per_sm = 0;
-    size_t smem = per_warp * warps;
-    for (;;) {
-        smem = per_warp * warps;
-        // one CTA per SM in the tensor-memory form: at least half the shared
-        // memory, so a second CTA never waits on a tensor-memory allocation
-        if (TM && smem < budget / 2 + 1024) smem = budget / 2 + 1024;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem);
-        if (e != cudaSuccess) return e;
-        if (per_sm >= 1 || warps == 1) break;
-        --warps;
+    C2<float> *A = reinterpret_cast<C2<float> *>(sm + Lay<float, NP>::wm);
+    const bool listed = tile_solved(P);
+    const long long cnt = listed ? *((volatile int *)(P.fb_count + 1)) : P.npix;
+    for (long long q = rest_next(P, lane); q < cnt; q = rest_next(P, lane)) {
+        const long long pp = P.cbase + (listed ? (long long)P.rest[q] : q);
+        if constexpr (NP <= 32) {
+            const int npix = pixel_load_gamma<NP, false>(P, pp, sm, lane, A);
+            float cfro = -1.f;
+            if (npix >= 0 && rows_coherence<NP>(P, pp, A, sm, cp, lane, &cfro))
+                pixel_solve<float, NP>(P, pp, sm, lane, npix, cp, cfro);
+        } else {
+            // two rows per lane: normalise in the slab, then copy the rows over
+            const int npix = pixel_load_gamma<NP>(P, pp, sm, lane, A);
+            if (npix >= 0) {
+                rows_from_smem<NP>(cp, A, lane);
+                pixel_solve<float, NP>(P, pp, sm, lane, npix, cp);
+            }
+        }
+        __syncwarp();
     }
-    if (per_sm < 1) per_sm = 1;
-    if (TM) per_sm = 1;
-    *warps_out = warps;
-    *per_sm_out = per_sm;
-    *smem_out = smem;
-    return cudaSuccess;
 }
+
+template <int NP> constexpr int rest_max_warps() { return NP <= 32 ? 20 : 5; }
+
+template <int NP>
+__global__ void __launch_bounds__(32 * rest_max_warps<NP>(), 1) k_rest(const __grid_constant__ KParams P)
+{
+    if (tile_solved(P) && *((volatile int *)(P.fb_count + 1)) == 0) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ uint32_t tslot;
+    const int tcols = tmem_cols_for(blockDim.x >> 5, NP);
+    const uint32_t tbase = tmem_alloc_cta(&tslot, warp, tcols);
+    const CRowsTmem<NP> cp{tbase + ((uint32_t)(32 * (warp & 3)) << 16) +
+                           (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp};
+    rest_loop<NP>(P, smem + (size_t)warp * Lay<float, NP>::bytes_noc, lane, cp);
+    tmem_free_cta(tbase, warp, tcols);
+}
+
+template <int NP>
+__global__ void __launch_bounds__(32 * rest_max_warps<NP>(), 1) k_rest_batch(const BatchEntry *__restrict__ ents, int nent)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ uint32_t tslot;
+    const int tcols = tmem_cols_for(blockDim.x >> 5, NP);
+    const uint32_t tbase = tmem_alloc_cta(&tslot, warp, tcols);
+    const CRowsTmem<NP> cp{tbase + ((uint32_t)(32 * (warp & 3)) << 16) +
+                           (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp};
+    for (int e = 0; e < nent; ++e) rest_loop<NP>(ents[e].P, smem + (size_t)warp * Lay<float, NP>::bytes_noc, lane, cp);
+    tmem_free_cta(tbase, warp, tcols);
+}
+
+// One CTA per SM for the kernels above: at least half the shared memory, so
+// that a second CTA never waits on a tensor-memory allocation
+constexpr size_t kSolveSmem = 224 * 1024;
+template <int G, int NL> static int solve_warps()
+{
+    using SH = SolveShape<G, NL>;
+    const int by_smem = int(kSolveSmem / SH::bytes), by_tmem = 4 * (512 / SH::cols);
+    const int w = by_smem < by_tmem ? by_smem : by_tmem;
+    return w < SH::max_warps ? w : SH::max_warps;
+}
+static size_t solve_smem(size_t per_warp, int warps) { return cmax(per_warp * warps, kSolveSmem / 2 + 1024); }
 
 template <typename K>
 static cudaError_t solve_configure(K kern, bool *configured)
@@ -245,7 +208,7 @@ static cudaError_t solve_configure(K kern, bool *configured)
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && configured[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
@@ -253,45 +216,71 @@ static cudaError_t solve_configure(K kern, bool *configured)
     return cudaSuccess;
 }
 
-template <int NP, bool TM>
-static cudaError_t launch_solve_t(const KParams &P, int num_sms, cudaStream_t st)
+// Grid and warps per CTA for `items` warp items: a full CTA per SM, or, when
+// there are fewer items than warps, as many SMs with fewer warps each
+static long long solve_grid(long long items, int num_sms, int *warps)
+{
+    const long long per = (items + num_sms - 1) / num_sms;
+    if (per < *warps) *warps = per < 1 ? 1 : (int)per;
+    const long long need = (items + *warps - 1) / *warps;
+    return need < num_sms ? (need > 0 ? need : 1) : num_sms;
+}
+
+template <int NP>
+static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
 {
     static bool configured[64] = {false};
-    cudaError_t e = solve_configure(k_solve<NP, TM>, configured);
+    cudaError_t e = solve_configure(k_rest<NP>, configured);
     if (e != cudaSuccess) return e;
-    int warps = 0, per_sm = 0;
-    size_t smem = 0;
-    if ((e = solve_shape<NP, TM>(k_solve<NP, TM>, &warps, &per_sm, &smem)) != cudaSuccess) return e;
-    long long blocks = (long long)num_sms * per_sm;
-    long long need = (SolveWarp<NP, TM>::items(P.npix) + warps - 1) / warps;
-    if (need < blocks) blocks = need > 0 ? need : 1;
-    k_solve<NP, TM><<<(unsigned)blocks, warps * 32, smem, st>>>(P);
+    int warps = rest_max_warps<NP>();
+    const long long blocks = solve_grid(P.npix, num_sms, &warps);
+    k_rest<NP><<<(unsigned)blocks, warps * 32, solve_smem(Lay<float, NP>::bytes_noc, warps), st>>>(P);
     return cudaGetLastError();
 }
 
-// attributes of k_solve_batch<NP, TM>, set once per device
-template <int NP, bool TM>
+template <int G, int NL>
+static cudaError_t launch_solve_t(const KParams &P, int num_sms, cudaStream_t st)
+{
+    constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
+    if (P.method == M_MLE || P.semantics == SEM_PL) {
+        static bool configured[64] = {false};
+        cudaError_t e = solve_configure(k_solve<G, NL>, configured);
+        if (e != cudaSuccess) return e;
+        int warps = solve_warps<G, NL>();
+        const long long blocks = solve_grid(SolveShape<G, NL>::items(P.npix), num_sms, &warps);
+        k_solve<G, NL><<<(unsigned)blocks, warps * 32, solve_smem(SolveShape<G, NL>::bytes, warps), st>>>(P);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return launch_rest_t<NP>(P, num_sms, st);
+}
+
+// attributes of the batch kernels, set once per device
+template <int G, int NL>
 static cudaError_t configure_solve_batch()
 {
-    static bool configured[64] = {false};
-    return solve_configure(k_solve_batch<NP, TM>, configured);
+    constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
+    static bool configured[64] = {false}, rest[64] = {false};
+    const cudaError_t e = solve_configure(k_solve_batch<G, NL>, configured);
+    return e != cudaSuccess ? e : solve_configure(k_rest_batch<NP>, rest);
 }
 
 // warps_req > 0: at most that many warps per CTA (the batch autotuner's
-// candidates); 0: as many as shared memory and registers allow
-template <int NP, bool TM>
+// candidates); 0: as many as fit
+template <int G, int NL>
 static cudaError_t launch_solve_batch_t(const BatchEntry *ents, int nent, long long total, int num_sms,
                                        cudaStream_t st, int warps_req)
 {
-    cudaError_t e = configure_solve_batch<NP, TM>();
+    constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
+    cudaError_t e = configure_solve_batch<G, NL>();
     if (e != cudaSuccess) return e;
-    int warps = 0, per_sm = 0;
-    size_t smem = 0;
-    if ((e = solve_shape<NP, TM>(k_solve_batch<NP, TM>, &warps, &per_sm, &smem, warps_req)) != cudaSuccess) return e;
-    long long blocks = (long long)num_sms * per_sm;
-    long long need = (SolveWarp<NP, TM>::items(total) + warps - 1) / warps;
-    if (need < blocks) blocks = need > 0 ? need : 1;
-    k_solve_batch<NP, TM><<<(unsigned)blocks, warps * 32, smem, st>>>(ents, nent, total);
+    int warps = solve_warps<G, NL>();
+    if (warps_req > 0 && warps > warps_req) warps = warps_req;
+    const long long blocks = solve_grid(SolveShape<G, NL>::items(total), num_sms, &warps);
+    k_solve_batch<G, NL><<<(unsigned)blocks, warps * 32, solve_smem(SolveShape<G, NL>::bytes, warps), st>>>(ents, nent, total);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    int rw = rest_max_warps<NP>();
+    const long long rb = solve_grid(total, num_sms, &rw);
+    k_rest_batch<NP><<<(unsigned)rb, rw * 32, solve_smem(Lay<float, NP>::bytes_noc, rw), st>>>(ents, nent);
     return cudaGetLastError();
 }
 

@@ -46,7 +46,8 @@ struct KParams {
     float cond_max;                     // largest inf-norm condition of |C| inverted in FP32
     float shift, shift_backoff;         // inverse-iteration shifts, in units of min(1, rho)
     int *fb_count;                      // FP64 work list (scratch): the 64-byte counter block of the
-                                        // run: +0 list length, +16 err, +32 slow, +48 work cursor
+                                        // run: +0 list length, +16 err, +32 slow, +48 work cursor;
+                                        // of the chunk: +4 rest list length, +52 its work cursor
     long long *fb_list;
     int fb_cap;
     unsigned *err;                      // error flags (scratch)
@@ -56,6 +57,7 @@ struct KParams {
     int *cinfo;                         // [pixel - cbase]: SHP count, or CI_* below
     long long cbase;                    // first pixel of the buffers
     int cstride;                        // floats per record
+    int *rest;                          // pixels (- cbase) that the register solve hands to pixel_solve
 };
 
 enum { CI_CENTRE = -1, CI_FEW = -2, CI_DEFER = -3 };
@@ -1391,6 +1393,19 @@ __device__ __forceinline__ void put_code(const KParams &P, long long pp, int lan
         P.tcorr[pp] = float(code);
         if (P.status) P.status[pp] = code;
     }
+}
+
+// the rest list of a chunk: appended to by the register solve, drawn from by
+// warps of k_rest
+__device__ __forceinline__ void rest_put(const KParams &P, long long pp)
+{
+    P.rest[atomicAdd(P.fb_count + 1, 1)] = int(pp - P.cbase);
+}
+__device__ __forceinline__ int rest_next(const KParams &P, int lane)
+{
+    int q = 0;
+    if (lane == 0) q = atomicAdd(P.fb_count + 13, 1);
+    return __shfl_sync(0xffffffffu, q, 0);
 }
 
 // Gather, Gamma and coherence (evd.cpp:514-582).  Returns the SHP count

@@ -91,7 +91,7 @@ struct fpl_server {
     int max_pieces = 256;
     fpl::BatchEntry *d_table = nullptr, *h_table = nullptr;
     fpl::BoxSeg *d_segs = nullptr, *h_segs = nullptr;   // Gamma segments of a wave's mixed pieces
-    void *d_rec = nullptr;                              // their Gamma records and tile infos
+    void *d_rec = nullptr;                              // their Gamma records, tile infos and rest lists
     size_t rec_cap = 0;
     void *d_wave = nullptr;
     size_t wave_bytes = 0;
@@ -218,13 +218,14 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
             infos += px;
         }
     const size_t rec_bytes = (sizeof(float) * rec_floats + 255) & ~size_t(255);
-    if (rec_floats && rec_bytes + sizeof(int) * infos > s->rec_cap) {
+    const size_t rec_need = rec_bytes + 2 * sizeof(int) * infos;
+    if (rec_floats && rec_need > s->rec_cap) {
         // the previous wave has finished (its event was waited for)
         if (s->d_rec) cudaFree(s->d_rec);
         s->d_rec = nullptr;
         s->rec_cap = 0;
-        if (cudaMalloc(&s->d_rec, rec_bytes + sizeof(int) * infos) != cudaSuccess) return false;
-        s->rec_cap = rec_bytes + sizeof(int) * infos;
+        if (cudaMalloc(&s->d_rec, rec_need) != cudaSuccess) return false;
+        s->rec_cap = rec_need;
     }
     float *recs = static_cast<float *>(s->d_rec);
     int *rinfo = reinterpret_cast<int *>(static_cast<char *>(s->d_rec) + rec_bytes);
@@ -246,6 +247,7 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         if (pc.mixed) {
             P.cbuf = reinterpret_cast<float2 *>(recs + roff);
             P.cinfo = rinfo + ioff;
+            P.rest = P.cinfo + infos;
             P.cbase = P.pix_begin;
             P.cstride = fpl::gram_box_record(P.nb);
             roff += P.npix * P.cstride;

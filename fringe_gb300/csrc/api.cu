@@ -2,10 +2,11 @@
 //
 // fpl_run replaces the OpenMP pixel loop of evd_process
 // (src/evd/evd.cpp:512-788; src/phase_link/phase_link.cpp:479-666) for a
-// scene held in memory.  The FP32 kernel handles every pixel; pixels whose
+// scene held in memory: the coherence sums on the tensor cores (gram_box.cu),
+// the eigen-solves from their records, chunk by chunk of rows; pixels whose
 // discrete decisions fall inside the FP32 rounding band are queued on the
-// device and settled by the FP64 kernel launched right behind it on the same
-// stream.  No host round trip separates the two passes.
+// device and settled by the FP64 kernel launched right behind on the same
+// stream.  No host round trip separates the passes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -298,24 +299,38 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
         return cudaSuccess;
     };
     if (ctx->profile && count_run) ctx->prof_runs++;
-    const bool mixed = job->precision == FPL_PREC_MIXED && fpl::gram_box_supported(P.nb, P.ny, P.nx);
+    bool tiled = fpl::gram_box_supported(P.nb, P.ny, P.nx);
+    int rows_per_chunk = 0;
+    long long chunk_px = 0;
+    const int rec = fpl::gram_box_record(P.nb);
+    if ((stages & ENQ_KERNELS) && tiled) {
+        // tensor-core Gamma records, then eigen-solves, chunk by chunk of rows
+        // so the records stay within a bounded buffer.  A record's value does not
+        // depend on the chunk, so the FP32 form, which needs no such buffer by itself,
+        // takes smaller chunks where the device memory is short.
+        rows_per_chunk = (int)std::max<long long>(1, std::max<long long>(P.cols, (1ll << 20)) / P.cols);
+        rows_per_chunk = std::min(rows_per_chunk, r1 - r0);
+        for (;;) {
+            chunk_px = (long long)rows_per_chunk * P.cols;
+            rc = grow(ctx, &ctx->d_cbuf, &ctx->cap_cbuf, sizeof(float) * (size_t)rec * chunk_px);
+            // tile information and rest list
+            if (!rc) rc = grow(ctx, &ctx->d_cinfo, &ctx->cap_cinfo, 2 * sizeof(int) * (size_t)chunk_px);
+            if (!rc) break;
+            if (rc != FPL_ERR_NOMEM || job->precision == FPL_PREC_MIXED) return rc;
+            cudaGetLastError();
+            if (rows_per_chunk == 1) { tiled = false; break; }
+            rows_per_chunk = (rows_per_chunk + 1) / 2;
+        }
+    }
     if (!(stages & ENQ_KERNELS)) {
         // settle only
-    } else if (mixed) {
-        // tensor-core Gamma records, then eigen-solves, chunk by chunk of
-        // rows so the records stay within a bounded buffer
-        const int rec = fpl::gram_box_record(P.nb);
-        const long long chunk_px_max = std::max<long long>(P.cols, (1ll << 20));
-        const int rows_per_chunk = (int)std::max<long long>(1, chunk_px_max / P.cols);
-        const long long chunk_px = (long long)std::min(rows_per_chunk, r1 - r0) * P.cols;
-        if ((rc = grow(ctx, &ctx->d_cbuf, &ctx->cap_cbuf, sizeof(float) * (size_t)rec * chunk_px))) return rc;
-        // tile information and rest list
-        if ((rc = grow(ctx, &ctx->d_cinfo, &ctx->cap_cinfo, 2 * sizeof(int) * (size_t)chunk_px))) return rc;
+    } else if (tiled) {
         for (int ra = r0; ra < r1; ra += rows_per_chunk) {
             const int rb = std::min(r1, ra + rows_per_chunk);
             KParams Q = P;
             Q.pix_begin = (long long)ra * P.cols;
             Q.npix = (long long)(rb - ra) * P.cols;
+            Q.parts = job->precision == FPL_PREC_MIXED ? 2 : 3;
             Q.cbuf = static_cast<float2 *>(ctx->d_cbuf);
             Q.cinfo = static_cast<int *>(ctx->d_cinfo);
             Q.rest = Q.cinfo + chunk_px;

@@ -1,26 +1,22 @@
-// batch.cu -- many phase-linking jobs in one persistent launch.
+// batch.cu -- many phase-linking jobs in one launch sequence.
 //
 // A batch holds device-memory jobs of different scene sizes, stack depths
-// (ministacks of different N), windows and methods.  Jobs whose padded depth
-// NP matches share one persistent kernel: warps take pixels from a global
-// counter over the concatenated pixel ranges of the jobs (dynamic scheduling
-// balances tiles of uneven size and uneven SHP counts), look up the pixel's
-// job and run the same per-pixel code as fpl_run.  A second persistent
-// kernel settles, in FP64, the pixels every job queued.  The whole sequence
-// (counter resets and the kernels of every depth class) can be captured once
-// into a CUDA graph and replayed.
-//
-// Jobs in the mixed-precision form (fpl_job::precision = FPL_PREC_MIXED) are
-// cut into row pieces and packed into waves of at most 2^20 pixels; a wave
-// is one persistent tensor-core Gamma launch over the tiles of all its
-// pieces and one persistent solve launch over all
-// its pixels (per padded depth), the Gamma records staying in a buffer
-// sized for one wave.  Their FP64 settle runs with the FP32 jobs' at the end.
+// (ministacks of different N), windows and methods.  Jobs are cut into row
+// pieces and packed into waves of at most 2^20 pixels; a wave is one persistent
+// tensor-core Gamma launch over the tiles of all its pieces (of both forms, two
+// or three bf16 parts per product) and, per padded depth, one persistent solve
+// launch over all its pixels for each kind of method, the Gamma records staying in a buffer
+// sized for one wave.  Jobs whose window the Gamma kernel does not take run the
+// plain FP32 kernel, one persistent launch per padded depth: warps take pixels
+// from a global counter over the concatenated pixel ranges of the jobs.  A last
+// persistent kernel settles, in FP64, the pixels every job queued.  The whole
+// sequence (counter resets and all kernels) can be captured once into a CUDA
+// graph and replayed.
 //
 // An optional autotuner times the candidate CTA shapes (warps per CTA) of
-// each depth class -- the FP32 batch launches and the mixed form's solve
-// launches -- on the batch itself and keeps the fastest per (form, NP,
-// window taps, mean SHP count) key in the context.
+// each depth class -- the plain FP32 launches and the solve launches -- on the
+// batch itself and keeps the fastest per (kind of launch, NP, window taps,
+// mean SHP count) key in the context.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -254,6 +250,7 @@ void fill_params(KParams &P, const fpl_job &jb, int r0, int r1, float amb, float
     P.cond_max = cond_max;
     P.shift = kDefaultShift;
     P.shift_backoff = kDefaultShiftBackoff;
+    P.parts = jb.precision == FPL_PREC_MIXED ? 2 : 3;
 }
 
 }  // namespace fpl
@@ -276,6 +273,7 @@ struct MixedWave {
     size_t seg_smem = 0;
     int ent_first[3] = {0, 0, 0}, ent_count[3] = {0, 0, 0};
     long long ent_total[3] = {0, 0, 0};
+    int ent_kinds[3] = {0, 0, 0};
 };
 
 struct fpl_batch {
@@ -309,7 +307,7 @@ int batch_enqueue(fpl_batch *b, cudaStream_t st)
     fpl_ctx *ctx = b->ctx;
     if (cudaMemsetAsync(b->d_scratch, 0, b->counter_bytes, st) != cudaSuccess) return FPL_ERR_CUDA;
     unsigned long long *work = reinterpret_cast<unsigned long long *>(
-        static_cast<char *>(b->d_scratch) + kJobCounterBytes * b->njobs);
+        static_cast<char *>(b->d_scratch) + kJobCounterBytes * b->nent);
     for (size_t c = 0; c < b->classes.size(); ++c) {
         const BatchClass &k = b->classes[c];
         if (fpl::launch_batch(k.np, b->d_table + k.first, k.count, k.total, work + c, k.warps, ctx->num_sms, st) !=
@@ -323,7 +321,7 @@ int batch_enqueue(fpl_batch *b, cudaStream_t st)
             return FPL_ERR_CUDA;
         for (int c = 0; c < 3; ++c)
             if (w.ent_count[c] && fpl::launch_solve_batch(kNP[c], b->d_ments + w.ent_first[c], w.ent_count[c],
-                                                          w.ent_total[c], ctx->num_sms, st,
+                                                          w.ent_total[c], w.ent_kinds[c], ctx->num_sms, st,
                                                           b->mixed_warps[c]) != cudaSuccess)
                 return FPL_ERR_CUDA;
     }
@@ -374,22 +372,30 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
         fpl_batch *b = new fpl_batch();
         b->ctx = ctx;
         b->njobs = njobs;
-        auto is_mixed = [&](const fpl_job &jb) {
-            return jb.precision == FPL_PREC_MIXED && fpl::gram_box_supported(jb.nbands, jb.half_window_y, jb.half_window_x);
+        auto is_tiled = [&](const fpl_job &jb) {
+            return fpl::gram_box_supported(jb.nbands, jb.half_window_y, jb.half_window_x);
         };
-        // FP32 jobs, grouped by padded depth
+        // jobs whose windows the Gamma kernel does not take (plain FP32 kernel), grouped by padded depth
         std::vector<int> order;
         for (int j = 0; j < njobs; ++j)
-            if (!is_mixed(jobs[j])) order.push_back(j);
+            if (!is_tiled(jobs[j])) order.push_back(j);
         std::stable_sort(order.begin(), order.end(),
                          [&](int a, int c) { return fpl::pick_np(jobs[a].nbands) < fpl::pick_np(jobs[c].nbands); });
         const int nf = (int)order.size();
-        // mixed jobs: row pieces of at most kWavePx pixels, packed into waves
+        // the others: row pieces of at most kWavePx pixels, packed into waves
         struct Piece { int job, ra, rb; long long px; };
-        const long long kWavePx = 1ll << 20;
+        // smaller waves where the device memory is short of their records
+        long long kWavePx = 1ll << 20;
+        {
+            size_t free_b = 0, total_b = 0, rec_px = 0;
+            for (int j = 0; j < njobs; ++j)
+                if (is_tiled(jobs[j])) rec_px = std::max(rec_px, 4 * (size_t)fpl::gram_box_record(jobs[j].nbands));
+            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
+                while (kWavePx > 65536 && (size_t)kWavePx * rec_px > free_b / 2) kWavePx /= 2;
+        }
         std::vector<Piece> pieces;
         for (int j = 0; j < njobs; ++j) {
-            if (!is_mixed(jobs[j])) continue;
+            if (!is_tiled(jobs[j])) continue;
             const fpl_job &jb = jobs[j];
             const int r0 = jb.row_begin, r1 = jb.row_end <= 0 ? jb.rows : jb.row_end;
             const int step = (int)std::max<long long>(1, kWavePx / jb.cols);
@@ -494,7 +500,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                     sg.P = pp[i];
                     sg.tile_offset = mw.seg_tiles;
                     mw.seg_tiles += fpl::gram_box_tiles(pp[i]);
-                    mw.seg_smem = std::max(mw.seg_smem, fpl::gram_box_smem(pp[i].nb, pp[i].ny, pp[i].nx));
+                    mw.seg_smem = std::max(mw.seg_smem, fpl::gram_box_smem(pp[i]));
                     segs.push_back(sg);
                 }
                 mw.seg_count = (int)segs.size() - mw.seg_first;
@@ -507,6 +513,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                         en.P = pp[i];
                         en.px_offset = mw.ent_total[c];
                         mw.ent_total[c] += pp[i].npix;
+                        mw.ent_kinds[c] |= fpl::solve_kind(pp[i]);
                         ments.push_back(en);
                     }
                     mw.ent_count[c] = (int)ments.size() - mw.ent_first[c];

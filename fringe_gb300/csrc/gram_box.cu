@@ -1,7 +1,7 @@
 // gram_box.cu -- coherence matrices on the 5th-generation tensor cores, one
 // tile of 128 pixels per GEMM.
 //
-// Mixed-precision form of the SHP gather + Gamma accumulation
+// The SHP gather + Gamma accumulation
 // (src/evd/evd.cpp:516-564, src/phase_link/phase_link.cpp:482-522).  For a
 // pixel p the reference sums x_q x_q^H over its SHPs q.  Written for a tile
 // of pixels at once this is a masked box filter of the per-sample outer
@@ -12,9 +12,15 @@
 //   A = the 0/1 SHP mask (exact in bf16), rows = the 128 pixels of an
 //       8 x 16 pixel tile, columns = the (8+Wy-1) x (16+Wx-1) union samples;
 //   B = the outer-product entries Re / Im x_qi conj(x_qj), formed in FP32
-//       (the reference's complex<float> products) and split into bf16
-//       hi + lo parts (16 significant bits), so D = A B_hi + A B_lo is
-//       accumulated in FP32 in tensor memory.
+//       (the reference's complex<float> products) and split into bf16 parts,
+//       so D = A B_1 + A B_2 (+ A B_3) is accumulated in FP32 in tensor memory:
+//       two parts (16 significant bits) in the mixed form, three in the FP32
+//       form, which hold all 24 bits of the product.  The error of the FP32
+//       form's results against 64 bits is that of the plain FP32 kernel or
+//       less (STBAS, N = 48: phases 2.9e-7 rad RMS from the oracle, plain kernel
+//       2.8e-7; EVD 9.3e-7 against 1.0e-6), and at 1024^2, N = 30, 11 x 21 its Gamma
+//       takes 6.7 ms (two parts: 4.6) of a 22.2 ms call; the plain kernel, 20 of
+//       whose 32 lanes hold sums, took 52 of 54 ms.
 // Each outer product is formed once per tile instead of once for every pixel
 // that uses it.  One thread issues tcgen05.mma (M = 128 pixels, N <= 256
 // Gamma entries, K = 16 samples) into one of two tensor-memory accumulators;
@@ -52,7 +58,8 @@ constexpr int BX_THREADS = 512;                    // 16 warps: the operand buil
 constexpr int BX_TR = 8, BX_TC = 16, BX_M = 128;   // pixel tile (MMA M)
 constexpr int BX_NCOL = 256;                       // Gamma columns per accumulator (MMA N)
 // samples per chunk (MMA K of one stage): 32, so that two accumulators (512
-// Gamma columns per pass) fit beside two operand stages and two sample buffers
+// Gamma columns per pass with two parts, 352 with three) fit beside two
+// operand stages and two sample buffers
 constexpr int BX_KC = 32;
 constexpr int BX_MAXK = 2048;                      // union samples per tile
 constexpr int BX_MAXW = BX_MAXK / 32;              // union mask words per pixel
@@ -62,26 +69,30 @@ constexpr int CI_SKIP = -100;                      // pixel outside this launch'
 constexpr unsigned ERR_TC_TIMEOUT = 2u;
 constexpr long long BX_SPIN_LIMIT = 1ll << 26;     // ~ seconds of polling
 
-template <int KC> struct BoxLay {
-    // tensor-memory accumulators of BX_NCOL columns each: with 32-sample
-    // chunks two fit beside two operand stages, so a pass covers 512 Gamma
-    // columns and a chunk's samples and mask are loaded and built once for
-    // both
+// shared memory of a CTA; NS: bf16 parts of a product.  Barriers, tables and
+// sample buffers come first, at the same place for both NS.
+template <int KC, int NS> struct BoxLay {
+    // tensor-memory accumulators of BX_NCOL columns each: a pass covers PCOL
+    // Gamma columns, and a chunk's samples and mask are loaded and built once for
+    // all of them
     static constexpr int NACC = (KC == 32) ? 2 : 1;
-    static constexpr int PCOL = NACC * BX_NCOL;               // Gamma columns per pass
+    static constexpr int PCOL = NS == 3 ? 352 : NACC * BX_NCOL;
+    static constexpr int TCOL = NACC * BX_NCOL;              // tensor-memory columns held
     static constexpr int SBO = KC * 16 + 16;                 // bytes between 8-row groups
     static constexpr int A_BYTES = (BX_M / 8) * SBO;
-    static constexpr int B_BYTES = (PCOL / 8) * SBO;         // one of hi / lo
-    static constexpr int STAGE = A_BYTES + 2 * B_BYTES;
+    static constexpr int B_BYTES = (PCOL / 8) * SBO;         // one part
+    static constexpr int STAGE = A_BYTES + NS * B_BYTES;
     static constexpr int MAXPAIR = 32;                       // date pairs: 64 dates
     static constexpr int XRS = KC * 16 + 16;                 // bytes per date-pair row of X
     static constexpr int X_BYTES = MAXPAIR * XRS;            // one of two sample buffers
-    static constexpr size_t OFF_X = 2 * (size_t)STAGE;
-    static constexpr size_t OFF_MISC = OFF_X + 2 * (size_t)X_BYTES;
+    static constexpr size_t OFF_MISC = 0;
     static constexpr size_t OFF_LUT = OFF_MISC + BX_MISC;          // 256 x 8 bf16 mask patterns
-    static constexpr size_t OFF_U = OFF_LUT + 256 * 16;
+    static constexpr size_t OFF_X = OFF_LUT + 256 * 16;
+    static constexpr size_t OFF_ST = OFF_X + 2 * (size_t)X_BYTES;  // two operand stages
+    static constexpr size_t OFF_U = OFF_ST + 2 * (size_t)STAGE;
     static constexpr size_t MAX_SMEM = OFF_U + (size_t)BX_M * BX_MAXW * 4;
     static_assert(MAX_SMEM <= 227 * 1024, "shared memory of one CTA");
+    static_assert(OFF_ST % 16 == 0 && STAGE % 16 == 0 && PCOL % 16 == 0, "operand alignment");
 };
 
 // union samples of a tile: (8 + 2 ny) rows of (16 + 2 nx) samples, packed
@@ -179,21 +190,26 @@ __device__ __forceinline__ bool split_range(float v)
     return v == 0.f || (a >= 8.8817842e-16f && a <= 1.1258999e15f);
 }
 
-// 8 values of one Gamma column into bf16 hi and lo rows (16 bytes each)
-__device__ __forceinline__ void store_split(unsigned char *dh, unsigned char *dl, const float *v)
+// 8 values of one Gamma column into NS bf16 rows (16 bytes each, pstride
+// apart): each part rounds what the parts before it left (exact differences)
+template <int NS>
+__device__ __forceinline__ void store_split(unsigned char *dst, uint32_t pstride, const float *v)
 {
-    uint32_t h[4], l[4];
+    uint32_t p[NS][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const __nv_bfloat162 hb = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-        const uint32_t hu = *reinterpret_cast<const uint32_t *>(&hb);
-        const float h0 = __uint_as_float(hu << 16), h1 = __uint_as_float(hu & 0xffff0000u);
-        const __nv_bfloat162 lb = __floats2bfloat162_rn(v[2 * q] - h0, v[2 * q + 1] - h1);
-        h[q] = hu;
-        l[q] = *reinterpret_cast<const uint32_t *>(&lb);
+        float a = v[2 * q], b = v[2 * q + 1];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+            const uint32_t u = *reinterpret_cast<const uint32_t *>(&t);
+            p[s][q] = u;
+            a -= __uint_as_float(u << 16);
+            b -= __uint_as_float(u & 0xffff0000u);
+        }
     }
-    *reinterpret_cast<uint4 *>(dh) = make_uint4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<uint4 *>(dl) = make_uint4(l[0], l[1], l[2], l[3]);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) *reinterpret_cast<uint4 *>(dst + s * pstride) = make_uint4(p[s][0], p[s][1], p[s][2], p[s][3]);
 }
 
 // pipeline state of a CTA, carried from tile to tile (and job to job)
@@ -233,10 +249,11 @@ __host__ __device__ __forceinline__ long long box_tiles(const KParams &P)
 
 // Gamma records of tile t of the launch described by P (all threads of the
 // CTA call it together)
-template <int KC>
-__device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uint32_t tbase, BoxPipe &st)
+template <int KC, int NS>
+__device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned char *smem, uint32_t tbase, BoxPipe &st)
 {
-    using L = BoxLay<KC>;
+    using L = BoxLay<KC, NS>;
+    unsigned char *stages = smem + L::OFF_ST;
     unsigned char *Xb = smem + L::OFF_X;
     unsigned char *misc = smem + L::OFF_MISC;
     uint64_t *mbar = reinterpret_cast<uint64_t *>(misc);                 // 2 stages
@@ -246,7 +263,7 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
     uint32_t *tbad = reinterpret_cast<uint32_t *>(misc + 3200);          // [W] out-of-range samples
     uint32_t *umask = reinterpret_cast<uint32_t *>(smem + L::OFF_U);     // [128][W]
     const uint4 *lut = reinterpret_cast<const uint4 *>(smem + L::OFF_LUT);
-    uint32_t *nm = reinterpret_cast<uint32_t *>(smem + L::STAGE);        // nmap words (stage 1, mask build only)
+    uint32_t *nm = reinterpret_cast<uint32_t *>(stages + L::STAGE);      // nmap words (stage 1, mask build only)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n = P.nb, dp = (n + 1) >> 1, nblk = dp * (dp + 1) / 2, ncolt = 8 * nblk;
@@ -409,8 +426,8 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
             // before it is overwritten; a thread whose wait gave up builds
             // nothing and the vote below stops the CTA
             const bool late = box_poll(mbar, st, s);
-            unsigned char *As = smem + s * L::STAGE;
-            unsigned char *Bh = As + L::A_BYTES, *Bl = Bh + L::B_BYTES;
+            unsigned char *As = stages + s * L::STAGE;
+            unsigned char *Bs = As + L::A_BYTES;
             const int k0 = ch * KC;
             // chunk g + 1 (the first chunk again after the last one of a
             // pass) is in registers; chunk g + 2 is loaded while this one
@@ -429,7 +446,7 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
                 const uint32_t bits = (umask[m * W + (b0 >> 5)] >> (b0 & 31)) & 0xffu;
                 *reinterpret_cast<uint4 *>(As + (m >> 3) * L::SBO + k8 * 128 + (m & 7) * 16) = lut[bits];
             }
-            // ---- B: outer-product entries, hi and lo ----
+            // ---- B: outer-product entries, NS parts ----
             // one thread per half core matrix: block bl's rows 4 ia .. 4 ia + 3
             // (entries (2a + ia, 2b), (2a + ia, 2b + 1), Re and Im) over the 8
             // samples of K group k8
@@ -439,15 +456,13 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
                 const int jacc = bl / (BX_NCOL / 8);
                 const int nm_j = (jacc == 0) ? nmma[0] : nmma[L::NACC - 1];
                 if ((bl - jacc * (BX_NCOL / 8)) * 8 >= nm_j) continue;          // read by no MMA
-                unsigned char *dh = Bh + bl * L::SBO + k8 * 128 + ia * 64;
-                unsigned char *dl = Bl + bl * L::SBO + k8 * 128 + ia * 64;
+                unsigned char *db = Bs + bl * L::SBO + k8 * 128 + ia * 64;
                 if (bl * 8 >= ncol) {
                     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        *reinterpret_cast<uint4 *>(dh + c * 16) = z;
-                        *reinterpret_cast<uint4 *>(dl + c * 16) = z;
-                    }
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int p = 0; p < NS; ++p) *reinterpret_cast<uint4 *>(db + p * L::B_BYTES + c * 16) = z;
                     continue;
                 }
                 const short2 ab = blk[cb / 8 + bl];
@@ -469,8 +484,8 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
                         re[q] = fmaf(xr, yr, xi * yi);          // Re x_i conj(x_j)
                         im[q] = fmaf(xi, yr, -(xr * yi));       // Im x_i conj(x_j)
                     }
-                    store_split(dh + (2 * jb) * 16, dl + (2 * jb) * 16, re);
-                    store_split(dh + (2 * jb + 1) * 16, dl + (2 * jb + 1) * 16, im);
+                    store_split<NS>(db + (2 * jb) * 16, L::B_BYTES, re);
+                    store_split<NS>(db + (2 * jb + 1) * 16, L::B_BYTES, im);
                 }
             }
             // the next chunk's samples go to the other buffer, which the
@@ -485,7 +500,7 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
             if (__syncthreads_or(late)) { st.timed_out = true; break; }
             if (tid == 0) {
                 fence_after_sync();
-                const uint32_t a0 = smem_addr(As), h0 = smem_addr(Bh), l0 = smem_addr(Bl);
+                const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
 #pragma unroll
                 for (int kk = 0; kk < KC / 16; ++kk) {
                     const uint64_t da = make_smem_desc(a0 + kk * 256, 128, L::SBO);
@@ -493,11 +508,11 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
                     for (int j = 0; j < L::NACC; ++j) {
                         if (nmma[j] == 0) continue;
                         const uint32_t boff = (uint32_t)(j * (BX_NCOL / 8) * L::SBO + kk * 256);
-                        const uint64_t dh = make_smem_desc(h0 + boff, 128, L::SBO);
-                        const uint64_t dl = make_smem_desc(l0 + boff, 128, L::SBO);
                         const uint32_t dt = tbase + (uint32_t)(j * BX_NCOL);
-                        tc_mma(dt, da, dh, idesc[j], (ch > 0 || kk > 0) ? 1u : 0u);
-                        tc_mma(dt, da, dl, idesc[j], 1u);
+#pragma unroll
+                        for (int p = 0; p < NS; ++p)
+                            tc_mma(dt, da, make_smem_desc(b0 + p * L::B_BYTES + boff, 128, L::SBO), idesc[j],
+                                   (ch > 0 || kk > 0 || p > 0) ? 1u : 0u);
                     }
                 }
                 tc_commit(&mbar[s]);
@@ -523,20 +538,19 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
             for (int w = 0; w < W; ++w) any |= tbad[w];
             clean = any == 0;
         }
-        // ---- epilogue: warp w reads TMEM lanes 32(w%4).., BX_CPW x 32 columns ----
+        // ---- epilogue: warp w reads TMEM lanes 32(w%4).., every fourth 32 columns ----
         // A lane holds its own pixel's columns; they are written out through
         // a 32 x 32 staging tile per warp (in the operand stages, which no
         // MMA reads any more: both stages were waited for above) so that
         // each store instruction writes four pixels' 128 contiguous bytes
         // instead of 32 pixels' 16.
         {
-            constexpr int BX_CPW = (L::PCOL / 32) / (BX_THREADS / 128);
             constexpr int SROW = 36;                        // staging row stride (floats)
             static_assert((BX_THREADS / 32) * 32 * SROW * 4 <= 2 * L::STAGE, "staging fits the stages");
-            float *stg = reinterpret_cast<float *>(smem) + warp * (32 * SROW);
+            float *stg = reinterpret_cast<float *>(stages) + warp * (32 * SROW);
             float *rec = reinterpret_cast<float *>(P.cbuf);
             const int q = warp & 3, h = warp >> 2;
-            for (int c32 = BX_CPW * h; c32 < BX_CPW * h + BX_CPW; ++c32) {
+            for (int c32 = h; c32 < L::PCOL / 32; c32 += BX_THREADS / 128) {
                 const int col0 = 32 * c32;
                 if (col0 >= ncol) break;
                 uint32_t v[32];
@@ -578,17 +592,18 @@ __device__ void box_tile(const KParams &P, long long t, unsigned char *smem, uin
 
 }
 
+// barriers, tables and tensor memory, the same for both NS
 template <int KC>
 __device__ __forceinline__ uint32_t box_setup(unsigned char *smem, BoxPipe &st)
 {
-    using L = BoxLay<KC>;
+    using L = BoxLay<KC, 2>;
     unsigned char *misc = smem + L::OFF_MISC;
     uint64_t *mbar = reinterpret_cast<uint64_t *>(misc);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 16);
     const int tid = threadIdx.x, warp = tid >> 5;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_addr(tmem_slot)), "r"(L::PCOL) : "memory");
+                     :: "r"(smem_addr(tmem_slot)), "r"(L::TCOL) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
@@ -621,7 +636,7 @@ __device__ __forceinline__ uint32_t box_setup(unsigned char *smem, BoxPipe &st)
 template <int KC>
 __device__ __forceinline__ void box_teardown(unsigned char *smem, uint32_t tbase, BoxPipe &st, unsigned *err)
 {
-    using L = BoxLay<KC>;
+    using L = BoxLay<KC, 2>;
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::OFF_MISC);
     const int tid = threadIdx.x, warp = tid >> 5;
     if (st.timed_out) {
@@ -638,19 +653,19 @@ __device__ __forceinline__ void box_teardown(unsigned char *smem, uint32_t tbase
     __syncthreads();
     fence_after_sync();
     if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(L::PCOL) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tbase), "r"(L::TCOL) : "memory");
     }
 }
 
-template <int KC>
-__global__ void __launch_bounds__(BX_THREADS, 1) k_gram_box(KParams P)
+template <int KC, int NS>
+__global__ void __launch_bounds__(BX_THREADS, 1) k_gram_box(const __grid_constant__ KParams P)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     BoxPipe st;
     const uint32_t tbase = box_setup<KC>(smem, st);
     const long long ntiles = box_tiles(P);
     for (long long t = blockIdx.x; t < ntiles && !st.timed_out; t += gridDim.x)
-        box_tile<KC>(P, t, smem, tbase, st);
+        box_tile<KC, NS>(P, t, smem, tbase, st);
     box_teardown<KC>(smem, tbase, st, P.err);
 }
 
@@ -669,26 +684,19 @@ __global__ void __launch_bounds__(BX_THREADS, 1) k_gram_batch(const BoxSeg *__re
             const int mid = (lo + hi + 1) >> 1;
             if (segs[mid].tile_offset <= t) lo = mid; else hi = mid - 1;
         }
-        box_tile<KC>(segs[lo].P, t - segs[lo].tile_offset, smem, tbase, st);
+        const KParams &P = segs[lo].P;
+        if (P.parts == 3) box_tile<KC, 3>(P, t - segs[lo].tile_offset, smem, tbase, st);
+        else box_tile<KC, 2>(P, t - segs[lo].tile_offset, smem, tbase, st);
     }
     box_teardown<KC>(smem, tbase, st, segs[0].P.err);
 }
 
 template <int KC>
-size_t box_smem(int ny, int nx)
+size_t box_smem(int ny, int nx, int parts)
 {
-    using L = BoxLay<KC>;
     const int uh = BX_TR + 2 * ny, uwp = box_union_cols(nx);
     const int kp = (uh * uwp + KC - 1) / KC * KC;
-    return L::OFF_U + (size_t)BX_M * (kp / 32) * 4;
-}
-
-// per-kernel flags: attributes set once per device
-template <int KC, bool BATCH>
-bool *box_flags()
-{
-    static bool f[64] = {false};
-    return f;
+    return (parts == 3 ? BoxLay<KC, 3>::OFF_U : BoxLay<KC, 2>::OFF_U) + (size_t)BX_M * (kp / 32) * 4;
 }
 
 template <typename K>
@@ -702,25 +710,32 @@ cudaError_t box_configure(K kern, size_t smem_max, bool *configured)
     return e;
 }
 
-template <int KC>
+template <int KC, int NS>
 cudaError_t launch_box_t(const KParams &P, int num_sms, cudaStream_t st)
 {
-    using L = BoxLay<KC>;
-    cudaError_t e = box_configure(k_gram_box<KC>, L::MAX_SMEM, box_flags<KC, false>());
+    static bool configured[64] = {false};
+    cudaError_t e = box_configure(k_gram_box<KC, NS>, BoxLay<KC, NS>::MAX_SMEM, configured);
     if (e != cudaSuccess) return e;
     const long long ntiles = box_tiles(P);
     long long blocks = num_sms;
     if (ntiles < blocks) blocks = ntiles > 0 ? ntiles : 1;
-    k_gram_box<KC><<<(unsigned)blocks, BX_THREADS, box_smem<KC>(P.ny, P.nx), st>>>(P);
+    k_gram_box<KC, NS><<<(unsigned)blocks, BX_THREADS, box_smem<KC>(P.ny, P.nx, NS), st>>>(P);
     return cudaGetLastError();
+}
+
+template <int KC>
+cudaError_t configure_box_batch()
+{
+    static bool configured[64] = {false};
+    constexpr size_t m2 = BoxLay<KC, 2>::MAX_SMEM, m3 = BoxLay<KC, 3>::MAX_SMEM;
+    return box_configure(k_gram_batch<KC>, m2 > m3 ? m2 : m3, configured);
 }
 
 template <int KC>
 cudaError_t launch_box_batch_t(const BoxSeg *segs, int nseg, long long total, size_t smem, int num_sms,
                                cudaStream_t st)
 {
-    using L = BoxLay<KC>;
-    cudaError_t e = box_configure(k_gram_batch<KC>, L::MAX_SMEM, box_flags<KC, true>());
+    cudaError_t e = configure_box_batch<KC>();
     if (e != cudaSuccess) return e;
     long long blocks = num_sms;
     if (total < blocks) blocks = total > 0 ? total : 1;
@@ -746,15 +761,11 @@ int gram_box_record(int nb)
 
 long long gram_box_tiles(const KParams &P) { return box_tiles(P); }
 
-size_t gram_box_smem(int nb, int ny, int nx)
-{
-    (void)nb;
-    return box_smem<BX_KC>(ny, nx);
-}
+size_t gram_box_smem(const KParams &P) { return box_smem<BX_KC>(P.ny, P.nx, P.parts); }
 
 cudaError_t prepare_gram_batch()
 {
-    return box_configure(k_gram_batch<BX_KC>, BoxLay<BX_KC>::MAX_SMEM, box_flags<BX_KC, true>());
+    return configure_box_batch<BX_KC>();
 }
 
 cudaError_t launch_gram_batch(const BoxSeg *segs, int nseg, long long total, size_t smem, int num_sms,
@@ -769,7 +780,7 @@ cudaError_t launch_gram_box(const KParams &P, int num_sms, cudaStream_t st)
     if (!gram_box_supported(P.nb, P.ny, P.nx) || P.cols <= 0 || P.pix_begin % P.cols || P.npix % P.cols)
         return cudaErrorInvalidValue;
     if (P.npix == 0) return cudaSuccess;
-    return launch_box_t<BX_KC>(P, num_sms, st);
+    return P.parts == 3 ? launch_box_t<BX_KC, 3>(P, num_sms, st) : launch_box_t<BX_KC, 2>(P, num_sms, st);
 }
 
 }  // namespace fpl

@@ -57,14 +57,16 @@ int solve_max_warps(int np)
     return 1;
 }
 
-cudaError_t launch_solve_batch(int np, const BatchEntry *ents, int nent, long long total, int num_sms,
+int solve_kind(const KParams &P) { return 1 << tile_kind(P); }
+
+cudaError_t launch_solve_batch(int np, const BatchEntry *ents, int nent, long long total, int kinds, int num_sms,
                                cudaStream_t st, int warps)
 {
     if (nent <= 0 || total <= 0) return cudaSuccess;
     switch (np) {
-    case 16: return launch_solve_batch_t<16, 2>(ents, nent, total, num_sms, st, warps);
-    case 32: return launch_solve_batch_t<16, 4>(ents, nent, total, num_sms, st, warps);
-    case 64: return launch_solve_batch_t<32, 4>(ents, nent, total, num_sms, st, warps);
+    case 16: return launch_solve_batch_t<16, 2>(ents, nent, total, kinds, num_sms, st, warps);
+    case 32: return launch_solve_batch_t<16, 4>(ents, nent, total, kinds, num_sms, st, warps);
+    case 64: return launch_solve_batch_t<32, 4>(ents, nent, total, kinds, num_sms, st, warps);
     }
     return cudaErrorInvalidValue;
 }

@@ -1,12 +1,14 @@
 // kernels_impl.cuh -- pixel kernels and their launchers (included by
 // kernels_f32.cu and kernels_f64.cu so the two precisions compile in parallel).
 //
-// k_pixels<float, NP>  : plain FP32 form over a contiguous pixel range.
+// k_solve, k_rest      : eigen-solves from the tensor-core Gamma records.
+// k_pixels<float, NP>  : plain FP32 kernel over a contiguous pixel range (windows
+//                        the Gamma kernel does not take, and runs without scratch).
 // k_pixels<double, NP> : FP64 form over the work list written by the FP32
 //                        pass (pixels whose discrete decisions fall inside the
 //                        FP32 rounding band), or over every pixel when no list
 //                        is given (used to check the FP64 form itself).
-// Both are persistent: the grid is sized to the resident capacity of the
+// All are persistent: the grid is sized to the resident capacity of the
 // GPU; warps stride over a pixel range, or draw work-list entries from a
 // cursor.
 #pragma once
@@ -52,11 +54,19 @@ __global__ void k_pixels(KParams P)
 }
 
 // ---- eigen-solves from the Gamma records ---------------------------------
-// MLE pixels (and phase_link's) are solved in registers by k_solve, G lanes per
-// pixel (solve_tile.cuh); those it hands back, and the pixels of the other
-// methods, by k_rest, a warp per pixel with its coherence rows in tensor memory
-// (pixel_solve).  Neither issues an MMA.
-__device__ __forceinline__ bool tile_solved(const KParams &P) { return P.method == M_MLE || P.semantics == SEM_PL; }
+// Pixels are solved in registers by k_solve, G lanes per pixel
+// (solve_tile.cuh); those it hands back, phase_link's with a bandwidth (MLE with
+// STBAS's temporal coherence) and those of bandwidth 1 by k_rest, a warp per pixel with its coherence
+// rows in tensor memory (pixel_solve).  Neither issues an MMA.
+enum { TK_REST = 0, TK_MLE = 1, TK_EVD = 2 };
+__host__ __device__ __forceinline__ int tile_kind(const KParams &P)
+{
+    if (P.semantics == SEM_PL) return P.method == M_STBAS ? TK_REST : TK_MLE;
+    // a bandwidth of 1 makes C tridiagonal: pixel_solve's reduction is exact
+    // there and keeps the phases of components that the eigenvector hardly has
+    if (P.method == M_STBAS && P.bw == 1) return TK_REST;
+    return P.method == M_MLE ? TK_MLE : TK_EVD;
+}
 
 template <int G, int NL> struct SolveShape {
     using M = Tile<G, NL>;
@@ -69,8 +79,8 @@ template <int G, int NL> struct SolveShape {
 };
 
 // Solve kernel over a pixel source: SRC(q) gives (launch, pixel) of item q
-// of [0, total).
-template <int G, int NL, typename SRC>
+// of [0, total); pixels of launches of another kind are left alone.
+template <int G, int NL, int KIND, typename SRC>
 __device__ __forceinline__ void solve_loop(long long total, const SRC &src)
 {
     using SH = SolveShape<G, NL>;
@@ -93,36 +103,38 @@ __device__ __forceinline__ void solve_loop(long long total, const SRC &src)
         const bool in = q0 + h < total;
         long long pp;
         const KParams &P = src(in ? q0 + h : q0, pp);
-        const bool valid = in && tile_solved(P);
+        const bool valid = in && tile_kind(P) == KIND;
         if (k + nw < items && q0 + SH::PX * nw + h < total) {
             long long pn;
             const KParams &Pn = src(q0 + SH::PX * nw + h, pn);
             tile_prefetch<G>(Pn, pn, g);
         }
         if (!__any_sync(0xffffffffu, valid)) continue;
-        const int state = tile_mle<G, NL>(P, pp, L, taddr, valid);
+        int state;
+        if constexpr (KIND == TK_MLE) state = tile_mle<G, NL>(P, pp, L, taddr, valid);
+        else state = tile_evd<G, NL>(P, pp, L, taddr, valid);
         if (valid && state == TILE_GENERAL && g == 0) rest_put(P, pp);
         __syncwarp();
     }
     tmem_free_cta(tbase, warp, tcols);
 }
 
-template <int G, int NL>
+template <int G, int NL, int KIND>
 __global__ void __launch_bounds__(32 * SolveShape<G, NL>::max_warps, 1) k_solve(const __grid_constant__ KParams P)
 {
     const KParams *p = &P;
-    solve_loop<G, NL>(P.npix, [p](long long q, long long &pp) -> const KParams & {
+    solve_loop<G, NL, KIND>(P.npix, [p](long long q, long long &pp) -> const KParams & {
         pp = p->pix_begin + q;
         return *p;
     });
 }
 
 // over many launches of one padded depth
-template <int G, int NL>
+template <int G, int NL, int KIND>
 __global__ void __launch_bounds__(32 * SolveShape<G, NL>::max_warps, 1) k_solve_batch(const BatchEntry *__restrict__ ents,
                                                                                      int nent, long long total)
 {
-    solve_loop<G, NL>(total, [&](long long q, long long &pp) -> const KParams & {
+    solve_loop<G, NL, KIND>(total, [&](long long q, long long &pp) -> const KParams & {
         int lo = 0, hi = nent - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -138,7 +150,7 @@ template <int NP>
 __device__ __forceinline__ void rest_loop(const KParams &P, unsigned char *sm, int lane, const CRowsTmem<NP> &cp)
 {
     C2<float> *A = reinterpret_cast<C2<float> *>(sm + Lay<float, NP>::wm);
-    const bool listed = tile_solved(P);
+    const bool listed = tile_kind(P) != TK_REST;
     const long long cnt = listed ? *((volatile int *)(P.fb_count + 1)) : P.npix;
     for (long long q = rest_next(P, lane); q < cnt; q = rest_next(P, lane)) {
         const long long pp = P.cbase + (listed ? (long long)P.rest[q] : q);
@@ -164,7 +176,7 @@ template <int NP> constexpr int rest_max_warps() { return NP <= 32 ? 20 : 5; }
 template <int NP>
 __global__ void __launch_bounds__(32 * rest_max_warps<NP>(), 1) k_rest(const __grid_constant__ KParams P)
 {
-    if (tile_solved(P) && *((volatile int *)(P.fb_count + 1)) == 0) return;
+    if (tile_kind(P) != TK_REST && *((volatile int *)(P.fb_count + 1)) == 0) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ uint32_t tslot;
@@ -238,20 +250,26 @@ static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <int G, int NL, int KIND>
+static cudaError_t launch_solve_kind(const KParams &P, int num_sms, cudaStream_t st)
+{
+    static bool configured[64] = {false};
+    cudaError_t e = solve_configure(k_solve<G, NL, KIND>, configured);
+    if (e != cudaSuccess) return e;
+    int warps = solve_warps<G, NL>();
+    const long long blocks = solve_grid(SolveShape<G, NL>::items(P.npix), num_sms, &warps);
+    k_solve<G, NL, KIND><<<(unsigned)blocks, warps * 32, solve_smem(SolveShape<G, NL>::bytes, warps), st>>>(P);
+    return cudaGetLastError();
+}
+
 template <int G, int NL>
 static cudaError_t launch_solve_t(const KParams &P, int num_sms, cudaStream_t st)
 {
     constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
-    if (P.method == M_MLE || P.semantics == SEM_PL) {
-        static bool configured[64] = {false};
-        cudaError_t e = solve_configure(k_solve<G, NL>, configured);
-        if (e != cudaSuccess) return e;
-        int warps = solve_warps<G, NL>();
-        const long long blocks = solve_grid(SolveShape<G, NL>::items(P.npix), num_sms, &warps);
-        k_solve<G, NL><<<(unsigned)blocks, warps * 32, solve_smem(SolveShape<G, NL>::bytes, warps), st>>>(P);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    return launch_rest_t<NP>(P, num_sms, st);
+    cudaError_t e = cudaSuccess;
+    if (tile_kind(P) == TK_MLE) e = launch_solve_kind<G, NL, TK_MLE>(P, num_sms, st);
+    else if (tile_kind(P) == TK_EVD) e = launch_solve_kind<G, NL, TK_EVD>(P, num_sms, st);
+    return e != cudaSuccess ? e : launch_rest_t<NP>(P, num_sms, st);
 }
 
 // attributes of the batch kernels, set once per device
@@ -259,15 +277,17 @@ template <int G, int NL>
 static cudaError_t configure_solve_batch()
 {
     constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
-    static bool configured[64] = {false}, rest[64] = {false};
-    const cudaError_t e = solve_configure(k_solve_batch<G, NL>, configured);
+    static bool mle[64] = {false}, evd[64] = {false}, rest[64] = {false};
+    cudaError_t e = solve_configure(k_solve_batch<G, NL, TK_MLE>, mle);
+    if (e == cudaSuccess) e = solve_configure(k_solve_batch<G, NL, TK_EVD>, evd);
     return e != cudaSuccess ? e : solve_configure(k_rest_batch<NP>, rest);
 }
 
-// warps_req > 0: at most that many warps per CTA (the batch autotuner's
-// candidates); 0: as many as fit
+// kinds: which kinds of pixels the entries hold (bit KIND); warps_req > 0: at
+// most that many warps per CTA (the batch autotuner's candidates); 0: as many
+// as fit
 template <int G, int NL>
-static cudaError_t launch_solve_batch_t(const BatchEntry *ents, int nent, long long total, int num_sms,
+static cudaError_t launch_solve_batch_t(const BatchEntry *ents, int nent, long long total, int kinds, int num_sms,
                                        cudaStream_t st, int warps_req)
 {
     constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
@@ -275,8 +295,10 @@ static cudaError_t launch_solve_batch_t(const BatchEntry *ents, int nent, long l
     if (e != cudaSuccess) return e;
     int warps = solve_warps<G, NL>();
     if (warps_req > 0 && warps > warps_req) warps = warps_req;
-    const long long blocks = solve_grid(SolveShape<G, NL>::items(total), num_sms, &warps);
-    k_solve_batch<G, NL><<<(unsigned)blocks, warps * 32, solve_smem(SolveShape<G, NL>::bytes, warps), st>>>(ents, nent, total);
+    const unsigned blocks = (unsigned)solve_grid(SolveShape<G, NL>::items(total), num_sms, &warps);
+    const size_t smem = solve_smem(SolveShape<G, NL>::bytes, warps);
+    if (kinds & (1 << TK_MLE)) k_solve_batch<G, NL, TK_MLE><<<blocks, warps * 32, smem, st>>>(ents, nent, total);
+    if (kinds & (1 << TK_EVD)) k_solve_batch<G, NL, TK_EVD><<<blocks, warps * 32, smem, st>>>(ents, nent, total);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int rw = rest_max_warps<NP>();
     const long long rb = solve_grid(total, num_sms, &rw);

@@ -52,7 +52,8 @@ struct KParams {
     int fb_cap;
     unsigned *err;                      // error flags (scratch)
     int *slow;                          // pixels that left the fast eigen path (scratch)
-    // mixed form: Gamma records from the tensor-core kernel
+    // Gamma records from the tensor-core kernel
+    int parts;                          // bf16 parts per product: 2 mixed form, 3 FP32 form
     float2 *cbuf;                       // [pixel - cbase][cstride floats] (pixel_load_gamma)
     int *cinfo;                         // [pixel - cbase]: SHP count, or CI_* below
     long long cbase;                    // first pixel of the buffers

@@ -8,11 +8,11 @@
 //     stages their inputs on a copy stream (stream-ordered allocation);
 //   * runs "waves" on a compute stream: every resident job whose inputs
 //     have arrived contributes a slice of rows (a fair share of the wave's
-//     pixel budget), and the slices of all jobs run as one persistent batch
-//     launch per padded depth and form (plain FP32; or, for jobs asking for
-//     the mixed-precision form, one tensor-core Gamma launch over the tiles
-//     of their slices and one solve launch) plus one FP64 settle launch --
-//     jobs that arrive while a wave runs join the next wave;
+//     pixel budget), and the slices of all jobs run as one tensor-core Gamma
+//     launch over their tiles and, per padded depth, solve launches (or one
+//     plain FP32 launch for windows the Gamma kernel does not take) plus one
+//     FP64 settle launch -- jobs that arrive while a wave runs join the next
+//     wave;
 //   * copies a finished job's outputs back on the copy stream, frees its
 //     device memory and wakes its waiters.
 // Copies overlap with waves.  Each pixel's result depends only on its own
@@ -65,7 +65,7 @@ struct Piece {
     SJob *job;
     int ra, rb;
     int np;
-    int mixed;     // 1: mixed-precision form
+    int tiled;     // 1: Gamma records on the tensor cores
 };
 
 constexpr size_t kPieceCounterBytes = 64;
@@ -90,7 +90,7 @@ struct fpl_server {
     cudaEvent_t ev_wave = nullptr;
     int max_pieces = 256;
     fpl::BatchEntry *d_table = nullptr, *h_table = nullptr;
-    fpl::BoxSeg *d_segs = nullptr, *h_segs = nullptr;   // Gamma segments of a wave's mixed pieces
+    fpl::BoxSeg *d_segs = nullptr, *h_segs = nullptr;   // Gamma segments of a wave's tiled pieces
     void *d_rec = nullptr;                              // their Gamma records, tile infos and rest lists
     size_t rec_cap = 0;
     void *d_wave = nullptr;
@@ -199,20 +199,17 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         const int ra = j->next_row, rb = std::min(j->r1, ra + rows);
         j->next_row = rb;
         if (!j->started) { j->started = true; j->t_first = clk::now(); }
-        const int mixed = (j->host.precision == FPL_PREC_MIXED &&
-                           fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x))
-                              ? 1
-                              : 0;
-        pieces.push_back({j, ra, rb, fpl::pick_np(j->host.nbands), mixed});
+        const int tiled = fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x) ? 1 : 0;
+        pieces.push_back({j, ra, rb, fpl::pick_np(j->host.nbands), tiled});
         total += (long long)(rb - ra) * j->host.cols;
     }
     std::stable_sort(pieces.begin(), pieces.end(), [](const Piece &a, const Piece &b) {
-        return a.np != b.np ? a.np < b.np : a.mixed < b.mixed;
+        return a.np != b.np ? a.np < b.np : a.tiled < b.tiled;
     });
-    // Gamma records of the wave's mixed pieces
+    // Gamma records of the wave's tiled pieces
     size_t rec_floats = 0, infos = 0;
     for (const Piece &pc : pieces)
-        if (pc.mixed) {
+        if (pc.tiled) {
             const size_t px = (size_t)(pc.rb - pc.ra) * pc.job->host.cols;
             rec_floats += px * fpl::gram_box_record(pc.job->host.nbands);
             infos += px;
@@ -224,7 +221,15 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         if (s->d_rec) cudaFree(s->d_rec);
         s->d_rec = nullptr;
         s->rec_cap = 0;
-        if (cudaMalloc(&s->d_rec, rec_need) != cudaSuccess) return false;
+        if (cudaMalloc(&s->d_rec, rec_need) != cudaSuccess) {
+            if (s->cfg.wave_pixels <= 65536) return false;
+            // short of device memory: smaller waves from here on
+            cudaGetLastError();
+            s->cfg.wave_pixels /= 2;
+            for (Piece &pc : pieces) pc.job->next_row = pc.ra;
+            pieces.clear();
+            return true;
+        }
         s->rec_cap = rec_need;
     }
     float *recs = static_cast<float *>(s->d_rec);
@@ -236,7 +241,7 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
     long long loff = 0, coff = 0;
     for (size_t e = 0; e < pieces.size(); ++e) {
         const Piece &pc = pieces[e];
-        if (e > 0 && (pieces[e - 1].np != pc.np || pieces[e - 1].mixed != pc.mixed)) coff = 0;
+        if (e > 0 && (pieces[e - 1].np != pc.np || pieces[e - 1].tiled != pc.tiled)) coff = 0;
         fpl::KParams &P = s->h_table[e].P;
         fpl::fill_params(P, pc.job->dev, pc.ra, pc.rb, kDefaultAmbScale, kDefaultCondMax);
         P.fb_count = reinterpret_cast<int *>(base + kPieceCounterBytes * e);
@@ -244,7 +249,7 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         P.slow = reinterpret_cast<int *>(base + kPieceCounterBytes * e + 32);
         P.fb_list = lists + loff;
         P.fb_cap = (int)P.npix;
-        if (pc.mixed) {
+        if (pc.tiled) {
             P.cbuf = reinterpret_cast<float2 *>(recs + roff);
             P.cinfo = rinfo + ioff;
             P.rest = P.cinfo + infos;
@@ -257,18 +262,18 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         coff += P.npix;
         loff += P.npix;
     }
-    // Gamma segments of the mixed pieces
+    // Gamma segments of the tiled pieces
     int nseg = 0;
     long long tiles = 0;
     size_t gsm = 0;
     for (size_t e = 0; e < pieces.size(); ++e) {
         const fpl::KParams &P = s->h_table[e].P;
-        if (!pieces[e].mixed) continue;
+        if (!pieces[e].tiled) continue;
         fpl::BoxSeg &sg = s->h_segs[nseg++];
         sg.P = P;
         sg.tile_offset = tiles;
         tiles += fpl::gram_box_tiles(P);
-        gsm = std::max(gsm, fpl::gram_box_smem(P.nb, P.ny, P.nx));
+        gsm = std::max(gsm, fpl::gram_box_smem(P));
     }
     if (nseg &&
         cudaMemcpyAsync(s->d_segs, s->h_segs, sizeof(fpl::BoxSeg) * nseg, cudaMemcpyHostToDevice,
@@ -285,14 +290,18 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
     size_t e = 0;
     int cls = 0;
     while (e < pieces.size()) {
-        const int np = pieces[e].np, mixed = pieces[e].mixed;
+        const int np = pieces[e].np, tiled = pieces[e].tiled;
         const size_t first = e;
         long long n_px = 0;
-        while (e < pieces.size() && pieces[e].np == np && pieces[e].mixed == mixed) n_px += s->h_table[e++].P.npix;
+        int kinds = 0;
+        while (e < pieces.size() && pieces[e].np == np && pieces[e].tiled == tiled) {
+            kinds |= fpl::solve_kind(s->h_table[e].P);
+            n_px += s->h_table[e++].P.npix;
+        }
         if (fpl::configure_np(np) != cudaSuccess) return false;
-        if (mixed) {
+        if (tiled) {
             if (fpl::prepare_mixed_batch(np) != cudaSuccess) return false;
-            if (fpl::launch_solve_batch(np, s->d_table + first, (int)(e - first), n_px, s->num_sms, s->s_compute) !=
+            if (fpl::launch_solve_batch(np, s->d_table + first, (int)(e - first), n_px, kinds, s->num_sms, s->s_compute) !=
                 cudaSuccess)
                 return false;
         } else if (fpl::launch_batch(np, s->d_table + first, (int)(e - first), n_px, work + cls,

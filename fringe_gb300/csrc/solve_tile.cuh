@@ -455,26 +455,30 @@ template <int G> __device__ __forceinline__ void tile_zero(const KParams &P, lon
     }
 }
 
-// A pixel per G lanes from its Gamma record (every lane of the warp calls
-// it; valid: this group has a pixel).  taddr: NB x 8 tensor-memory columns of the
-// warp, where C waits between its uses.  Returns TILE_GENERAL where
-// pixel_solve has to take the pixel over (its outputs untouched).
-template <int G, int NL>
-__device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const TileLane &L, uint32_t taddr, bool valid)
+// f(x, block index) on the lanes that hold diagonal blocks: (x, RT x + lr / 4)
+template <int G, int NL, typename F> __device__ __forceinline__ void tile_on_diag(const TileLane &L, F &&f)
 {
     using M = Tile<G, NL>;
-    constexpr int NB = M::NB, RT = M::RT, LRN = M::LRN, NLC = M::NLC;
+#pragma unroll
+    for (int x = 0; x < NL; ++x)
+#pragma unroll
+        for (int h = 0; h < M::RT; ++h)
+            if ((L.lr & 3) == L.lc && (L.lr >> 2) == h) f(x, M::blk(x, M::RT * x + h));
+}
+
+// Record to coherence (in A and in tensor memory at taddr) and the start
+// vector, C 1 normalised (in z).  MLE: the pixel's method is; else EVD or STBAS
+// (whose C is banded).  Returns the outcome so far; cfro = |C|_F.
+template <int G, int NL, bool MLE>
+__device__ __forceinline__ int tile_begin(const KParams &P, long long pp, const TileLane &L, uint32_t taddr, bool valid,
+                                          CBlk (&A)[Tile<G, NL>::NB], float &cfro)
+{
+    using M = Tile<G, NL>;
+    constexpr int RT = M::RT, LRN = M::LRN, NLC = M::NLC;
     const int n = P.nb, dp = (n + 1) >> 1;
     const bool plink = P.semantics == SEM_PL;
-    const bool dlane = (L.lr & 3) == L.lc;                 // holds diagonal blocks: (x, RT x + dh)
+    const bool dlane = (L.lr & 3) == L.lc;
     const int dh = L.lr >> 2;
-    auto on_diag = [&](auto &&f) {                         // f(x, block index) on the lanes that hold it
-#pragma unroll
-        for (int x = 0; x < NL; ++x)
-#pragma unroll
-            for (int h = 0; h < RT; ++h)
-                if (dlane && dh == h) f(x, M::blk(x, RT * x + h));
-    };
     int state = valid ? TILE_RUN : TILE_DONE;
     int npix = 0;
 
@@ -490,7 +494,6 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
         }
         npix = info;
     }
-    CBlk A[NB];
     {
         const float4 *rec =
             reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(P.cbuf) + (valid ? pp - P.cbase : 0) * (long long)P.cstride);
@@ -519,7 +522,7 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
     // ---- coherence (evd.cpp:566-582) --------------------------------------------
     bool bad = false;
     const uint32_t yv = L.mem + M::v;
-    on_diag([&](int x, int b) {
+    tile_on_diag<G, NL>(L, [&](int x, int b) {
         const int i = 2 * (LRN * x + L.lr);
         const float p0 = lo2(A[b].dr), p1 = hi2(A[b].dr);
         bad |= i < n && (!(p0 > 0.f) || !isfinite(p0));
@@ -544,6 +547,13 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
                 k.di = mul2(k.di, d);
                 k.er = mul2(k.er, e);
                 k.ei = mul2(k.ei, e);
+                if (!MLE && P.method == M_STBAS) {               // evd.cpp:695-706
+                    const int d = 2 * (LRN * mi + L.lr - 4 * li - L.lc), bw = P.bw;     // i - j
+                    if (abs(d) > bw) k.dr = k.di = 0ull;
+                    const f32x2 m = pk(abs(d + 1) > bw ? 0.f : 1.f, abs(d - 1) > bw ? 0.f : 1.f);
+                    k.er = mul2(k.er, m);
+                    k.ei = mul2(k.ei, m);
+                }
                 const bool dg = li >= RT * mi && dlane && dh == li - RT * mi;
                 if (dg) {                                        // unit diagonal
                     const int i = 2 * (LRN * mi + L.lr);
@@ -566,17 +576,17 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
     }
     if (state == TILE_RUN && bad) {
         tile_zero<G>(P, pp, L.g);
-        put_code(P, pp, L.g, -1);
+        put_code(P, pp, L.g, MLE ? -1 : -6);
         state = TILE_DONE;
     }
-    if (state == TILE_RUN && !plink && npix < n) {
+    if (MLE && state == TILE_RUN && !plink && npix < n) {
         // fewer SHPs than dates: rank-deficient (see pixel_solve)
         tile_zero<G>(P, pp, L.g);
         put_code(P, pp, L.g, -2);
         state = TILE_DONE;
     }
     if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
-    const float cfro = sqrtf(fs);
+    cfro = sqrtf(fs);
 
     // ---- C to tensor memory; start vector C 1, normalised (rows of C) -------------
     {
@@ -626,164 +636,34 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
                      inv * hi2(ri[x]));
         }
     }
-    // the groups' steps run together: the padding's pivots are 1
-    const int tp = G == 32 ? dp : max(__shfl_sync(0xffffffffu, dp, 0), __shfl_sync(0xffffffffu, dp, 16));
-    const float amb = P.amb * (float)n * Eps<float>::v, thr = 1.0e-6f;
-    float sigma = 0.f;
-    // pass 0: lambda_min(C) > 1e-6 by the factorisation of C - (1e-6 + band) I,
-    // the inverse of |C|, M; pass 1: the factor of M - sigma I.  One loop, so that the unrolled
-    // factorisation is in the code once.
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1) {
-            // |C| and its inverse (evd.cpp:586-664)
-            RBlk K[NB];
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                uint32_t w[8];
-                tmem_ld8(taddr + 8u * (uint32_t)b, w);
-                float a[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    // entries: D lo, D hi, E lo, E hi
-                    const float x = __uint_as_float(w[(e & 1) + 4 * (e >> 1)]), y = __uint_as_float(w[(e & 1) + 4 * (e >> 1) + 2]);
-                    const float m2 = fmaf(x, x, y * y);
-                    a[e] = m2 * rsqrtf(fmaxf(m2, 1e-37f));
-                }
-                K[b].d = pk(a[0], a[1]);
-                K[b].e = pk(a[2], a[3]);
-            }
-            on_diag([&](int, int b) { K[b].d = pk(1.f, 1.f); });
-            const float anorm = tile_inf_norm<G, NL>(K, L);
-            bool ok = true;
-            tile_sweep_seg<G, NL, 0>(K, L, tp, ok);
-            // inv|C| = -K, its diagonal 2 - K
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                K[b].d ^= 0x8000000080000000ull;
-                K[b].e ^= 0x8000000080000000ull;
-            }
-            on_diag([&](int, int b) { K[b].d = add2(K[b].d, pk(2.f, 2.f)); });
-            const float xnorm = tile_inf_norm<G, NL>(K, L);
-            if (state == TILE_RUN && !ok) state = TILE_GENERAL;
-            if (state == TILE_RUN && (!(anorm * xnorm <= P.cond_max) || (!plink && !(1.f / xnorm > thr + amb * (float)n)))) {
-                // condition too large for an FP32 inverse, or 1/||inv|C||| within the band of 1e-6
-                tile_zero<G>(P, pp, L.g);
-                defer_fp64(P, pp, L.g);
-                state = TILE_DONE;
-            }
-            if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
-            // M = inv|C| o C and the Rayleigh quotient of the start vector
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                uint32_t w[8];
-                tmem_ld8(taddr + 8u * (uint32_t)b, w);
-                A[b].dr = mul2(pk(__uint_as_float(w[0]), __uint_as_float(w[1])), K[b].d);
-                A[b].di = mul2(pk(__uint_as_float(w[2]), __uint_as_float(w[3])), K[b].d);
-                A[b].er = mul2(pk(__uint_as_float(w[4]), __uint_as_float(w[5])), K[b].e);
-                A[b].ei = mul2(pk(__uint_as_float(w[6]), __uint_as_float(w[7])), K[b].e);
-            }
-            f32x2 zr[NLC], zi[NLC], q2 = 0ull;
-#pragma unroll
-            for (int li = 0; li < NLC; ++li) lds4(L.mem + M::z + 16u * (uint32_t)(4 * li + L.lc), zr[li], zi[li]);
-            const f32x2 two = pk(2.f, 2.f), minus = pk(-1.f, -1.f);
-#pragma unroll
-            for (int mi = 0; mi < NL; ++mi) {
-                // y = sum_li weight M z, in the rows' order (D) and swapped (E)
-                f32x2 yr = 0ull, yi = 0ull, sr = 0ull, si = 0ull;
-#pragma unroll
-                for (int li = 0; li < RT * (mi + 1); ++li) {
-                    const CBlk &b = A[M::blk(mi, li)];
-                    const f32x2 nzi = mul2(zi[li], minus);
-                    if (li == RT * mi) {               // the blocks below the diagonal count twice
-                        yr = mul2(yr, two); yi = mul2(yi, two); sr = mul2(sr, two); si = mul2(si, two);
-                    }
-                    yr = fma2(b.di, nzi, fma2(b.dr, zr[li], yr));
-                    yi = fma2(b.di, zr[li], fma2(b.dr, zi[li], yi));
-                    sr = fma2(b.ei, nzi, fma2(b.er, zr[li], sr));
-                    si = fma2(b.ei, zr[li], fma2(b.er, zi[li], si));
-                }
-                f32x2 xr, xi;
-                lds4(L.mem + M::z + 16u * (uint32_t)(LRN * mi + L.lr), xr, xi);
-                q2 = fma2(xr, yr, fma2(xi, yi, q2));
-                q2 = fma2(swap2(xr), sr, fma2(swap2(xi), si, q2));
-            }
-            const float rho = gsum<G>(lo2(q2) + hi2(q2));
-            sigma = P.shift * fminf(rho, 1.f);
-            // lambda_1 > sigma > 1e-6 + band settles the -7 test; the band by
-            // |M|_F <= sqrt(n) ||inv|C|||_inf (see pixel_solve)
-            const float dM = plink ? 0.f : amb * sqrtf((float)n) * xnorm;
-            if (state == TILE_RUN && !(sigma > thr + dM)) state = TILE_GENERAL;
-            // the padding keeps a unit pivot
-            on_diag([&](int x, int b) {
-                const int i = 2 * (LRN * x + L.lr);
-                A[b].dr = pk(i < n ? lo2(A[b].dr) - sigma : 1.f, i + 1 < n ? hi2(A[b].dr) - sigma : 1.f);
-            });
-        } else {
-            if (__all_sync(0xffffffffu, plink || state != TILE_RUN)) continue;   // phase_link has no such test
-            const float sh = thr + amb * cfro;
-            on_diag([&](int, int b) { A[b].dr = add2(A[b].dr, pk(-sh, -sh)); });
-        }
-        bool ok = true;
-        tile_ldl_seg<G, NL, 0>(A, L, tp, ok);
-        if (state == TILE_RUN && !ok && (pass == 1 || !plink)) state = TILE_GENERAL;
-        if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
-        __syncwarp();
-    }
+    __syncwarp();
+    return state;
+}
 
-    // ---- inverse iteration (warp_inverse_iteration's rule, pair per lane) -----------
-    f32x2 zr, zi;
-    lds4(L.mem + M::z + 16u * (uint32_t)(L.g < M::T ? L.g : 0), zr, zi);
-    float z0r = lo2(zr), z1r = hi2(zr), z0i = lo2(zi), z1i = hi2(zi);
-    if (L.g >= dp) z0r = z1r = z0i = z1i = 0.f;
-    // the pixel's own samples, needed at the end: their loads overlap the iteration
-    float2 own[2];
+// the pixel's own samples of dates 2 g, 2 g + 1 (from the reference date on),
+// loaded ahead of the iteration that they are needed after
+__device__ __forceinline__ void tile_own(const KParams &P, long long pp, const TileLane &L, bool go, float2 (&own)[2])
+{
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int i = 2 * L.g + h;
         own[h] = make_float2(0.f, 0.f);
-        if (state == TILE_RUN && i < n && i >= P.mini - 1) own[h] = __ldg(P.stack + i * P.plane + pp);
+        if (go && i < P.nb && i >= P.mini - 1) own[h] = __ldg(P.stack + i * P.plane + pp);
     }
-    const float tol = 1e-5f;
-    float rprev = -1.f, cprev = 1.f, gap_good = 0.f;
-    bool run = state == TILE_RUN;
-    if (run) state = TILE_GENERAL;                    // unless it converges
-#pragma unroll 1
-    for (int it = 0; it < 10 && __any_sync(0xffffffffu, run); ++it) {
-        float x0r = z0r, x1r = z1r, x0i = z0i, x1i = z1i;
-        tile_solve<G, NL>(L, tp, x0r, x1r, x0i, x1i);
-        const float xx = gsum<G>(fmaf(x0r, x0r, x0i * x0i) + fmaf(x1r, x1r, x1i * x1i));
-        const float xv = gsum<G>(fmaf(x0r, z0r, x0i * z0i) + fmaf(x1r, z1r, x1i * z1i));
-        const float dl = xv / xx;                     // rho - sigma
-        const float a0r = fmaf(-dl, x0r, z0r), a0i = fmaf(-dl, x0i, z0i), a1r = fmaf(-dl, x1r, z1r), a1i = fmaf(-dl, x1i, z1i);
-        const float inv = rsqrtf(xx);
-        const float rn = sqrtf(gsum<G>(fmaf(a0r, a0r, a0i * a0i) + fmaf(a1r, a1r, a1i * a1i))) * inv;
-        if (run) {
-            z0r = x0r * inv;
-            z1r = x1r * inv;
-            z0i = x0i * inv;
-            z1i = x1i * inv;
-            if (rprev > 0.f) {
-                const float c = rn / rprev, crate = fmaxf(c, cprev);
-                if (crate < 0.9f) {
-                    const float gap = dl * (1.f / crate - 1.f);
-                    gap_good = gap;
-                    if (rn <= tol * gap) { state = TILE_RUN; run = false; }
-                }
-                if (run && it >= 3 && c > 0.9f) {
-                    if (rn <= 20.f * tol * gap_good) state = TILE_RUN;
-                    run = false;
-                }
-                cprev = c;
-            }
-            rprev = rn;
-        }
-    }
-    if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+}
 
+// Phases, compressed SLC and temporal coherence of the eigenvector z (pair
+// 2 g, 2 g + 1 on lane g) where fin; stbas: only pairs within the bandwidth
+// count in the temporal coherence.  Every lane calls it.
+template <int G, int NL>
+__device__ __forceinline__ void tile_finish(const KParams &P, long long pp, const TileLane &L, uint32_t taddr, bool fin,
+                                            bool stbas, float z0r, float z1r, float z0i, float z1i, const float2 (&own)[2])
+{
+    using M = Tile<G, NL>;
+    constexpr int RT = M::RT, LRN = M::LRN, NLC = M::NLC;
+    const int n = P.nb;
     // ---- phase referencing (evd.cpp:738-749) -----------------------------------------
     const int mref = P.mini - 1;
-    const bool fin = state == TILE_RUN;
     float ur, ui;
     {
         const float er = (mref & 1) ? z1r : z0r, ei = (mref & 1) ? z1i : z0i;
@@ -841,10 +721,11 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
                     }
                 };
                 const float jr = lo2(pr[li]), ji = lo2(pi[li]), kr = hi2(pr[li]), ki = hi2(pi[li]);
-                term(0, jr, ji, all, w0r, w0i);          // (i, j)
-                term(1, kr, ki, all, w1r, w1i);          // (i', j')
-                term(4, jr, ji, some, w1r, w1i);         // (i', j)
-                term(5, kr, ki, all, w0r, w0i);          // (i, j')
+                const int d = stbas ? P.bw - 2 * (m - l) : 1;        // pairs at most the bandwidth apart
+                term(0, jr, ji, all && d >= 0, w0r, w0i);            // (i, j)
+                term(1, kr, ki, all && d >= 0, w1r, w1i);            // (i', j')
+                term(4, jr, ji, some && d >= 1, w1r, w1i);           // (i', j)
+                term(5, kr, ki, all && d >= -1, w0r, w0i);           // (i, j')
             }
             f32x2 ar, ai;
             lds4(L.mem + M::z + 16u * (uint32_t)(LRN * mi + L.lr), ar, ai);
@@ -864,12 +745,368 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
     if (fin && L.g == 0) {
         const float den = (float)(n - mref);
         P.comp[pp] = make_float2(cr / den, ci / den);
-        P.tcorr[pp] = sqrtf(tr * tr + ti * ti) / (float)(n * (n - 1) / 2);   // 0/0 = NaN for one date, as the reference
+        const int pairs = stbas ? (n - P.bw) * P.bw + P.bw * (P.bw - 1) / 2 : n * (n - 1) / 2;
+        P.tcorr[pp] = sqrtf(tr * tr + ti * ti) / (float)pairs;   // 0/0 = NaN for one date, as the reference
         if (P.status) P.status[pp] = 0;
     }
-    return fin ? (int)TILE_DONE : state;
 }
 
+// MLE: a pixel per G lanes from its Gamma record (every lane of the warp calls
+// it; valid: this group has a pixel).  taddr: NB x 8 tensor-memory columns of the
+// warp, where C waits between its uses.  Returns TILE_GENERAL where
+// pixel_solve has to take the pixel over (its outputs untouched).
+template <int G, int NL>
+__device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const TileLane &L, uint32_t taddr, bool valid)
+{
+    using M = Tile<G, NL>;
+    constexpr int NB = M::NB, RT = M::RT, LRN = M::LRN, NLC = M::NLC;
+    const int n = P.nb, dp = (n + 1) >> 1;
+    const bool plink = P.semantics == SEM_PL;
+    CBlk A[NB];
+    float cfro = 0.f;
+    int state = tile_begin<G, NL, true>(P, pp, L, taddr, valid, A, cfro);
+    if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+    // the groups' steps run together: the padding's pivots are 1
+    const int tp = G == 32 ? dp : max(__shfl_sync(0xffffffffu, dp, 0), __shfl_sync(0xffffffffu, dp, 16));
+    const float amb = P.amb * (float)n * Eps<float>::v, thr = 1.0e-6f;
+    float sigma = 0.f;
+    // pass 0: lambda_min(C) > 1e-6 by the factorisation of C - (1e-6 + band) I,
+    // the inverse of |C|, M; pass 1: the factor of M - sigma I.  One loop, so that the unrolled
+    // factorisation is in the code once.
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1) {
+            // |C| and its inverse (evd.cpp:586-664)
+            RBlk K[NB];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                uint32_t w[8];
+                tmem_ld8(taddr + 8u * (uint32_t)b, w);
+                float a[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    // entries: D lo, D hi, E lo, E hi
+                    const float x = __uint_as_float(w[(e & 1) + 4 * (e >> 1)]), y = __uint_as_float(w[(e & 1) + 4 * (e >> 1) + 2]);
+                    const float m2 = fmaf(x, x, y * y);
+                    a[e] = m2 * rsqrtf(fmaxf(m2, 1e-37f));
+                }
+                K[b].d = pk(a[0], a[1]);
+                K[b].e = pk(a[2], a[3]);
+            }
+            tile_on_diag<G, NL>(L, [&](int, int b) { K[b].d = pk(1.f, 1.f); });
+            const float anorm = tile_inf_norm<G, NL>(K, L);
+            bool ok = true;
+            tile_sweep_seg<G, NL, 0>(K, L, tp, ok);
+            // inv|C| = -K, its diagonal 2 - K
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                K[b].d ^= 0x8000000080000000ull;
+                K[b].e ^= 0x8000000080000000ull;
+            }
+            tile_on_diag<G, NL>(L, [&](int, int b) { K[b].d = add2(K[b].d, pk(2.f, 2.f)); });
+            const float xnorm = tile_inf_norm<G, NL>(K, L);
+            if (state == TILE_RUN && !ok) state = TILE_GENERAL;
+            if (state == TILE_RUN && (!(anorm * xnorm <= P.cond_max) || (!plink && !(1.f / xnorm > thr + amb * (float)n)))) {
+                // condition too large for an FP32 inverse, or 1/||inv|C||| within the band of 1e-6
+                tile_zero<G>(P, pp, L.g);
+                defer_fp64(P, pp, L.g);
+                state = TILE_DONE;
+            }
+            if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+            // M = inv|C| o C and the Rayleigh quotient of the start vector
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                uint32_t w[8];
+                tmem_ld8(taddr + 8u * (uint32_t)b, w);
+                A[b].dr = mul2(pk(__uint_as_float(w[0]), __uint_as_float(w[1])), K[b].d);
+                A[b].di = mul2(pk(__uint_as_float(w[2]), __uint_as_float(w[3])), K[b].d);
+                A[b].er = mul2(pk(__uint_as_float(w[4]), __uint_as_float(w[5])), K[b].e);
+                A[b].ei = mul2(pk(__uint_as_float(w[6]), __uint_as_float(w[7])), K[b].e);
+            }
+            f32x2 zr[NLC], zi[NLC], q2 = 0ull;
+#pragma unroll
+            for (int li = 0; li < NLC; ++li) lds4(L.mem + M::z + 16u * (uint32_t)(4 * li + L.lc), zr[li], zi[li]);
+            const f32x2 two = pk(2.f, 2.f), minus = pk(-1.f, -1.f);
+#pragma unroll
+            for (int mi = 0; mi < NL; ++mi) {
+                // y = sum_li weight M z, in the rows' order (D) and swapped (E)
+                f32x2 yr = 0ull, yi = 0ull, sr = 0ull, si = 0ull;
+#pragma unroll
+                for (int li = 0; li < RT * (mi + 1); ++li) {
+                    const CBlk &b = A[M::blk(mi, li)];
+                    const f32x2 nzi = mul2(zi[li], minus);
+                    if (li == RT * mi) {               // the blocks below the diagonal count twice
+                        yr = mul2(yr, two); yi = mul2(yi, two); sr = mul2(sr, two); si = mul2(si, two);
+                    }
+                    yr = fma2(b.di, nzi, fma2(b.dr, zr[li], yr));
+                    yi = fma2(b.di, zr[li], fma2(b.dr, zi[li], yi));
+                    sr = fma2(b.ei, nzi, fma2(b.er, zr[li], sr));
+                    si = fma2(b.ei, zr[li], fma2(b.er, zi[li], si));
+                }
+                f32x2 xr, xi;
+                lds4(L.mem + M::z + 16u * (uint32_t)(LRN * mi + L.lr), xr, xi);
+                q2 = fma2(xr, yr, fma2(xi, yi, q2));
+                q2 = fma2(swap2(xr), sr, fma2(swap2(xi), si, q2));
+            }
+            const float rho = gsum<G>(lo2(q2) + hi2(q2));
+            sigma = P.shift * fminf(rho, 1.f);
+            // lambda_1 > sigma > 1e-6 + band settles the -7 test; the band by
+            // |M|_F <= sqrt(n) ||inv|C|||_inf (see pixel_solve)
+            const float dM = plink ? 0.f : amb * sqrtf((float)n) * xnorm;
+            if (state == TILE_RUN && !(sigma > thr + dM)) state = TILE_GENERAL;
+            // the padding keeps a unit pivot
+            tile_on_diag<G, NL>(L, [&](int x, int b) {
+                const int i = 2 * (LRN * x + L.lr);
+                A[b].dr = pk(i < n ? lo2(A[b].dr) - sigma : 1.f, i + 1 < n ? hi2(A[b].dr) - sigma : 1.f);
+            });
+        } else {
+            if (__all_sync(0xffffffffu, plink || state != TILE_RUN)) continue;   // phase_link has no such test
+            const float sh = thr + amb * cfro;
+            tile_on_diag<G, NL>(L, [&](int, int b) { A[b].dr = add2(A[b].dr, pk(-sh, -sh)); });
+        }
+        bool ok = true;
+        tile_ldl_seg<G, NL, 0>(A, L, tp, ok);
+        if (state == TILE_RUN && !ok && (pass == 1 || !plink)) state = TILE_GENERAL;
+        if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+        __syncwarp();
+    }
+
+    // ---- inverse iteration (warp_inverse_iteration's rule, pair per lane) -----------
+    f32x2 zr, zi;
+    lds4(L.mem + M::z + 16u * (uint32_t)(L.g < M::T ? L.g : 0), zr, zi);
+    float z0r = lo2(zr), z1r = hi2(zr), z0i = lo2(zi), z1i = hi2(zi);
+    if (L.g >= dp) z0r = z1r = z0i = z1i = 0.f;
+    float2 own[2];
+    tile_own(P, pp, L, state == TILE_RUN, own);
+    const float tol = 1e-5f;
+    float rprev = -1.f, cprev = 1.f, gap_good = 0.f;
+    bool run = state == TILE_RUN;
+    if (run) state = TILE_GENERAL;                    // unless it converges
+#pragma unroll 1
+    for (int it = 0; it < 10 && __any_sync(0xffffffffu, run); ++it) {
+        float x0r = z0r, x1r = z1r, x0i = z0i, x1i = z1i;
+        tile_solve<G, NL>(L, tp, x0r, x1r, x0i, x1i);
+        const float xx = gsum<G>(fmaf(x0r, x0r, x0i * x0i) + fmaf(x1r, x1r, x1i * x1i));
+        const float xv = gsum<G>(fmaf(x0r, z0r, x0i * z0i) + fmaf(x1r, z1r, x1i * z1i));
+        const float dl = xv / xx;                     // rho - sigma
+        const float a0r = fmaf(-dl, x0r, z0r), a0i = fmaf(-dl, x0i, z0i), a1r = fmaf(-dl, x1r, z1r), a1i = fmaf(-dl, x1i, z1i);
+        const float inv = rsqrtf(xx);
+        const float rn = sqrtf(gsum<G>(fmaf(a0r, a0r, a0i * a0i) + fmaf(a1r, a1r, a1i * a1i))) * inv;
+        if (run) {
+            z0r = x0r * inv;
+            z1r = x1r * inv;
+            z0i = x0i * inv;
+            z1i = x1i * inv;
+            if (rprev > 0.f) {
+                const float c = rn / rprev, crate = fmaxf(c, cprev);
+                if (crate < 0.9f) {
+                    const float gap = dl * (1.f / crate - 1.f);
+                    gap_good = gap;
+                    if (rn <= tol * gap) { state = TILE_RUN; run = false; }
+                }
+                if (run && it >= 3 && c > 0.9f) {
+                    if (rn <= 20.f * tol * gap_good) state = TILE_RUN;
+                    run = false;
+                }
+                cprev = c;
+            }
+            rprev = rn;
+        }
+    }
+    if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+
+    tile_finish<G, NL>(P, pp, L, taddr, state == TILE_RUN, false, z0r, z1r, z0i, z1i, own);
+    return state == TILE_RUN ? (int)TILE_DONE : state;
+}
+
+// y = C z for the coherence in A and the vector in shared memory: the row
+// sums of pair LRN x + lr in (yr, yi)[x] on the diagonal lanes
+template <int G, int NL>
+__device__ __forceinline__ void tile_matvec(const CBlk (&A)[Tile<G, NL>::NB], const TileLane &L, f32x2 (&yr)[NL],
+                                            f32x2 (&yi)[NL])
+{
+    using M = Tile<G, NL>;
+    constexpr int RT = M::RT, LRN = M::LRN, NLC = M::NLC;
+    const f32x2 minus = pk(-1.f, -1.f);
+    f32x2 cr[NLC], ci[NLC];
+#pragma unroll
+    for (int x = 0; x < NLC; ++x) cr[x] = ci[x] = 0ull;
+#pragma unroll
+    for (int mi = 0; mi < NL; ++mi) {
+        f32x2 xr, xi, dr = 0ull, di = 0ull, er = 0ull, ei = 0ull;
+        lds4(L.mem + M::z + 16u * (uint32_t)(LRN * mi + L.lr), xr, xi);
+        const f32x2 sr = swap2(xr), si = swap2(xi), nxr = mul2(xr, minus), nsr = swap2(nxr);
+#pragma unroll
+        for (int li = 0; li < RT * (mi + 1); ++li) {
+            const CBlk &b = A[M::blk(mi, li)];
+            f32x2 zr, zi;
+            lds4(L.mem + M::z + 16u * (uint32_t)(4 * li + L.lc), zr, zi);
+            const f32x2 nzi = mul2(zi, minus);
+            dr = fma2(b.di, nzi, fma2(b.dr, zr, dr));
+            di = fma2(b.di, zr, fma2(b.dr, zi, di));
+            er = fma2(b.ei, nzi, fma2(b.er, zr, er));
+            ei = fma2(b.ei, zr, fma2(b.er, zi, ei));
+            if (li < RT * mi) {                          // the mirrored block: conj(C_ij) z_i
+                cr[li] = fma2(b.di, xi, fma2(b.dr, xr, cr[li]));
+                ci[li] = fma2(b.di, nxr, fma2(b.dr, xi, ci[li]));
+                cr[li] = fma2(b.ei, si, fma2(b.er, sr, cr[li]));
+                ci[li] = fma2(b.ei, nsr, fma2(b.er, si, ci[li]));
+            }
+        }
+        yr[mi] = add2(dr, swap2(er));
+        yi[mi] = add2(di, swap2(ei));
+    }
+    tile_row_sums<G, NL>(yr, cr, L);
+    tile_row_sums<G, NL>(yi, ci, L);
+}
+
+// EVD and STBAS (evd.cpp:689-732): the eigenvector of the largest eigenvalue
+// of C.  Power iteration with warp_power's stopping rule; where it contracts
+// slowly (banded coherences do, their eigenvalues cluster), inverse iteration
+// with mu I - C, mu just above the Rayleigh quotient: the factorisation
+// certifies mu > lambda_max, so the iteration converges to that eigenvector, and
+// a shift by the residual converges in a few steps.  Before, such pixels took the
+// Householder reduction: 22.8 -> 5.2 ms at 256 x 384, N = 45, bandwidth 10.
+template <int G, int NL>
+__device__ __forceinline__ int tile_evd(const KParams &P, long long pp, const TileLane &L, uint32_t taddr, bool valid)
+{
+    using M = Tile<G, NL>;
+    constexpr int NB = M::NB, LRN = M::LRN;
+    const int n = P.nb, dp = (n + 1) >> 1;
+    const bool dlane = (L.lr & 3) == L.lc;
+    CBlk A[NB];
+    float cfro = 0.f;
+    int state = tile_begin<G, NL, false>(P, pp, L, taddr, valid, A, cfro);
+    if (!__any_sync(0xffffffffu, state == TILE_RUN)) return state;
+    float2 own[2];
+    tile_own(P, pp, L, state == TILE_RUN, own);
+
+    float rho = 1.f, rn = 0.f, rprev = -1.f, pratio = 1.f;
+    bool run = state == TILE_RUN, slow = false;
+#pragma unroll 1
+    for (int it = 1; it < 96 && __any_sync(0xffffffffu, run); ++it) {
+        f32x2 yr[NL], yi[NL];
+        tile_matvec<G, NL>(A, L, yr, yi);
+        float zy = 0.f, yy = 0.f, rr = 0.f;
+        if (dlane) {
+#pragma unroll
+            for (int x = 0; x < NL; ++x) {
+                f32x2 zr, zi;
+                lds4(L.mem + M::z + 16u * (uint32_t)(LRN * x + L.lr), zr, zi);
+                const f32x2 a = fma2(zr, yr[x], mul2(zi, yi[x])), b = fma2(yr[x], yr[x], mul2(yi[x], yi[x]));
+                zy += lo2(a) + hi2(a);
+                yy += lo2(b) + hi2(b);
+            }
+        }
+        const float q = gsum<G>(zy);                        // z is normalised
+        yy = gsum<G>(yy);
+        if (dlane) {
+#pragma unroll
+            for (int x = 0; x < NL; ++x) {
+                f32x2 zr, zi;
+                lds4(L.mem + M::z + 16u * (uint32_t)(LRN * x + L.lr), zr, zi);
+                const f32x2 nq = pk(-q, -q), a = fma2(zr, nq, yr[x]), b = fma2(zi, nq, yi[x]), c = fma2(a, a, mul2(b, b));
+                rr += lo2(c) + hi2(c);
+            }
+        }
+        const float r = sqrtf(gsum<G>(rr)), inv = rsqrtf(yy);
+        __syncwarp();
+        if (run) {
+            if (dlane) {
+#pragma unroll
+                for (int x = 0; x < NL; ++x)
+                    sts4(L.mem + M::z + 16u * (uint32_t)(LRN * x + L.lr), inv * lo2(yr[x]), inv * hi2(yr[x]),
+                         inv * lo2(yi[x]), inv * hi2(yi[x]));
+            }
+            // eigenvector error ~ rn / gap, the gap about rho (1 - contraction)
+            const float ratio = rprev > 0.f ? fminf(r / rprev, 1.f) : 1.f;
+            rho = q;
+            rn = r;
+            rprev = r;
+            pratio = ratio;
+            if (it >= 2 && r <= 4e-6f * q * fmaxf(1.f - ratio, 0.05f)) run = false;
+            else if (it >= 6 && ratio > 0.8f) { run = false; slow = true; }
+        }
+        __syncwarp();
+    }
+    slow = slow || run;
+    f32x2 vr, vi;
+    lds4(L.mem + M::z + 16u * (uint32_t)(L.g < M::T ? L.g : 0), vr, vi);
+    float z0r = lo2(vr), z1r = hi2(vr), z0i = lo2(vi), z1i = hi2(vi);
+    if (L.g >= dp) z0r = z1r = z0i = z1i = 0.f;
+    if (__any_sync(0xffffffffu, slow)) {
+        if (slow && L.g == 0) atomicAdd(P.slow, 1);
+        const int tp = G == 32 ? dp : max(__shfl_sync(0xffffffffu, dp, 0), __shfl_sync(0xffffffffu, dp, 16));
+        // mu above rho by three times the estimate r^2 / gap of lambda_max - rho,
+        // at most by the residual; the gap from the contraction, dl (1 / c - 1)
+        const float tol = 1e-7f;
+        // (a gap below 0.2% of rho: the reduction to tridiagonal form tells the
+        // eigenvalues apart better)
+        bool hard = false;
+        float gap = -1.f, up = fminf(rn, 3.f * rn * rn / (rho * fmaxf(1.f - pratio, 0.02f)));
+#pragma unroll 1
+        for (int att = 0; att < 6 && __any_sync(0xffffffffu, slow && !hard); ++att) {
+            up = fmaxf(up, 2e-5f * rho);
+            const float mu = rho + up;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                uint32_t w[8];
+                tmem_ld8(taddr + 8u * (uint32_t)b, w);
+                A[b].dr = pk(-__uint_as_float(w[0]), -__uint_as_float(w[1]));
+                A[b].di = pk(-__uint_as_float(w[2]), -__uint_as_float(w[3]));
+                A[b].er = pk(-__uint_as_float(w[4]), -__uint_as_float(w[5]));
+                A[b].ei = pk(-__uint_as_float(w[6]), -__uint_as_float(w[7]));
+            }
+            tile_on_diag<G, NL>(L, [&](int x, int b) {
+                const int i = 2 * (LRN * x + L.lr);
+                A[b].dr = pk(i < n ? mu - 1.f : 1.f, i + 1 < n ? mu - 1.f : 1.f);
+            });
+            bool ok = true;
+            tile_ldl_seg<G, NL, 0>(A, L, tp, ok);
+            __syncwarp();
+            if (!ok) up *= 8.f;                             // mu was below lambda_max
+            bool act = slow && ok && !hard;
+            float rp = -1.f;
+#pragma unroll 1
+            for (int it = 0; it < 6 && __any_sync(0xffffffffu, act); ++it) {
+                float x0r = z0r, x1r = z1r, x0i = z0i, x1i = z1i;
+                tile_solve<G, NL>(L, tp, x0r, x1r, x0i, x1i);
+                const float xx = gsum<G>(fmaf(x0r, x0r, x0i * x0i) + fmaf(x1r, x1r, x1i * x1i));
+                const float xv = gsum<G>(fmaf(x0r, z0r, x0i * z0i) + fmaf(x1r, z1r, x1i * z1i));
+                const float dl = xv / xx;                   // mu - rho
+                const float a0r = fmaf(-dl, x0r, z0r), a0i = fmaf(-dl, x0i, z0i), a1r = fmaf(-dl, x1r, z1r),
+                            a1i = fmaf(-dl, x1i, z1i);
+                const float inv = rsqrtf(xx);
+                const float r = sqrtf(gsum<G>(fmaf(a0r, a0r, a0i * a0i) + fmaf(a1r, a1r, a1i * a1i))) * inv;
+                if (act) {
+                    z0r = x0r * inv;
+                    z1r = x1r * inv;
+                    z0i = x0i * inv;
+                    z1i = x1i * inv;
+                    rho = mu - dl;
+                    if (rp > 0.f) {
+                        // the gap by this contraction, unless rounding ended it; the
+                        // smallest one seen counts, early contractions being the faster ones
+                        const float c = r / rp;
+                        const bool floor_ = r <= 1e-6f * dl;
+                        if (c < 0.95f && !floor_) {
+                            const float gn = dl * (1.f / c - 1.f);
+                            gap = gap > 0.f ? fminf(gap, gn) : gn;
+                        }
+                        if (it >= (att > 0 ? 1 : 2) && (r <= tol * gap || (floor_ && !(gap < dl && gap > 0.f)))) { slow = false; act = false; }
+                        else if (c > 0.25f) act = false;    // a closer shift
+                        if (gap > 0.f && gap < 2e-3f * rho) hard = true;
+                    }
+                    rp = r;
+                    up = gap > 0.f ? fminf(r, 3.f * r * r / gap) : r;
+                }
+            }
+        }
+        if (state == TILE_RUN && (slow || hard)) state = TILE_GENERAL;
+    }
+    tile_finish<G, NL>(P, pp, L, taddr, state == TILE_RUN, P.method == M_STBAS, z0r, z1r, z0i, z1i, own);
+    return state == TILE_RUN ? (int)TILE_DONE : state;
+}
 // L2 prefetch of a pixel's Gamma record by the lanes of its group
 template <int G> __device__ __forceinline__ void tile_prefetch(const KParams &P, long long pp, int g)
 {

@@ -43,8 +43,10 @@ enum fpl_semantics {         /* which reference module's loop is mirrored */
 };
 
 enum fpl_precision {
-    FPL_PREC_FP32 = 0,       /* plain FP32 form (FP64 only to settle ambiguous decisions) */
-    FPL_PREC_MIXED = 1       /* BF16 split-precision tensor-core coherence matrix */
+    FPL_PREC_FP32 = 0,       /* FP32 form (FP64 only to settle ambiguous decisions): products in
+                              * FP32, summed in FP32 -- on the tensor cores as three exact BF16
+                              * parts, or by the plain kernel where the window is too large */
+    FPL_PREC_MIXED = 1       /* coherence sums of products in two BF16 parts */
 };
 
 enum fpl_memory {
@@ -153,18 +155,18 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out);
 
 /* ---- batches of jobs ------------------------------------------------------
  * Many device-memory jobs -- scenes or ministacks of different size, stack
- * depth, window and method -- run as one persistent launch per padded depth
- * (16 / 32 / 64 dates), with warps taking pixels dynamically across jobs,
- * followed by one FP64 settle launch.  Replaces running the evd module once
+ * depth, window and method -- run as waves of persistent launches, followed by
+ * one FP64 settle launch per padded depth (16 / 32 / 64 dates).  Replaces running the evd module once
  * per ministack (src/sequential/sequential.py:193-254 calls evd_process in a
  * loop).  FPL_BATCH_GRAPH captures the launch sequence into a CUDA graph at
  * creation; fpl_batch_run replays it (buffers are fixed, their contents may
  * change between runs).  FPL_BATCH_AUTOTUNE times candidate CTA shapes on
  * the batch at creation and caches the fastest per (form, depth, window,
- * mean SHP count) in the context.  Jobs with precision FPL_PREC_MIXED run
- * the mixed form: cut into row pieces, packed into waves of <= 2^20 pixels,
- * one tensor-core Gamma launch over the tiles and one solve launch over the
- * pixels of each wave. */
+ * mean SHP count) in the context.  Jobs are cut into row pieces, packed into
+ * waves of <= 2^20 pixels (fewer where device memory is short), with one
+ * tensor-core Gamma launch over the tiles and one solve launch per padded depth
+ * and kind of method over the pixels of each wave.  Jobs whose window the Gamma
+ * kernel does not take run one persistent plain FP32 launch per padded depth. */
 #define FPL_BATCH_GRAPH 1
 #define FPL_BATCH_AUTOTUNE 2
 typedef struct fpl_batch fpl_batch;
@@ -207,8 +209,8 @@ int fpl_server_destroy(fpl_server *srv);
  * For callers that cannot call cudaMalloc -- an application whose device
  * memory belongs to another allocator, or a service that must not allocate
  * after start-up.  Same job and results as fpl_run_async on device buffers
- * in the plain FP32 form (a job asking for the mixed form runs the FP32 form
- * here: the mixed form's coherence records need gigabytes of scratch), on
+ * by the plain FP32 kernel (so does a job asking for the mixed form
+ * here: the Gamma records of the other entry points need gigabytes of scratch), on
  * the current CUDA device, but no context is needed and nothing is
  * allocated: the kernels' scratch is a fixed array inside the library, held
  * by every GPU that loads it until the process exits.  Every call looks up
@@ -249,8 +251,8 @@ int fpl_ctx_profile(fpl_ctx *ctx, double *fp32_ms, double *fp64_ms, int *runs);
  * FPL_KTAG_FP32 + FPL_KTAG_GRAM + FPL_KTAG_SOLVE, the FP64 one FPL_KTAG_FP64). */
 enum fpl_kernel_tag {
     FPL_KTAG_FP32 = 0,       /* plain FP32 pixel kernel (gather + Gamma + solve) */
-    FPL_KTAG_GRAM = 1,       /* mixed form: tensor-core Gamma records            */
-    FPL_KTAG_SOLVE = 2,      /* mixed form: eigen-solves from the records        */
+    FPL_KTAG_GRAM = 1,       /* tensor-core Gamma records                        */
+    FPL_KTAG_SOLVE = 2,      /* eigen-solves from the records                    */
     FPL_KTAG_FP64 = 3,       /* FP64 settle pass                                 */
     FPL_KTAG_COUNT = 4
 };

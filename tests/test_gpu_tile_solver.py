@@ -47,3 +47,22 @@ def test_every_outcome_beside_another(gpu_lib, n):
         g = phase_link(stack, nmap, (4, 8), semantics=semantics, precision="mixed")
         o = oracle.run(stack, nmap, 4, 8, semantics=semantics)
         assert_parity(compare(g, o), phase_tol=1e-3, tcorr_tol=2e-4)
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 8, 15, 16, 17, 24, 25, 31, 32, 33, 45, 48, 49, 64])
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+def test_evd_and_stbas(gpu_lib, n, precision):
+    """Largest eigenvectors: power iteration, and the shifted inverse
+    iteration that banded coherences need."""
+    from fringe_gb300 import phase_link
+    stack, nmap = synth.scene("voronoi", 11, 19, n, 6, 7, seed=300 + n)
+    runs = [dict(method="EVD")]
+    if n >= 4:
+        runs += [dict(method="STBAS", band_width=b) for b in sorted({1, n // 3 + 1, n - 2})]
+        runs += [dict(method="STBAS", band_width=2, semantics="phase_link", mini_stack_count=2)]
+    for kw in runs:
+        g = phase_link(stack, nmap, (6, 7), precision=precision, **kw)
+        o = oracle.run(stack, nmap, 6, 7, **kw)
+        m = compare(g, o)
+        assert m["valid_both"] > 100, (kw, m)
+        assert_parity(m, phase_tol=1e-3, tcorr_tol=2e-4)

@@ -47,7 +47,7 @@ __global__ void k_pixels(KParams P)
     } else {
         int cnt = *((volatile int *)P.fb_count);
         cnt = cnt < P.fb_cap ? cnt : P.fb_cap;
-        for (long long q = fb_next(P, lane); q < cnt; q = fb_next(P, lane))
+        for (long long q = list_first(); q < cnt; q = fb_next(P, lane))
             process_pixel<T, NP>(P, P.fb_list[q], sm, lane, taddr);
     }
     if constexpr (CInTmem<T, NP>::value || CRowsTmemF<T, NP>::value) tmem_free_cta(tbase, warp, (uint32_t)tcols);
@@ -152,7 +152,7 @@ __device__ __forceinline__ void rest_loop(const KParams &P, unsigned char *sm, i
     C2<float> *A = reinterpret_cast<C2<float> *>(sm + Lay<float, NP>::wm);
     const bool listed = tile_kind(P) != TK_REST;
     const long long cnt = listed ? *((volatile int *)(P.fb_count + 1)) : P.npix;
-    for (long long q = rest_next(P, lane); q < cnt; q = rest_next(P, lane)) {
+    for (long long q = list_first(); q < cnt; q = rest_next(P, lane)) {
         const long long pp = P.cbase + (listed ? (long long)P.rest[q] : q);
         if constexpr (NP <= 32) {
             const int npix = pixel_load_gamma<NP, false>(P, pp, sm, lane, A);

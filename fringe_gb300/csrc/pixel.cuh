@@ -1369,15 +1369,19 @@ __device__ __forceinline__ void acc_prod<double>(C2<double> &acc, float2 a, floa
     acc.y += double(im);
 }
 
-// next entry of the FP64 work list for this warp: warps draw entries from a
-// cursor in the run's counter block (zeroed with it), so the SMs whose
-// pixels were cheap take more of them
-__device__ __forceinline__ long long fb_next(const KParams &P, int lane)
+// Entries of a work list for this warp: the first is dealt out, CTA by CTA (a
+// short list then has one entry per SM: drawn from the cursor from the start, 15 pixels
+// all went to the first CTA's warps, which share the SM's FP64 pipe), further
+// ones are drawn from a cursor in the run's counter block (zeroed with it), so the SMs
+// whose pixels were cheap take more of them.
+__device__ __forceinline__ long long list_first() { return blockIdx.x + (long long)gridDim.x * (threadIdx.x >> 5); }
+__device__ __forceinline__ long long list_next(int *cursor, int lane)
 {
     int q = 0;
-    if (lane == 0) q = atomicAdd(P.fb_count + 12, 1);
-    return __shfl_sync(0xffffffffu, q, 0);
+    if (lane == 0) q = atomicAdd(cursor, 1);
+    return (long long)gridDim.x * (blockDim.x >> 5) + __shfl_sync(0xffffffffu, q, 0);
 }
+__device__ __forceinline__ long long fb_next(const KParams &P, int lane) { return list_next(P.fb_count + 12, lane); }
 
 __device__ __forceinline__ void defer_fp64(const KParams &P, long long pp, int lane)
 {
@@ -1396,18 +1400,12 @@ __device__ __forceinline__ void put_code(const KParams &P, long long pp, int lan
     }
 }
 
-// the rest list of a chunk: appended to by the register solve, drawn from by
-// warps of k_rest
+// the rest list of a chunk: appended to by the register solve, read by k_rest
 __device__ __forceinline__ void rest_put(const KParams &P, long long pp)
 {
     P.rest[atomicAdd(P.fb_count + 1, 1)] = int(pp - P.cbase);
 }
-__device__ __forceinline__ int rest_next(const KParams &P, int lane)
-{
-    int q = 0;
-    if (lane == 0) q = atomicAdd(P.fb_count + 13, 1);
-    return __shfl_sync(0xffffffffu, q, 0);
-}
+__device__ __forceinline__ long long rest_next(const KParams &P, int lane) { return list_next(P.fb_count + 13, lane); }
 
 // Gather, Gamma and coherence (evd.cpp:514-582).  Returns the SHP count
 // with C in the warp's slab, or -1 when the pixel is finished (skipped or

@@ -48,6 +48,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "pixel.cuh"
 
@@ -83,7 +84,7 @@ template <int KC, int NS> struct BoxLay {
     static constexpr int B_BYTES = (PCOL / 8) * SBO;         // one part
     static constexpr int STAGE = A_BYTES + NS * B_BYTES;
     static constexpr int MAXPAIR = 32;                       // date pairs: 64 dates
-    static constexpr int XRS = KC * 16 + 16;                 // bytes per date-pair row of X
+    static constexpr int XRS = KC * 16 + 16;                 // bytes per date pair of X (see put)
     static constexpr int X_BYTES = MAXPAIR * XRS;            // one of two sample buffers
     static constexpr size_t OFF_MISC = 0;
     static constexpr size_t OFF_LUT = OFF_MISC + BX_MISC;          // 256 x 8 bf16 mask patterns
@@ -190,22 +191,23 @@ __device__ __forceinline__ bool split_range(float v)
     return v == 0.f || (a >= 8.8817842e-16f && a <= 1.1258999e15f);
 }
 
-// 8 values of one Gamma column into NS bf16 rows (16 bytes each, pstride
-// apart): each part rounds what the parts before it left (exact differences)
+// 8 values of one Gamma column (as pairs) into NS bf16 rows (16 bytes each,
+// pstride apart): each part rounds what the parts before it left (exact
+// differences)
 template <int NS>
-__device__ __forceinline__ void store_split(unsigned char *dst, uint32_t pstride, const float *v)
+__device__ __forceinline__ void store_split(unsigned char *dst, uint32_t pstride, const f32x2 (&v)[4])
 {
     uint32_t p[NS][4];
+    const f32x2 minus = pk(-1.f, -1.f);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        float a = v[2 * q], b = v[2 * q + 1];
+        f32x2 a = v[q];
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+            const __nv_bfloat162 t = __floats2bfloat162_rn(lo2(a), hi2(a));
             const uint32_t u = *reinterpret_cast<const uint32_t *>(&t);
             p[s][q] = u;
-            a -= __uint_as_float(u << 16);
-            b -= __uint_as_float(u & 0xffff0000u);
+            if (s + 1 < NS) a = fma2(pk(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)), minus, a);
         }
     }
 #pragma unroll
@@ -342,7 +344,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     }
     // (the prologue's barrier orders these before any use)
 
-    // samples of chunk k0 (date pairs interleaved): each thread loads one
+    // samples of chunk k0: each thread loads one
     // sample for up to BX_XPT dates into registers (64 dates over the CTA);
     // put() stores them in one of two sample buffers (chunk g in buffer
     // g & 1) and flags samples outside the split range in tbad.  The loads
@@ -395,7 +397,11 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
                 xbad = true;
                 x = make_float2(0.f, 0.f);
             }
-            *reinterpret_cast<float2 *>(xd + (d >> 1) * L::XRS + sidx * 16 + (d & 1) * 8) = x;
+            // per date pair: Re and Im of the first date, then of the second,
+            // KC samples each (the build reads runs of samples)
+            float *xp = reinterpret_cast<float *>(xd + (d >> 1) * L::XRS + (d & 1) * (8 * KC)) + sidx;
+            xp[0] = x.x;
+            xp[KC] = x.y;
         }
         if (xbad) atomicOr(tbad + ((k0 + sidx) >> 5), 1u << ((k0 + sidx) & 31));
     };
@@ -419,6 +425,22 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
             const int nc = min(BX_NCOL, ncol - j * BX_NCOL);
             nmma[j] = nc > 0 ? (nc + 15) & ~15 : 0;
             idesc[j] = make_idesc(nmma[j] > 0 ? nmma[j] : 16);
+        }
+        // this thread's share of the B build, the same in every chunk: block bl's
+        // rows 4 ia .. 4 ia + 3 (entries (2a + ia, 2b), (2a + ia, 2b + 1), Re and Im)
+        // over the 8 samples of K group k8; zero: columns that pad the last MMA to 16
+        constexpr int K8 = KC / 8;
+        static_assert(2 * (L::PCOL / 8) * K8 <= BX_THREADS, "one item per thread");
+        const int nb8 = (ncol + 15) / 16 * 2;
+        int it_off = -1, it_a = 0, it_b = 0;
+        bool it_zero = false;
+        if (tid < 2 * nb8 * K8) {
+            const int r8 = tid / nb8, bl = tid - r8 * nb8, ia = r8 & 1, k8 = r8 >> 1;
+            it_off = bl * L::SBO + k8 * 128 + ia * 64;
+            it_zero = bl * 8 >= ncol;
+            const short2 ab = blk[cb / 8 + (it_zero ? 0 : bl)];
+            it_a = ab.x * L::XRS + ia * (8 * KC) + k8 * 32;
+            it_b = ab.y * L::XRS + k8 * 32;
         }
         for (int ch = 0; ch < nchunk; ++ch) {
             const int s = st.gstep & 1;
@@ -447,45 +469,39 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
                 *reinterpret_cast<uint4 *>(As + (m >> 3) * L::SBO + k8 * 128 + (m & 7) * 16) = lut[bits];
             }
             // ---- B: outer-product entries, NS parts ----
-            // one thread per half core matrix: block bl's rows 4 ia .. 4 ia + 3
-            // (entries (2a + ia, 2b), (2a + ia, 2b + 1), Re and Im) over the 8
-            // samples of K group k8
-            constexpr int NBL = L::PCOL / 8;                 // column blocks of the pass
-            for (int e = late ? 2 * NBL * (KC / 8) : tid; e < 2 * NBL * (KC / 8); e += BX_THREADS) {
-                const int bl = e % NBL, ia = (e / NBL) & 1, k8 = e / (2 * NBL);
-                const int jacc = bl / (BX_NCOL / 8);
-                const int nm_j = (jacc == 0) ? nmma[0] : nmma[L::NACC - 1];
-                if ((bl - jacc * (BX_NCOL / 8)) * 8 >= nm_j) continue;          // read by no MMA
-                unsigned char *db = Bs + bl * L::SBO + k8 * 128 + ia * 64;
-                if (bl * 8 >= ncol) {
+            // two samples per packed operation; the products round as
+            // fma(xr, yr, xi yi) and fma(xi, yr, -(xr yi))
+            if (it_off >= 0 && !late) {
+                unsigned char *db = Bs + it_off;
+                if (it_zero) {
                     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
 #pragma unroll
                         for (int p = 0; p < NS; ++p) *reinterpret_cast<uint4 *>(db + p * L::B_BYTES + c * 16) = z;
-                    continue;
-                }
-                const short2 ab = blk[cb / 8 + bl];
-                const unsigned char *sa = Xc + ab.x * L::XRS + k8 * 128;
-                const unsigned char *sb = Xc + ab.y * L::XRS + k8 * 128;
-                float2 pa[8];          // per sample: x_{2a + ia}
-                float4 pb[8];          // per sample: x_{2b}, x_{2b+1}
+                } else {
+                    auto run8 = [](const unsigned char *src, f32x2 (&v)[4]) {
+                        const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(src);
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(src + 16);
+                        v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
+                    };
+                    f32x2 xr[4], xi[4], nxr[4];
+                    run8(Xc + it_a, xr);
+                    run8(Xc + it_a + 4 * KC, xi);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) pa[q] = *reinterpret_cast<const float2 *>(sa + q * 16 + ia * 8);
+                    for (int q = 0; q < 4; ++q) nxr[q] = xr[q] ^ 0x8000000080000000ull;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) pb[q] = *reinterpret_cast<const float4 *>(sb + q * 16);
+                    for (int jb = 0; jb < 2; ++jb) {           // i = 2a + ia, j = 2b + jb
+                        f32x2 yr[4], yi[4], v[4];
+                        run8(Xc + it_b + jb * (8 * KC), yr);
+                        run8(Xc + it_b + jb * (8 * KC) + 4 * KC, yi);
 #pragma unroll
-                for (int jb = 0; jb < 2; ++jb) {           // i = 2a + ia, j = 2b + jb
-                    float re[8], im[8];
+                        for (int q = 0; q < 4; ++q) v[q] = fma2(xr[q], yr[q], mul2(xi[q], yi[q]));       // Re x_i conj(x_j)
+                        store_split<NS>(db + (2 * jb) * 16, L::B_BYTES, v);
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float xr = pa[q].x, xi = pa[q].y;
-                        const float yr = jb ? pb[q].z : pb[q].x, yi = jb ? pb[q].w : pb[q].y;
-                        re[q] = fmaf(xr, yr, xi * yi);          // Re x_i conj(x_j)
-                        im[q] = fmaf(xi, yr, -(xr * yi));       // Im x_i conj(x_j)
+                        for (int q = 0; q < 4; ++q) v[q] = fma2(xi[q], yr[q], mul2(nxr[q], yi[q]));      // Im x_i conj(x_j)
+                        store_split<NS>(db + (2 * jb + 1) * 16, L::B_BYTES, v);
                     }
-                    store_split<NS>(db + (2 * jb) * 16, L::B_BYTES, re);
-                    store_split<NS>(db + (2 * jb + 1) * 16, L::B_BYTES, im);
                 }
             }
             // the next chunk's samples go to the other buffer, which the

@@ -55,7 +55,10 @@
 namespace fpl {
 namespace {
 
-constexpr int BX_THREADS = 512;                    // 16 warps: the operand build hides latency
+// 16 warps in two groups of 8 that take alternate chunks: their loads,
+// arithmetic and stores overlap (in step on one chunk, the phases followed one
+// another)
+constexpr int BX_THREADS = 512, BX_GRP = 256;
 constexpr int BX_TR = 8, BX_TC = 16, BX_M = 128;   // pixel tile (MMA M)
 constexpr int BX_NCOL = 256;                       // Gamma columns per accumulator (MMA N)
 // samples per chunk (MMA K of one stage): 32, so that two accumulators (512
@@ -214,27 +217,51 @@ __device__ __forceinline__ void store_split(unsigned char *dst, uint32_t pstride
     for (int s = 0; s < NS; ++s) *reinterpret_cast<uint4 *>(dst + s * pstride) = make_uint4(p[s][0], p[s][1], p[s][2], p[s][3]);
 }
 
-// pipeline state of a CTA, carried from tile to tile (and job to job)
+// pipeline state of a CTA, carried from tile to tile (and job to job).  Step n
+// (a chunk) uses operand stage n & 1 and is built by group n & 1; its k-th use
+// of the stage (k = n >> 1) completes phase k of the stage's two barriers: full
+// (built, an arrival per thread of the group) and empty (its MMAs are done).
 struct BoxPipe {
-    uint32_t pend;      // per stage: MMAs in flight
-    uint32_t par;       // per stage: mbarrier parity
-    unsigned gstep;     // chunks issued
+    unsigned base;      // steps before this tile
+    unsigned issued;    // one past the last step whose MMAs this thread issued
     bool timed_out;
     int blk_dp;         // date pairs the block table was built for
 };
+struct BoxBars {
+    uint64_t full[2], empty[2];
+    uint32_t tmem_slot;
+    int dead;           // a wait gave up: the others stop waiting
+};
 
-// this thread's wait for the MMAs of stage s (if any are pending); true if
-// the wait gave up.  Every thread polls the barrier itself, so no CTA
-// barrier is needed before the stage is overwritten.
-__device__ __forceinline__ bool box_poll(uint64_t *mbar, BoxPipe &st, int s)
+// bounded wait for step n on a pair of barriers; true if it gave up (or
+// another wait had)
+__device__ __forceinline__ bool box_wait(uint64_t *pair, unsigned n, volatile int *dead)
 {
-    if (!(st.pend & (1u << s))) return false;
     long long spins = 0;
-    while (!mbar_try_wait(&mbar[s], (st.par >> s) & 1u))
-        if (++spins > BX_SPIN_LIMIT) return true;
-    st.par ^= 1u << s;
-    st.pend &= ~(1u << s);
+    while (!mbar_try_wait(&pair[n & 1], (n >> 1) & 1u)) {
+        if (*dead || ++spins > BX_SPIN_LIMIT) {
+            *dead = 1;
+            return true;
+        }
+    }
     return false;
+}
+
+// barrier of a group's threads; true if any of them passes true
+__device__ __forceinline__ bool group_or(int grp, bool v)
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)v), "r"(1 + grp), "n"(BX_GRP) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void group_sync(int grp)
+{
+    asm volatile("barrier.cta.sync %0, %1;" :: "r"(1 + grp), "n"(BX_GRP) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_addr(mbar)) : "memory");
 }
 
 // tiles of the rows [ra, rb) of a launch: 8-row tiles on the absolute grid
@@ -258,7 +285,8 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     unsigned char *stages = smem + L::OFF_ST;
     unsigned char *Xb = smem + L::OFF_X;
     unsigned char *misc = smem + L::OFF_MISC;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(misc);                 // 2 stages
+    BoxBars *bars = reinterpret_cast<BoxBars *>(misc);
+    volatile int *dead = &bars->dead;
     int *pinfo = reinterpret_cast<int *>(misc + 64);                     // 128
     int *pdefer = reinterpret_cast<int *>(misc + 64 + 512);              // 128
     short2 *blk = reinterpret_cast<short2 *>(misc + 64 + 1024);          // <= 528 blocks
@@ -280,6 +308,52 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     const int min_neigh = (P.semantics == SEM_PL) ? P.min_neigh : 2;   // evd.cpp:566
     const long long plane = P.plane;
     const int R0 = box_first_row(P) + int(t / ntc) * BX_TR, C0 = int(t % ntc) * BX_TC;
+    const int grp = (tid / BX_GRP) & 1, gt = tid % BX_GRP;      // group and thread of it
+
+    // samples of a chunk: each thread of the group that builds it loads one
+    // sample for up to BX_XPT dates into registers (64 dates over the group), a
+    // whole step of the other group ahead; put() stores them in the group's sample buffer and
+    // flags samples outside the split range in tbad
+    constexpr int BX_XPT = 2 * L::MAXPAIR * KC / BX_GRP;
+    static_assert(BX_XPT >= 1 && BX_XPT * (BX_GRP / KC) == 2 * L::MAXPAIR, "date coverage");
+    const int sidx = gt % KC, d0 = gt / KC;
+    const int gtot = npass * nchunk;
+    const int g0 = (grp - (int)(st.base & 1)) & 1;              // the group's first step of the tile
+    float2 xv[BX_XPT];
+    // a group's chunks advance by two, cyclically over the tile: the union row
+    // and column of this thread's next sample advance by 2 KC, with a division
+    // only at the start (of chunks 0 and 1)
+    int us[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        us[h][0] = (h * KC + sidx) / uwp;
+        us[h][1] = h * KC + sidx - us[h][0] * uwp;
+    }
+    int fch = (nchunk > 1) ? g0 : 0, fur = fch ? us[1][0] : us[0][0], fuc = fch ? us[1][1] : us[0][1];
+    const float2 *sbase = P.stack + (long long)d0 * plane;
+    auto fetch = [&]() {
+        const int r = R0 - P.ny + fur, c = C0 - P.nx + fuc;
+        const bool valid = fur < uh && r >= 0 && r < rows && c >= 0 && c < cols;
+        const float2 *src = sbase + (valid ? (long long)r * cols + c : 0ll);
+#pragma unroll
+        for (int q = 0; q < BX_XPT; ++q) {
+            const int d = d0 + q * (BX_GRP / KC);
+            float2 x = make_float2(0.f, 0.f);
+            if (valid && d < n) x = __ldg(src + (long long)(q * (BX_GRP / KC)) * plane);
+            xv[q] = x;
+        }
+        fch += 2;
+        if (fch >= nchunk) {
+            fch -= nchunk;
+            if (fch >= nchunk) fch -= nchunk;
+            fur = fch ? us[1][0] : us[0][0];
+            fuc = fch ? us[1][1] : us[0][1];
+        } else {
+            fuc += 2 * KC;
+            while (fuc >= uwp) { fuc -= uwp; ++fur; }
+        }
+    };
+    if (g0 < gtot) fetch();
 
     // Gamma column blocks (a, b), a <= b, of this stack depth
     if (st.blk_dp != dp) {
@@ -342,55 +416,14 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         }
         pinfo[m] = info;
     }
-    // (the prologue's barrier orders these before any use)
-
-    // samples of chunk k0: each thread loads one
-    // sample for up to BX_XPT dates into registers (64 dates over the CTA);
-    // put() stores them in one of two sample buffers (chunk g in buffer
-    // g & 1) and flags samples outside the split range in tbad.  The loads
-    // run two chunks ahead of the build: chunk c waits in xa (c even) or xb
-    // (c odd), chosen by a branch so both stay in registers, and no copy
-    // between them waits for loads in flight.
-    constexpr int BX_XPT = 2 * L::MAXPAIR * KC / BX_THREADS;
-    static_assert(BX_XPT >= 1 && BX_XPT * (BX_THREADS / KC) == 2 * L::MAXPAIR, "date coverage");
-    const int sidx = tid % KC, d0 = tid / KC;
-    float2 xa[BX_XPT], xb[BX_XPT];
-    // chunks are loaded in cyclic order (0, 1, .., nchunk - 1, 0, ..): the
-    // union row and column of this thread's next sample advance by KC
-    // (< 3 union rows of >= 16 samples) and return to the start after the
-    // last chunk, with no division per chunk
-    const int ur0 = sidx / uwp, uc0 = sidx - ur0 * uwp;
-    int fur = ur0, fuc = uc0, fch = 0;
-    const float2 *sbase = P.stack + (long long)d0 * plane;
-    auto fetch = [&](float2 (&xo)[BX_XPT]) {
-        const int r = R0 - P.ny + fur, c = C0 - P.nx + fuc;
-        const bool valid = fur < uh && r >= 0 && r < rows && c >= 0 && c < cols;
-        const float2 *src = sbase + (valid ? (long long)r * cols + c : 0ll);
-#pragma unroll
-        for (int q = 0; q < BX_XPT; ++q) {
-            const int d = d0 + q * (BX_THREADS / KC);
-            float2 x = make_float2(0.f, 0.f);
-            if (valid && d < n) x = __ldg(src + (long long)(q * (BX_THREADS / KC)) * plane);
-            xo[q] = x;
-        }
-        if (++fch == nchunk) {
-            fch = 0;
-            fur = ur0;
-            fuc = uc0;
-        } else {
-            fuc += KC;
-            if (fuc >= uwp) { fuc -= uwp; ++fur; }
-            if (fuc >= uwp) { fuc -= uwp; ++fur; }
-        }
-    };
     // range checks: always in the first pass; in later passes only if the
     // first found an out-of-range sample in the tile (clean: it found none)
     bool clean = false;
-    auto put = [&](unsigned char *xd, int k0, const float2 (&xv)[BX_XPT]) {
+    auto put = [&](unsigned char *xd, int k0) {
         bool xbad = false;
 #pragma unroll
         for (int q = 0; q < BX_XPT; ++q) {
-            const int d = d0 + q * (BX_THREADS / KC);
+            const int d = d0 + q * (BX_GRP / KC);
             if (d >= 2 * dp) break;
             float2 x = xv[q];
             if (!clean && (!split_range(x.x) || !split_range(x.y))) {
@@ -405,13 +438,6 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         }
         if (xbad) atomicOr(tbad + ((k0 + sidx) >> 5), 1u << ((k0 + sidx) & 31));
     };
-    static_assert(KC <= 2 * BX_TC, "a chunk advances at most two union rows");
-    // prologue: the first chunk of the tile into buffer 0, the second one
-    // into xb
-    const int gtot = npass * nchunk;
-    fetch(xa);
-    put(Xb, 0, xa);
-    if (gtot > 1) fetch(xb);
     __syncthreads();
 
     for (int pass = 0; pass < npass && !st.timed_out; ++pass) {
@@ -426,75 +452,83 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
             nmma[j] = nc > 0 ? (nc + 15) & ~15 : 0;
             idesc[j] = make_idesc(nmma[j] > 0 ? nmma[j] : 16);
         }
-        // this thread's share of the B build, the same in every chunk: block bl's
-        // rows 4 ia .. 4 ia + 3 (entries (2a + ia, 2b), (2a + ia, 2b + 1), Re and Im)
-        // over the 8 samples of K group k8; zero: columns that pad the last MMA to 16
-        constexpr int K8 = KC / 8;
-        static_assert(2 * (L::PCOL / 8) * K8 <= BX_THREADS, "one item per thread");
-        const int nb8 = (ncol + 15) / 16 * 2;
-        int it_off = -1, it_a = 0, it_b = 0;
-        bool it_zero = false;
-        if (tid < 2 * nb8 * K8) {
-            const int r8 = tid / nb8, bl = tid - r8 * nb8, ia = r8 & 1, k8 = r8 >> 1;
-            it_off = bl * L::SBO + k8 * 128 + ia * 64;
-            it_zero = bl * 8 >= ncol;
-            const short2 ab = blk[cb / 8 + (it_zero ? 0 : bl)];
-            it_a = ab.x * L::XRS + ia * (8 * KC) + k8 * 32;
-            it_b = ab.y * L::XRS + k8 * 32;
-        }
-        for (int ch = 0; ch < nchunk; ++ch) {
-            const int s = st.gstep & 1;
-            // the stage's previous MMAs (two chunks back) must be done
-            // before it is overwritten; a thread whose wait gave up builds
-            // nothing and the vote below stops the CTA
-            const bool late = box_poll(mbar, st, s);
-            unsigned char *As = stages + s * L::STAGE;
-            unsigned char *Bs = As + L::A_BYTES;
-            const int k0 = ch * KC;
-            // chunk g + 1 (the first chunk again after the last one of a
-            // pass) is in registers; chunk g + 2 is loaded while this one
-            // is built, into the array chunk g left
-            const int g = pass * nchunk + ch;
-            const bool more = g + 1 < gtot;
-            const unsigned char *Xc = Xb + (g & 1) * L::X_BYTES;
-            if (g + 2 < gtot) {
-                if (g & 1) fetch(xb);
-                else fetch(xa);
-            }
-            // ---- A: SHP mask rows ----
-            for (int e = late ? BX_M * (KC / 8) : tid; e < BX_M * (KC / 8); e += BX_THREADS) {
-                const int m = e & (BX_M - 1), k8 = e >> 7;
-                const int b0 = k0 + k8 * 8;
-                const uint32_t bits = (umask[m * W + (b0 >> 5)] >> (b0 & 31)) & 0xffu;
-                *reinterpret_cast<uint4 *>(As + (m >> 3) * L::SBO + k8 * 128 + (m & 7) * 16) = lut[bits];
-            }
-            // ---- B: outer-product entries, NS parts ----
-            // two samples per packed operation; the products round as
-            // fma(xr, yr, xi yi) and fma(xi, yr, -(xr yi))
-            if (it_off >= 0 && !late) {
-                unsigned char *db = Bs + it_off;
-                if (it_zero) {
-                    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+        bool late = false;
+        {
+            // this thread's share of the B build, the same in every chunk of the pass:
+            // block bl's rows 4 ia .. 4 ia + 3 (entries (2a + ia, 2b), (2a + ia, 2b + 1), Re
+            // and Im) over the 8 samples of K group k8; off < 0: none; zero: columns
+            // that pad the last MMA to 16
+            constexpr int K8 = KC / 8, NIT = 2;
+            static_assert(2 * (L::PCOL / 8) * K8 <= NIT * BX_GRP, "items of a chunk");
+            const int nb8 = (ncol + 15) / 16 * 2;
+            int it_off[NIT], it_a[NIT], it_b[NIT];
+            bool it_zero[NIT];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+            for (int i = 0; i < NIT; ++i) {
+                const int e = gt + i * BX_GRP;
+                it_off[i] = -1;
+                it_a[i] = it_b[i] = 0;
+                it_zero[i] = false;
+                if (e < 2 * nb8 * K8) {
+                    const int r8 = e / nb8, bl = e - r8 * nb8, ia = r8 & 1, k8 = r8 >> 1;
+                    it_off[i] = bl * L::SBO + k8 * 128 + ia * 64;
+                    it_zero[i] = bl * 8 >= ncol;
+                    const short2 ab = blk[cb / 8 + (it_zero[i] ? 0 : bl)];
+                    it_a[i] = ab.x * L::XRS + ia * (8 * KC) + k8 * 32;
+                    it_b[i] = ab.y * L::XRS + k8 * 32;
+                }
+            }
+            unsigned char *As = stages + grp * L::STAGE, *Bs = As + L::A_BYTES;
+            unsigned char *X = Xb + grp * L::X_BYTES;
+            int ch = (g0 - pass * nchunk) & 1;                  // the group's first chunk of the pass
+            for (int g = pass * nchunk + ch; ch < nchunk; g += 2, ch += 2) {
+                const unsigned step = st.base + (unsigned)g;
+                const int k0 = ch * KC;
+                // the MMAs that read the stage two steps ago must be done, and the
+                // group's last build have read the sample buffer
+                late = late || (step >= 2 && box_wait(bars->empty, step - 2, dead));
+                if (group_or(grp, late)) { late = true; break; }
+                put(X, k0);
+                group_sync(grp);
+                if (g + 2 < gtot) fetch();
+                // ---- A: SHP mask rows ----
 #pragma unroll
-                        for (int p = 0; p < NS; ++p) *reinterpret_cast<uint4 *>(db + p * L::B_BYTES + c * 16) = z;
-                } else {
+                for (int e = gt; e < BX_M * K8; e += BX_GRP) {
+                    const int m = e & (BX_M - 1), k8 = e >> 7;
+                    const int b0 = k0 + k8 * 8;
+                    const uint32_t bits = (umask[m * W + (b0 >> 5)] >> (b0 & 31)) & 0xffu;
+                    *reinterpret_cast<uint4 *>(As + (m >> 3) * L::SBO + k8 * 128 + (m & 7) * 16) = lut[bits];
+                }
+                // ---- B: outer-product entries, NS parts ----
+                // two samples per packed operation; the products round as
+                // fma(xr, yr, xi yi) and fma(xi, yr, -(xr yi))
+#pragma unroll
+                for (int i = 0; i < NIT; ++i) {
+                    if (it_off[i] < 0) continue;
+                    unsigned char *db = Bs + it_off[i];
+                    if (it_zero[i]) {
+                        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+#pragma unroll
+                            for (int p = 0; p < NS; ++p) *reinterpret_cast<uint4 *>(db + p * L::B_BYTES + c * 16) = z;
+                        continue;
+                    }
                     auto run8 = [](const unsigned char *src, f32x2 (&v)[4]) {
                         const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(src);
                         const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(src + 16);
                         v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
                     };
                     f32x2 xr[4], xi[4], nxr[4];
-                    run8(Xc + it_a, xr);
-                    run8(Xc + it_a + 4 * KC, xi);
+                    run8(X + it_a[i], xr);
+                    run8(X + it_a[i] + 4 * KC, xi);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) nxr[q] = xr[q] ^ 0x8000000080000000ull;
 #pragma unroll
                     for (int jb = 0; jb < 2; ++jb) {           // i = 2a + ia, j = 2b + jb
                         f32x2 yr[4], yi[4], v[4];
-                        run8(Xc + it_b + jb * (8 * KC), yr);
-                        run8(Xc + it_b + jb * (8 * KC) + 4 * KC, yi);
+                        run8(X + it_b[i] + jb * (8 * KC), yr);
+                        run8(X + it_b[i] + jb * (8 * KC) + 4 * KC, yi);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) v[q] = fma2(xr[q], yr[q], mul2(xi[q], yi[q]));       // Re x_i conj(x_j)
                         store_split<NS>(db + (2 * jb) * 16, L::B_BYTES, v);
@@ -503,41 +537,46 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
                         store_split<NS>(db + (2 * jb + 1) * 16, L::B_BYTES, v);
                     }
                 }
-            }
-            // the next chunk's samples go to the other buffer, which the
-            // previous chunk's build (before the previous barrier) read last
-            if (more) {
-                unsigned char *Xn = Xb + ((g + 1) & 1) * L::X_BYTES;
-                const int kn = ((g + 1) % nchunk) * KC;
-                if (g & 1) put(Xn, kn, xa);
-                else put(Xn, kn, xb);
-            }
-            fence_async_smem();
-            if (__syncthreads_or(late)) { st.timed_out = true; break; }
-            if (tid == 0) {
-                fence_after_sync();
-                const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
+                fence_async_smem();
+                mbar_arrive(&bars->full[grp]);
+                // one thread of the group, another warp's each time, issues the
+                // step's MMAs once all have arrived and the previous step's (another
+                // thread's, into the same accumulators) are done
+                if (warp == 8 * grp + (int)((step >> 1) & 7u)) {
+                    if (lane == 0) {
+                        late = box_wait(bars->full, step, dead) || (step >= 1 && box_wait(bars->empty, step - 1, dead));
+                        if (!late) {
+                            fence_after_sync();
+                            const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
 #pragma unroll
-                for (int kk = 0; kk < KC / 16; ++kk) {
-                    const uint64_t da = make_smem_desc(a0 + kk * 256, 128, L::SBO);
+                            for (int kk = 0; kk < KC / 16; ++kk) {
+                                const uint64_t da = make_smem_desc(a0 + kk * 256, 128, L::SBO);
 #pragma unroll
-                    for (int j = 0; j < L::NACC; ++j) {
-                        if (nmma[j] == 0) continue;
-                        const uint32_t boff = (uint32_t)(j * (BX_NCOL / 8) * L::SBO + kk * 256);
-                        const uint32_t dt = tbase + (uint32_t)(j * BX_NCOL);
+                                for (int j = 0; j < L::NACC; ++j) {
+                                    if (nmma[j] == 0) continue;
+                                    const uint32_t boff = (uint32_t)(j * (BX_NCOL / 8) * L::SBO + kk * 256);
+                                    const uint32_t dt = tbase + (uint32_t)(j * BX_NCOL);
 #pragma unroll
-                        for (int p = 0; p < NS; ++p)
-                            tc_mma(dt, da, make_smem_desc(b0 + p * L::B_BYTES + boff, 128, L::SBO), idesc[j],
-                                   (ch > 0 || kk > 0 || p > 0) ? 1u : 0u);
+                                    for (int p = 0; p < NS; ++p)
+                                        tc_mma(dt, da, make_smem_desc(b0 + p * L::B_BYTES + boff, 128, L::SBO), idesc[j],
+                                               (ch > 0 || kk > 0 || p > 0) ? 1u : 0u);
+                                }
+                            }
+                            tc_commit(&bars->empty[step & 1]);
+                            st.issued = step + 1;
+                        }
                     }
+                    __syncwarp();
                 }
-                tc_commit(&mbar[s]);
             }
-            st.pend |= 1u << s;
-            ++st.gstep;
         }
-        if (st.timed_out) return;
-        const bool late = box_poll(mbar, st, 0) || box_poll(mbar, st, 1);
+        __syncwarp();
+        // the pass's MMAs: its last step and the one before
+        {
+            const unsigned last = st.base + (unsigned)((pass + 1) * nchunk - 1);
+            if (!late) late = box_wait(bars->empty, last, dead);
+            if (!late && last >= 1) late = box_wait(bars->empty, last - 1, dead);
+        }
         if (pass == 0 && tid < BX_M) {
             // every sample of the tile has been stored (the last one before
             // the last chunk's barrier): a pixel with an out-of-range SHP
@@ -597,6 +636,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         __syncthreads();
     }
     if (st.timed_out) return;
+    st.base += (unsigned)gtot;
     if (tid < BX_M) {
         const int m = tid, info = pinfo[m];
         if (info != CI_SKIP) {
@@ -613,18 +653,19 @@ template <int KC>
 __device__ __forceinline__ uint32_t box_setup(unsigned char *smem, BoxPipe &st)
 {
     using L = BoxLay<KC, 2>;
-    unsigned char *misc = smem + L::OFF_MISC;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(misc);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 16);
+    BoxBars *bars = reinterpret_cast<BoxBars *>(smem + L::OFF_MISC);
     const int tid = threadIdx.x, warp = tid >> 5;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_addr(tmem_slot)), "r"(L::TCOL) : "memory");
+                     :: "r"(smem_addr(&bars->tmem_slot)), "r"(L::TCOL) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&bars->full[s], BX_GRP);
+            mbar_init(&bars->empty[s], 1);
+        }
+        bars->dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // mask patterns: entry b holds 8 bf16 values, 1 where bit q of b is set
@@ -636,15 +677,14 @@ __device__ __forceinline__ uint32_t box_setup(unsigned char *smem, BoxPipe &st)
             v[q] = ((b >> (2 * q)) & 1 ? 0x3F80u : 0u) | ((b >> (2 * q + 1)) & 1 ? 0x3F800000u : 0u);
         lut[b] = make_uint4(v[0], v[1], v[2], v[3]);
     }
-    st.pend = 0;
-    st.par = 0;
-    st.gstep = 0;
+    st.base = 0;
+    st.issued = 0;
     st.timed_out = false;
     st.blk_dp = -1;
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    return *tmem_slot;
+    return bars->tmem_slot;
 }
 
 // on a timeout: record the error, give the MMAs in flight a second bounded
@@ -653,15 +693,15 @@ template <int KC>
 __device__ __forceinline__ void box_teardown(unsigned char *smem, uint32_t tbase, BoxPipe &st, unsigned *err)
 {
     using L = BoxLay<KC, 2>;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::OFF_MISC);
+    BoxBars *bars = reinterpret_cast<BoxBars *>(smem + L::OFF_MISC);
     const int tid = threadIdx.x, warp = tid >> 5;
     if (st.timed_out) {
         if (tid == 0) atomicOr(err, ERR_TC_TIMEOUT);
-        for (int s = 0; s < 2; ++s) {
-            if (st.pend & (1u << s)) {
-                long long spins = 0;
-                while (!mbar_try_wait(&mbar[s], (st.par >> s) & 1u) && ++spins < BX_SPIN_LIMIT) {
-                }
+        // threads that issued MMAs wait for their last ones
+        if (st.issued > 0) {
+            const unsigned n = st.issued - 1;
+            long long spins = 0;
+            while (!mbar_try_wait(&bars->empty[n & 1], (n >> 1) & 1u) && ++spins < BX_SPIN_LIMIT) {
             }
         }
     }

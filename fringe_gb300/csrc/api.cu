@@ -360,7 +360,7 @@ __global__ void k_pack_settled(const long long *__restrict__ list, const int *__
          k += (long long)gridDim.x * blockDim.x) {
         const long long e = k / (nb + 3);
         const int slot = (int)(k - e * (nb + 3));
-        const long long pp = list[e];
+        const long long pp = list[e] < 0 ? ~list[e] : list[e];
         float2 v;
         if (slot < nb) v = phase[slot * plane + pp];
         else if (slot == nb) v = comp[pp];

@@ -88,7 +88,7 @@ __global__ void k_batch_fp64(const BatchEntry *__restrict__ jobs, int njobs)
         int cnt = *((volatile int *)P.fb_count);
         cnt = cnt < P.fb_cap ? cnt : P.fb_cap;
         for (long long q = list_first(); q < cnt; q = fb_next(P, lane))
-            process_pixel<double, NP>(P, P.fb_list[q], sm, lane, taddr);
+            settle_pixel<NP>(P, P.fb_list[q], sm, lane, taddr);
     }
     if constexpr (CInTmem<double, NP>::value) tmem_free_cta(tbase, warp, 512);
 }

@@ -4,10 +4,11 @@
 // k_solve, k_rest      : eigen-solves from the tensor-core Gamma records.
 // k_pixels<float, NP>  : plain FP32 kernel over a contiguous pixel range (windows
 //                        the Gamma kernel does not take, and runs without scratch).
-// k_pixels<double, NP> : FP64 form over the work list written by the FP32
-//                        pass (pixels whose discrete decisions fall inside the
-//                        FP32 rounding band), or over every pixel when no list
-//                        is given (used to check the FP64 form itself).
+// k_pixels<double, NP> : the work list written by the FP32 pass (pixels whose
+//                        discrete decisions fall inside the FP32 rounding band)
+//                        in float-float, then FP64 (settle_pixel), or FP64 over
+//                        every pixel when no list is given (used to check the
+//                        other forms).
 // All are persistent: the grid is sized to the resident capacity of the
 // GPU; warps stride over a pixel range, or draw work-list entries from a
 // cursor.
@@ -43,12 +44,15 @@ __global__ void k_pixels(KParams P)
         taddr = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp;
     }
     if (sizeof(T) == 4 || P.fb_list == nullptr) {
-        for (long long q = gw; q < P.npix; q += nw) process_pixel<T, NP>(P, P.pix_begin + q, sm, lane, taddr);
+        for (long long q = gw; q < P.npix; q += nw) {
+            if constexpr (sizeof(T) == 4) process_pixel<T, NP>(P, P.pix_begin + q, sm, lane, taddr);
+            else fp64_pixel<NP>(P, P.pix_begin + q, sm, lane, taddr);
+        }
     } else {
         int cnt = *((volatile int *)P.fb_count);
         cnt = cnt < P.fb_cap ? cnt : P.fb_cap;
         for (long long q = list_first(); q < cnt; q = fb_next(P, lane))
-            process_pixel<T, NP>(P, P.fb_list[q], sm, lane, taddr);
+            settle_pixel<NP>(P, P.fb_list[q], sm, lane, taddr);
     }
     if constexpr (CInTmem<T, NP>::value || CRowsTmemF<T, NP>::value) tmem_free_cta(tbase, warp, (uint32_t)tcols);
 }

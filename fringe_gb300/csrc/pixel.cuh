@@ -20,13 +20,20 @@
 // "is |Gamma| positive definite") whose FP32 answer lies inside a rounding
 // band, and |Gamma| whose condition estimate is too large for an FP32
 // inverse, are not settled in FP32: the pixel is appended to a list and
-// recomputed by the same code instantiated with T = double.
+// recomputed by the same code instantiated with T = ff (float-float, with bands
+// and a condition limit of its own), and where that leaves a decision open, or the
+// samples lie outside its range, with T = double.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
+#include "ff.cuh"
+
 namespace fpl {
+using fpl_ff::ff;
 
 // ------------------------------------------------------------------------
 // parameters shared by all pixel kernels
@@ -107,7 +114,12 @@ template <typename T> __device__ __forceinline__ void cfma(C2<T> &acc, C2<T> a, 
     acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
 }
 
-// b -= a * y and b -= conj(a) * y as fused multiply-adds
+// b -= a * conj(y), b -= a * y and b -= conj(a) * y as fused multiply-adds
+template <typename T> __device__ __forceinline__ void fms_mulc(C2<T> &b, C2<T> a, C2<T> y)
+{
+    b.x = fma(-a.x, y.x, fma(-a.y, y.y, b.x));
+    b.y = fma(a.x, y.y, fma(-a.y, y.x, b.y));
+}
 template <typename T> __device__ __forceinline__ void fms_mul(C2<T> &b, C2<T> a, C2<T> y)
 {
     b.x = fma(-a.x, y.x, fma(a.y, y.y, b.x));
@@ -140,6 +152,7 @@ template <typename T> __device__ __forceinline__ T warp_min(T v)
 
 template <typename T> struct Eps;
 template <> struct Eps<float> { static constexpr float v = 1.1920929e-7f; static constexpr float tiny = 1.17549435e-38f; };
+template <> struct Eps<ff> { static constexpr double v = 1.4210854715202004e-14, tiny = 1e-30; };   // 2^-46
 template <> struct Eps<double> { static constexpr double v = 2.220446049250313e-16; static constexpr double tiny = 2.2250738585072014e-308; };
 
 // fast division where only a rounding-level result is needed (Sturm counts)
@@ -182,28 +195,30 @@ template <typename T, int NP> struct Lay {
 // and normalised: it sits right after the gather staging, over the work
 // matrix (which the solve uses only after C has been copied out), and the
 // vectors follow it.  91.6 KB per warp instead of 141 KB: two warps per SM.
-template <> struct Lay<double, 64> {
+template <typename T> struct Lay64W {
     static constexpr int NP = 64;
     static constexpr int LD = NP + 1;
     static constexpr int XS = NP + 2;
-    static constexpr size_t mat = sizeof(C2<double>) * NP * LD;
+    static constexpr size_t mat = sizeof(C2<T>) * NP * LD;
     static constexpr size_t wm = 0;
     static constexpr size_t stage = align16(sizeof(float2) * 32 * XS);  // gather staging at wm
     static constexpr size_t wm_bytes = align16(cmax(mat, stage));
     static constexpr size_t xr = wm + align16(mat / 2);
     static constexpr size_t cm = stage;                               // Gamma / C while it is formed
     static constexpr size_t vv = cmax(wm + wm_bytes, cm + align16(mat));
-    static constexpr size_t ww = align16(vv + sizeof(C2<double>) * NP);
-    static constexpr size_t tu = align16(ww + sizeof(C2<double>) * NP);
-    static constexpr size_t dd = align16(tu + sizeof(C2<double>) * NP);
-    static constexpr size_t ee = align16(dd + sizeof(double) * NP);
-    static constexpr size_t e2 = align16(ee + sizeof(double) * NP);
-    static constexpr size_t yy = align16(e2 + sizeof(double) * NP);
-    static constexpr size_t wk = align16(yy + sizeof(double) * NP);
-    static constexpr size_t ph = align16(wk + sizeof(double) * 5 * NP);
+    static constexpr size_t ww = align16(vv + sizeof(C2<T>) * NP);
+    static constexpr size_t tu = align16(ww + sizeof(C2<T>) * NP);
+    static constexpr size_t dd = align16(tu + sizeof(C2<T>) * NP);
+    static constexpr size_t ee = align16(dd + sizeof(T) * NP);
+    static constexpr size_t e2 = align16(ee + sizeof(T) * NP);
+    static constexpr size_t yy = align16(e2 + sizeof(T) * NP);
+    static constexpr size_t wk = align16(yy + sizeof(T) * NP);
+    static constexpr size_t ph = align16(wk + sizeof(T) * 5 * NP);
     static constexpr size_t bytes_noc = align16(ph + sizeof(float2) * NP);
     static constexpr size_t bytes = bytes_noc;
 };
+template <> struct Lay<double, 64> : Lay64W<double> {};
+template <> struct Lay<ff, 64> : Lay64W<ff> {};
 
 // while Gamma is summed the gather staging, the coherence and the vectors
 // (1/sqrt(P) among them) are all live, so they must not overlap; the work
@@ -213,7 +228,7 @@ static_assert(Lay<double, 64>::vv >= Lay<double, 64>::cm + Lay<double, 64>::mat,
 static_assert(Lay<double, 64>::vv >= Lay<double, 64>::wm + Lay<double, 64>::wm_bytes, "vectors overlap W");
 static_assert(2 * Lay<double, 64>::bytes <= 224 * 1024, "two warps per CTA");
 
-// kernels whose warps hold C in tensor memory in the FP64 form
+// kernels whose warps hold C in tensor memory in the FP64 and float-float forms
 template <typename T, int NP> struct CInTmem {
     static constexpr bool value = sizeof(T) == 8 && NP == 64;
 };
@@ -324,14 +339,28 @@ template <int NP> struct CRowsTmem {
     }
 };
 
-// The same rows of an FP64 C: a complex double is four 32-bit columns, so
+// The same rows of an FP64 or float-float C: a value is two 32-bit words, a
+// complex one four columns, so
 // row slot h starts 4*NP columns after slot h-1 (at 64 dates the warp's
 // two row slots fill the 512 columns of its lane quadrant).
-template <int NP> struct CRowsTmemD {
+__device__ __forceinline__ void words_of(double x, uint32_t &a, uint32_t &b)
+{
+    a = (uint32_t)__double2loint(x);
+    b = (uint32_t)__double2hiint(x);
+}
+__device__ __forceinline__ void words_of(ff x, uint32_t &a, uint32_t &b)
+{
+    a = __float_as_uint(x.l);
+    b = __float_as_uint(x.h);
+}
+__device__ __forceinline__ void of_words(uint32_t a, uint32_t b, double &x) { x = __hiloint2double((int)b, (int)a); }
+__device__ __forceinline__ void of_words(uint32_t a, uint32_t b, ff &x) { x = ff(__uint_as_float(b), __uint_as_float(a)); }
+
+template <typename T, int NP> struct CRowsTmemD {
     static_assert(NP <= 64, "at most two rows per lane");
     static constexpr uint32_t kColsPerWarp = 4u * NP * ((NP + 31) / 32);
     uint32_t taddr;      // lane quadrant << 16 | first column of the warp
-    __device__ __forceinline__ void load(int h, int c, C2<double> (&v)[8]) const
+    __device__ __forceinline__ void load(int h, int c, C2<T> (&v)[8]) const
     {
         const uint32_t a = taddr + (uint32_t)(4 * NP * h) + 32u * (uint32_t)c;
 #pragma unroll
@@ -339,12 +368,13 @@ template <int NP> struct CRowsTmemD {
             uint32_t r[16];
             tmem_ld16(a + 16u * (uint32_t)half, r);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                v[4 * half + k] = cmk<double>(__hiloint2double((int)r[4 * k + 1], (int)r[4 * k]),
-                                              __hiloint2double((int)r[4 * k + 3], (int)r[4 * k + 2]));
+            for (int k = 0; k < 4; ++k) {
+                of_words(r[4 * k], r[4 * k + 1], v[4 * half + k].x);
+                of_words(r[4 * k + 2], r[4 * k + 3], v[4 * half + k].y);
+            }
         }
     }
-    __device__ __forceinline__ void store(int h, int c, const C2<double> (&v)[8]) const
+    __device__ __forceinline__ void store(int h, int c, const C2<T> (&v)[8]) const
     {
         const uint32_t a = taddr + (uint32_t)(4 * NP * h) + 32u * (uint32_t)c;
 #pragma unroll
@@ -352,11 +382,9 @@ template <int NP> struct CRowsTmemD {
             uint32_t r[16];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const C2<double> x = v[4 * half + k];
-                r[4 * k] = (uint32_t)__double2loint(x.x);
-                r[4 * k + 1] = (uint32_t)__double2hiint(x.x);
-                r[4 * k + 2] = (uint32_t)__double2loint(x.y);
-                r[4 * k + 3] = (uint32_t)__double2hiint(x.y);
+                const C2<T> x = v[4 * half + k];
+                words_of(x.x, r[4 * k], r[4 * k + 1]);
+                words_of(x.y, r[4 * k + 2], r[4 * k + 3]);
             }
             tmem_st16(a + 16u * (uint32_t)half, r);
         }
@@ -472,8 +500,12 @@ __device__ bool warp_chol_c(C2<T> *A, int n, C2<T> *col, int lane)
                 for (int u = 0; u < 4; ++u) a[u] = Ai[k + u];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    a[u].x -= li.x * l[u].x + li.y * l[u].y;
-                    a[u].y -= li.y * l[u].x - li.x * l[u].y;
+                    if constexpr (std::is_same<T, ff>::value) {
+                        fms_mulc(a[u], li, l[u]);
+                    } else {
+                        a[u].x -= li.x * l[u].x + li.y * l[u].y;
+                        a[u].y -= li.y * l[u].x - li.x * l[u].y;
+                    }
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
@@ -718,7 +750,11 @@ __device__ bool warp_sweep_inverse(T *A, int n, T *rowk, T *inf_norm, int lane, 
 #pragma unroll
                 for (int u = 0; u < 8; ++u) x[u] = Ai[j + u];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) Ai[j + u] = fma(b, r[u], a * x[u]);
+                for (int u = 0; u < 8; ++u) {
+                    if constexpr (std::is_same<T, ff>::value) x[u] = own ? T(0) : x[u];
+                    else x[u] = a * x[u];
+                    Ai[j + u] = fma(b, r[u], x[u]);
+                }
             }
             for (; j < n; ++j) Ai[j] = fma(b, rowk[j], a * Ai[j]);
             Ai[k] = own ? -rp : f;
@@ -906,8 +942,18 @@ __device__ void warp_tridiag(C2<T> *A, int n, T *d, T *e, C2<T> *tau, C2<T> *vv,
                     } else {
                         v0 = vv[j]; v1 = vv[j + 1]; w0 = ww[j]; w1 = ww[j + 1];
                     }
-                    if (j > k) Ai[j] = csub(Ai[j], cadd(cmulc(vi, w0), cmulc(wi, v0)));
-                    if (j + 1 < n) Ai[j + 1] = csub(Ai[j + 1], cadd(cmulc(vi, w1), cmulc(wi, v1)));
+                    if constexpr (std::is_same<T, ff>::value) {
+                        C2<T> a0 = Ai[j], a1 = Ai[j + 1 < n ? j + 1 : j];
+                        fms_mulc(a0, vi, w0);
+                        fms_mulc(a1, vi, w1);
+                        fms_mulc(a0, wi, v0);
+                        fms_mulc(a1, wi, v1);
+                        if (j > k) Ai[j] = a0;
+                        if (j + 1 < n) Ai[j + 1] = a1;
+                    } else {
+                        if (j > k) Ai[j] = csub(Ai[j], cadd(cmulc(vi, w0), cmulc(wi, v0)));
+                        if (j + 1 < n) Ai[j + 1] = csub(Ai[j + 1], cadd(cmulc(vi, w1), cmulc(wi, v1)));
+                    }
                 }
             }
             __syncwarp();
@@ -952,8 +998,8 @@ __device__ T warp_tridiag_eig(const T *d, const T *e, T *e2, int n, int index, T
     gu = warp_max(gu);
     em = warp_max(em);
     __syncwarp();
-    const T eps = Eps<T>::v;
-    const T pivmin = Eps<T>::tiny * max(T(1), em) * T(4);
+    const T eps = T(Eps<T>::v);
+    const T pivmin = T(Eps<T>::tiny) * max(T(1), em) * T(4);
     const T tnorm = max(abs(gl), abs(gu));
     const T fudge = T(2.1) * eps * tnorm * T(n) + T(2) * pivmin;
     T lo = max(gl - fudge, lo_hint), hi = min(gu + fudge, hi_hint);
@@ -988,7 +1034,7 @@ __device__ void tridiag_inverse_iteration(const T *d, const T *e, int n, T lam, 
 {
     if (lane == 0) {
         T *rdg = wk, *u1 = wk + n, *u2 = wk + 2 * n, *l = wk + 3 * n, *pv = wk + 4 * n;
-        const T eps = Eps<T>::v * (tnorm > T(0) ? tnorm : T(1));
+        const T eps = T(Eps<T>::v) * (tnorm > T(0) ? tnorm : T(1));
         T dgi = d[0] - lam;
         T u1i = (n > 1) ? e[0] : T(0);
         T dnext = (n > 1) ? d[1] - lam : T(0);
@@ -1101,7 +1147,7 @@ __device__ bool warp_power(const CP &cp, int n, unsigned char *sm, int lane, C2<
     for (int i = lane; i < NP; i += 32) vv[i] = cmk<T>(i < n ? T(1) : T(0), T(0));
     __syncwarp();
     T rprev = T(-1);
-    const T tol = (sizeof(T) == 4) ? T(4e-6) : T(1e-13);
+    const T tol = (sizeof(T) == 4) ? T(4e-6) : (std::is_same<T, ff>::value ? T(1e-12) : T(1e-13));
     for (int it = 0; it < 96; ++it) {
         C2<T> u[2];
         rows_matvec<T, NP>(cp, n, vv, u[0], u[1], lane);
@@ -1208,9 +1254,9 @@ __device__ int warp_inverse_iteration(C2<T> *W, int n, T sigma, unsigned char *s
     if (!warp_chol_any<T, LD, NP, true>(W, n, col, lane)) return -1;
     T d0 = T(0), d1 = T(0);
     chol_strict_lower<T, LD, NP>(W, n, d0, d1, lane);
-    const T tol = (sizeof(T) == 4) ? T(1e-5) : T(1e-12);
+    const T tol = (sizeof(T) == 4) ? T(1e-5) : T(1e-11);   // well under the outputs' FP32 rounding
     T rprev = T(-1), cprev = T(1), gap_good = T(0);
-    for (int it = 0; it < 10; ++it) {
+    for (int it = 0; it < (sizeof(T) == 4 ? 10 : 32); ++it) {
         C2<T> x0 = z0, x1 = z1;
         warp_chol_solve<T, LD, NP>(W, n, d0, d1, x0, x1, lane);
         const T xx = warp_sum(cabs2(x0) + cabs2(x1));
@@ -1238,6 +1284,8 @@ __device__ int warp_inverse_iteration(C2<T> *W, int n, T sigma, unsigned char *s
             }
             // residual no longer decreasing: rounding floor
             if (it >= 3 && c > T(0.9)) return (rn <= T(20) * tol * gap_good) ? 1 : 0;
+            // a nearer shift is the shorter way to nine digits
+            if (sizeof(T) != 4 && it >= 3 && crate > T(0.4)) return 0;
             cprev = c;
         }
         rprev = rn;
@@ -1269,7 +1317,7 @@ __device__ bool abs_not_pd(const CP &cp, const T *rk, int k, int n, T amb, T *ub
     constexpr int H = RowShape<NP>::H;
     for (int i = lane; i < NP; i += 32) ub[i] = (i < k) ? -rk[i] : (i == k ? T(1) : T(0));
     __syncwarp();
-    const T g = T(2 * (n + 1)) * Eps<T>::v;
+    const T g = T(2 * (n + 1)) * T(Eps<T>::v);
     T band = T(0), anorm = T(0);
     for (int it = 0;; ++it) {
         T q = T(0), s = T(0), v2 = T(0), f2 = T(0), rmax = T(0);
@@ -1369,6 +1417,19 @@ __device__ __forceinline__ void acc_prod<double>(C2<double> &acc, float2 a, floa
     acc.y += double(im);
 }
 
+// float-float form: the same products, summed exactly to 2^-48
+template <>
+__device__ __forceinline__ void acc_prod<ff>(C2<ff> &acc, float2 a, float2 b)
+{
+    const float re = __fadd_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+    const float im = __fsub_rn(__fmul_rn(a.y, b.x), __fmul_rn(a.x, b.y));
+    float e;
+    acc.x.h = fpl_ff::two_sum(acc.x.h, re, e);
+    acc.x.l = __fadd_rn(acc.x.l, e);
+    acc.y.h = fpl_ff::two_sum(acc.y.h, im, e);
+    acc.y.l = __fadd_rn(acc.y.l, e);
+}
+
 // Entries of a work list for this warp: the first is dealt out, CTA by CTA (a
 // short list then has one entry per SM: drawn from the cursor from the start, 15 pixels
 // all went to the first CTA's warps, which share the SM's FP64 pipe), further
@@ -1383,11 +1444,13 @@ __device__ __forceinline__ long long list_next(int *cursor, int lane)
 }
 __device__ __forceinline__ long long fb_next(const KParams &P, int lane) { return list_next(P.fb_count + 12, lane); }
 
-__device__ __forceinline__ void defer_fp64(const KParams &P, long long pp, int lane)
+// range: the pixel's samples lie outside the range of the split (and of
+// float-float): straight to FP64, marked by the complement
+__device__ __forceinline__ void defer_fp64(const KParams &P, long long pp, int lane, bool range = false)
 {
     if (lane == 0) {
         int idx = atomicAdd(P.fb_count, 1);
-        if (idx < P.fb_cap) P.fb_list[idx] = pp;
+        if (idx < P.fb_cap) P.fb_list[idx] = range ? ~pp : pp;
         else atomicOr(P.err, ERR_FB_OVERFLOW);
     }
 }
@@ -1408,8 +1471,9 @@ __device__ __forceinline__ void rest_put(const KParams &P, long long pp)
 __device__ __forceinline__ long long rest_next(const KParams &P, int lane) { return list_next(P.fb_count + 13, lane); }
 
 // Gather, Gamma and coherence (evd.cpp:514-582).  Returns the SHP count
-// with C in the warp's slab, or -1 when the pixel is finished (skipped or
-// coded) and its outputs are written.
+// with C in the warp's slab, -1 when the pixel is finished (skipped or
+// coded) and its outputs are written, or PX_OPEN (float-float) when it is left to FP64.
+constexpr int PX_OPEN = -2;
 // Gamma (upper triangle and diagonal of the warp's C slab) to coherence
 // (evd.cpp:569-582, phase_link.cpp:527-538): C_ij = Gamma_ij / sqrt(P_i P_j),
 // lower triangle by conjugation, unit diagonal.  A non-finite result is
@@ -1423,9 +1487,20 @@ __device__ bool gamma_to_coherence(const KParams &P, long long pp, C2<T> *Cm, un
     const int n = P.nb;
     const bool plink = (P.semantics == SEM_PL);
     bool bad = false;
+    if constexpr (std::is_same<T, ff>::value) {
+        // the sums' low parts have grown past the high parts' last bit
+        for (int i = lane; i < n; i += 32)
+            for (int j = i; j < n; ++j) {
+                C2<T> &g = Cm[i * LD + j];
+                g = cmk<T>(fpl_ff::quick(g.x.h, g.x.l), fpl_ff::quick(g.y.h, g.y.l));
+            }
+        __syncwarp();
+    }
     for (int i = lane; i < n; i += 32) {
         T Pi = Cm[i * LD + i].x;
         bad |= !(Pi > T(0)) || !isfinite(Pi);
+        // float-float keeps its low parts well above FP32's smallest number only inside this range
+        if constexpr (std::is_same<T, ff>::value) bad |= !(Pi.h > 1e-20f && Pi.h < 1e30f);
         yv[i] = T(1) / sqrt(Pi);
     }
     bad = __any_sync(0xffffffffu, bad);
@@ -1437,8 +1512,12 @@ __device__ bool gamma_to_coherence(const KParams &P, long long pp, C2<T> *Cm, un
                 C2<T> g = Cm[i * LD + j];
                 C2<T> c;
                 if (sizeof(T) == 8) {
-                    T den = sqrt(Cm[i * LD + i].x * Cm[j * LD + j].x);
-                    c = cmk<T>(g.x / den, g.y / den);
+                    if constexpr (std::is_same<T, ff>::value) {
+                        c = cscale(g, ri * yv[j]);
+                    } else {
+                        T den = sqrt(Cm[i * LD + i].x * Cm[j * LD + j].x);
+                        c = cmk<T>(g.x / den, g.y / den);
+                    }
                 } else {
                     c = cscale(g, ri * yv[j]);
                 }
@@ -1457,8 +1536,9 @@ __device__ bool gamma_to_coherence(const KParams &P, long long pp, C2<T> *Cm, un
     }
     if (bad) {
         // non-finite coherence: LAPACK's answer on NaN input is undefined;
-        // the first eigen call is reported as failed.
-        put_code(P, pp, lane, (!plink && P.method != M_MLE) ? -6 : -1);
+        // the first eigen call is reported as failed (by the FP64 form, whose
+        // range is the reference's, when this is float-float).
+        if (!std::is_same<T, ff>::value) put_code(P, pp, lane, (!plink && P.method != M_MLE) ? -6 : -1);
         return false;
     }
     return true;
@@ -1614,16 +1694,18 @@ __device__ int pixel_coherence(const KParams &P, long long pp, unsigned char *sm
         return -1;
     }
 
-    if (!gamma_to_coherence<T, NP>(P, pp, Cm, sm, lane)) return -1;
+    if (!gamma_to_coherence<T, NP>(P, pp, Cm, sm, lane)) return std::is_same<T, ff>::value ? PX_OPEN : -1;
     return npix;
 }
 
 
 // Eigen-solve and outputs for a pixel whose coherence C is reached through
 // the row policy cp (the warp's slab, or tensor memory), evd.cpp:584-786,
-// phase_link.cpp:540-665.
+// phase_link.cpp:540-665.  Decisions inside the rounding band: FP32 appends the
+// pixel to the list and returns true, float-float returns false (for FP64 to
+// take over).
 template <typename T, int NP, typename CP>
-__device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, int lane, int npix,
+__device__ bool pixel_solve(const KParams &P, long long pp, unsigned char *sm, int lane, int npix,
                             const CP &cp, T cfro = T(-1))
 {
     using L = Lay<T, NP>;
@@ -1638,8 +1720,12 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
     const long long plane = P.plane;
     const bool plink = (P.semantics == SEM_PL);
 
-    const bool fp32 = sizeof(T) == 4;
-    const T amb = T(P.amb) * T(n) * Eps<T>::v;          // rounding band unit (FP32 only)
+    constexpr bool fp32 = sizeof(T) == 4, banded = !std::is_same<T, double>::value;
+    auto open = [&]() {
+        if (fp32) defer_fp64(P, pp, lane);
+        return fp32;
+    };
+    const T amb = T(P.amb) * T(n) * T(Eps<T>::v);       // rounding band unit (not FP64)
     const T thr = T(1.0e-6);
     int mode = 0;       // 0 = MLE eigvec of M, 1 = largest eigvec of C
     int pstatus = 0;
@@ -1706,7 +1792,7 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
             ok = warp_sweep_inverse<T, LD, NP>(Xr, nn, yv, &xnorm, lane, &kfail);
             rk = yv;
         }
-        if (!fp32) return ok ? 1 : -1;
+        if (!banded) return ok ? 1 : -1;
         if (!ok) {
             // FP32 pivot failure: |C| clearly not positive definite, or
             // positive definite but too close to singular for FP32 (settled
@@ -1714,7 +1800,8 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
             T *ub = reinterpret_cast<T *>(sm + L::wk) + 3 * NP;     // past the sweep's rows
             return abs_not_pd<T, NP>(cp, rk, kfail, nn, amb, ub, lane) ? -1 : 0;
         }
-        if (!(anorm * xnorm <= T(P.cond_max))) return 0;
+        // (float-float: the inverse keeps 2^-46 times the condition)
+        if (!(anorm * xnorm <= (fp32 ? T(P.cond_max) : T(1e6f)))) return 0;
         return 1;
     };
 
@@ -1726,19 +1813,19 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
             // smallest eigenvalue is 0 up to FP32 product rounding (far
             // below 1e-6): the reference reports -2.
             put_code(P, pp, lane, -2);
-            return;
+            return true;
         }
-        const T dC = fp32 ? amb * (cfro >= T(0) ? cfro : fro_c()) : T(0);
+        const T dC = banded ? amb * (cfro >= T(0) ? cfro : fro_c()) : T(0);
         const int r = lam_min_test_c<T, LD, NP>(cp, Wm, col, n, thr, dC, lane);
-        if (r == 0) { defer_fp64(P, pp, lane); return; }
-        if (r < 0) { put_code(P, pp, lane, -2); return; }
+        if (r == 0) return open();
+        if (r < 0) { put_code(P, pp, lane, -2); return true; }
     }
     if (mle_evd || plink) {
         // |C| and its inverse: evd.cpp:623-664 (check, then inverse);
         // phase_link.cpp:540-618 (MLE if |C| is invertible, else EVD).  One
         // call site for both modules.
         const int r = abs_inverse();
-        if (r == 0) { defer_fp64(P, pp, lane); return; }
+        if (r == 0) return open();
         if (plink) {
             if (r > 0) {
                 mode = 0;
@@ -1751,9 +1838,9 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
                 // not positive definite (FP64, or proved in FP32 by
                 // abs_not_pd), so lambda_min(|C|) <= 0 < 1e-6
                 put_code(P, pp, lane, -4);
-                return;
+                return true;
             }
-            if (!fp32) {
+            if (!banded) {
                 // lambda_min(|C|) >= 1/||inv|C|||_inf settles the 1e-6 test
                 // unless the inverse is large
                 T xn = T(0);
@@ -1785,16 +1872,16 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
                     __syncwarp();
                     if (!warp_chol_c<T, LD, NP>(Wm, n, col, lane)) {
                         put_code(P, pp, lane, -4);
-                        return;
+                        return true;
                     }
                     __syncwarp();
                     abs_inverse();
                 }
             } else {
                 // lambda_min(|C|) >= 1 / ||inv|C|||_inf, so a small inverse
-                // norm settles the 1e-6 test; anything else is settled in FP64
+                // norm settles the 1e-6 test; anything else is left open
                 const T dA = amb * T(n);
-                if (!(T(1) / xnorm > thr + dA)) { defer_fp64(P, pp, lane); return; }
+                if (!(T(1) / xnorm > thr + dA)) return open();
             }
             mode = 0;
         }
@@ -1861,7 +1948,7 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
         // 2-norm of the symmetric inv|C| is at most its inf-norm) settles
         // without a pass over M; the exact value is formed while M is in Wm
         // whenever a decision is not settled by the bound.
-        const bool need_band = fp32 && !plink;
+        const bool need_band = banded && !plink;
         dM = need_band ? amb * sqrt(T(n)) * xnorm : T(0);
         bool dM_exact = !need_band;
         auto exact_dM = [&]() {
@@ -1872,7 +1959,11 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
         };
         __syncwarp();
         bool done = false;
-        if (fp32) {
+        // float-float: from 33 dates on (30 dates, 788 entries: 0.48 ms on the
+        // Householder path, 0.95 ms here, where slow contraction falls back;
+        // 64 dates, 1451 entries: 11.1 and 9.7 ms); phase_link's M has no bound
+        // to shift under (50 dates: 0.65 and 1.26 ms)
+        if (fp32 || (banded && NP == 64 && !plink)) {
             // inverse iteration from the EVD direction, shifted just below
             // the Rayleigh quotient (the smallest eigenvalue is close to 1)
             warp_power_start<T, NP>(cp, n, kPowerStartIters, sm, lane, z0, z1);
@@ -1902,7 +1993,7 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
                         form_M();
                     }
                     if (st == 1 || attempt == 1) break;
-                    if (lane == 0) atomicAdd(P.slow, 1);
+                    if (fp32 && lane == 0) atomicAdd(P.slow, 1);
                     T sigma1;
                     if (st == 0) {
                         // slow: shift again just below the current Rayleigh
@@ -1956,13 +2047,13 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
     if (eig_index) lam = warp_eigpair<T, NP>(Wm, n, eig_index, eig_lo, eig_hi, sm, lane, z0, z1);
     if (mode == 0) {
         if (eig_index && !plink) {
-            if (fp32 && lam < thr + dM && lam >= thr - dM) { defer_fp64(P, pp, lane); return; }
-            if (lam < thr) { put_code(P, pp, lane, -7); return; }
+            if (banded && lam < thr + dM && lam >= thr - dM) return open();
+            if (lam < thr) { put_code(P, pp, lane, -7); return true; }
         }
     } else {
         // trace(C) = n, so lambda_max >= 1: the -7 test of evd.cpp:718-726
         // cannot trigger for a finite C.
-        if (!plink && lam < thr) { put_code(P, pp, lane, -7); return; }
+        if (!plink && lam < thr) { put_code(P, pp, lane, -7); return true; }
     }
 
     // ---- phase referencing (evd.cpp:738-749) ------------------------------
@@ -2056,6 +2147,7 @@ __device__ void pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
             if (P.status) P.status[pp] = pstatus;
         }
     }
+    return true;
 }
 
 
@@ -2099,7 +2191,7 @@ __device__ int pixel_load_gamma(const KParams &P, long long pp, unsigned char *s
         return -1;
     }
     if (info == CI_DEFER) {
-        defer_fp64(P, pp, lane);
+        defer_fp64(P, pp, lane, true);
         return -1;
     }
     const float4 *rec4 =
@@ -2228,23 +2320,46 @@ __device__ bool rows_coherence(const KParams &P, long long pp, const C2<float> *
 // CRowsTmemF<T, NP> (C is formed in shared memory, then moved there before
 // the solve reuses that memory)
 template <typename T, int NP>
-__device__ void process_pixel(const KParams &P, long long pp, unsigned char *sm, int lane, uint32_t taddr = 0)
+__device__ bool process_pixel(const KParams &P, long long pp, unsigned char *sm, int lane, uint32_t taddr = 0)
 {
     const int npix = pixel_coherence<T, NP>(P, pp, sm, lane);
-    if (npix < 0) return;
+    if (npix < 0) return npix != PX_OPEN;
     const C2<T> *Cm = reinterpret_cast<const C2<T> *>(sm + CmOffset<T, NP>::value);
     if constexpr (CInTmem<T, NP>::value) {
-        const CRowsTmemD<NP> cp{taddr};
+        const CRowsTmemD<T, NP> cp{taddr};
         rows_from_smem<NP>(cp, Cm, lane);
-        pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
+        return pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
     } else if constexpr (CRowsTmemF<T, NP>::value) {
         const CRowsTmem<NP> cp{taddr};
         rows_from_smem<NP>(cp, Cm, lane);
-        pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
+        return pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
     } else {
         const CRowsSmem<T, NP> cp{const_cast<C2<T> *>(Cm), lane};
-        pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
+        return pixel_solve<T, NP>(P, pp, sm, lane, npix, cp);
     }
+}
+
+// A work-list entry: float-float, then FP64 where that leaves the pixel
+// open (out of line: 6 of 396 entries do at 333x517 with 23 dates, 5 of 1451 at
+// 384x320 with 64).  The FP64 pipe's two operations per SM and clock bound the
+// list before; float-float is bound by the latency of one pixel's chain (two
+// warps per SM at 64 dates, whose matrix takes 67 KB of shared memory).  List kernel
+// alone, FP64 -> float-float: 384x320, 64 dates 26.1 -> 9.7 ms (1451 entries);
+// 1024x1024, 30 dates 1.6 -> 0.45 ms (788); 1023x777, 15 dates 0.44 -> 0.19 ms (15).
+// Against FP64 for every pixel (n 10..64) the codes are the same and the
+// phases differ by at most 1e-7 rad, FP32's rounding of the output.
+template <int NP>
+__device__ __noinline__ void fp64_pixel(const KParams &P, long long pp, unsigned char *sm, int lane, uint32_t taddr)
+{
+    process_pixel<double, NP>(P, pp, sm, lane, taddr);
+}
+template <int NP>
+__device__ __forceinline__ void settle_pixel(const KParams &P, long long entry, unsigned char *sm, int lane, uint32_t taddr)
+{
+    const long long pp = entry < 0 ? ~entry : entry;
+    if (entry >= 0 && process_pixel<ff, NP>(P, pp, sm, lane, taddr)) return;
+    __syncwarp();
+    fp64_pixel<NP>(P, pp, sm, lane, taddr);
 }
 
 }  // namespace fpl

@@ -454,7 +454,7 @@ __device__ __forceinline__ int tile_begin(const KParams &P, long long pp, const 
         const int info = P.cinfo[loc];
         if (info < 0) {
             tile_zero<G>(P, pp, L.g);
-            if (info == CI_DEFER) defer_fp64(P, pp, L.g);
+            if (info == CI_DEFER) defer_fp64(P, pp, L.g, true);
             else if (P.status && L.g == 0) P.status[pp] = (info == CI_CENTRE) ? 1 : 2;
             state = TILE_DONE;
         }

@@ -29,9 +29,10 @@
 // within the band of the 1e-6 test, |C| not positive definite, a shift above
 // lambda_1, slow convergence -- the pixel goes on a list for pixel_solve, which decides
 // as it always did.  Solve kernels on GB300: 2048^2, N = 30, 11 x 21, 91.9 ->
-// 54.8 ms (9.4 k warp instructions per pixel, 57% of the issue slots); 384 x 320,
-// N = 64, ill-conditioned, 37.7 -> 12.6 ms; 333 x 517, N = 23, 2.77 -> 1.43 ms;
-// 1023 x 777, N = 15, 4.29 -> 3.31 ms.
+// 50.9 ms; 384 x 320, N = 64, ill-conditioned, 37.7 -> 9.7 ms; 333 x 517, N = 23,
+// 2.77 -> 1.34 ms; 1023 x 777, N = 15, 4.29 -> 3.18 ms.  The FMA pipe bounds it (a
+// packed multiply-add holds it for 2.3 clocks), then instruction fetch: swaps and signs
+// are therefore moves and bit operations, not products (1024^2, N = 30, 13.75 -> 12.7 ms).
 #pragma once
 #include "f32x2.cuh"
 #include "pixel.cuh"
@@ -157,7 +158,7 @@ __device__ __forceinline__ void tile_ldl_step(CBlk (&A)[Tile<G, NL>::NB], const 
 #pragma unroll
         for (int mi = MS; mi < NL; ++mi) {
             const CBlk &b = A[M::blk(mi, S)];
-            const uint32_t a = (mi == MS && L.lr == tr) ? diag : at(LRN * mi + L.lr);
+            const uint32_t a = (!LOW && mi == MS && L.lr == tr) ? diag : at(LRN * mi + L.lr);
             if (mi > MS || L.lr >= tr) {
                 if (PAR == 0) sts4(a, lo2(b.dr), lo2(b.er), lo2(b.di), lo2(b.ei));
                 else sts4(a, hi2(b.er), hi2(b.dr), hi2(b.ei), hi2(b.di));
@@ -176,22 +177,24 @@ __device__ __forceinline__ void tile_ldl_step(CBlk (&A)[Tile<G, NL>::NB], const 
     f32x2 cr[NLC - S], ci[NLC - S];
 #pragma unroll
     for (int li = S; li < NLC; ++li)
-        lds4((li == S && L.lc == tl) ? diag : at(4 * li + L.lc), cr[li - S], ci[li - S]);
-    const f32x2 r2 = pk(r, r), nr2 = pk(nr, nr);
+        lds4((!LOW && li == S && L.lc == tl) ? diag : at(4 * li + L.lc), cr[li - S], ci[li - S]);
+    const f32x2 nr2 = pk(nr, nr);
+    f32x2 nci[NLC - S];
+#pragma unroll
+    for (int li = S; li < NLC; ++li) nci[li - S] = ci[li - S] ^ 0x8000000080000000ull;
 #pragma unroll
     for (int mi = MS; mi < NL; ++mi) {
         f32x2 vr, vi;
-        lds4((mi == MS && L.lr == tr) ? diag : at(LRN * mi + L.lr), vr, vi);
-        const f32x2 sr = mul2(vr, nr2), si = mul2(vi, nr2), pr = mul2(vr, r2);
-        const f32x2 srs = pk(nr * hi2(vr), nr * lo2(vr)), sis = pk(nr * hi2(vi), nr * lo2(vi)),
-                    prs = pk(r * hi2(vr), r * lo2(vr));
+        lds4((!LOW && mi == MS && L.lr == tr) ? diag : at(LRN * mi + L.lr), vr, vi);
+        const f32x2 sr = mul2(vr, nr2), si = mul2(vi, nr2);
+        const f32x2 srs = swap2(sr), sis = swap2(si);
 #pragma unroll
         for (int li = S; li < RT * (mi + 1); ++li) {
             CBlk &b = A[M::blk(mi, li)];
             b.dr = fma2(si, ci[li - S], fma2(sr, cr[li - S], b.dr));
-            b.di = fma2(pr, ci[li - S], fma2(si, cr[li - S], b.di));
+            b.di = fma2(sr, nci[li - S], fma2(si, cr[li - S], b.di));
             b.er = fma2(sis, ci[li - S], fma2(srs, cr[li - S], b.er));
-            b.ei = fma2(prs, ci[li - S], fma2(sis, cr[li - S], b.ei));
+            b.ei = fma2(srs, nci[li - S], fma2(sis, cr[li - S], b.ei));
         }
     }
 }
@@ -253,7 +256,7 @@ __device__ __forceinline__ void tile_sweep_step(RBlk (&K)[Tile<G, NL>::NB], cons
 #pragma unroll
     for (int mi = 0; mi < NL; ++mi) {
         const f32x2 v = lds2(vb + 8u * (uint32_t)(LRN * mi + L.lr));
-        const f32x2 s = mul2(v, pk(nr, nr)), ss = pk(nr * hi2(v), nr * lo2(v));
+        const f32x2 s = mul2(v, pk(nr, nr)), ss = swap2(s);
 #pragma unroll
         for (int li = 0; li < RT * (mi + 1); ++li) {
             RBlk &b = K[M::blk(mi, li)];

@@ -29,10 +29,12 @@
 // within the band of the 1e-6 test, |C| not positive definite, a shift above
 // lambda_1, slow convergence -- the pixel goes on a list for pixel_solve, which decides
 // as it always did.  Solve kernels on GB300: 2048^2, N = 30, 11 x 21, 91.9 ->
-// 50.9 ms; 384 x 320, N = 64, ill-conditioned, 37.7 -> 9.7 ms; 333 x 517, N = 23,
-// 2.77 -> 1.34 ms; 1023 x 777, N = 15, 4.29 -> 3.18 ms.  The FMA pipe bounds it (a
+// 47.8 ms; 384 x 320, N = 64, ill-conditioned, 37.7 -> 9.1 ms; 333 x 517, N = 23,
+// 2.77 -> 1.27 ms; 1023 x 777, N = 15, 4.29 -> 3.00 ms.  The FMA pipe bounds it (a
 // packed multiply-add holds it for 2.3 clocks), then instruction fetch: swaps and signs
 // are therefore moves and bit operations, not products (1024^2, N = 30, 13.75 -> 12.7 ms).
+// Tried and slower: one copy of an elimination or sweep step's code for both columns of a
+// pair, or of the sweep for all pivots (its branches cost more than the fetches: 8 to 15%).
 #pragma once
 #include "f32x2.cuh"
 #include "pixel.cuh"
@@ -334,81 +336,95 @@ __device__ __forceinline__ float tile_inf_norm(const RBlk (&K)[Tile<G, NL>::NB],
 }
 
 // (L D L^H) x = b with the factor of tile_ldl (columns v = l d in W): lane g of the
-// group holds the pair b = rows 2 g, 2 g + 1 in (re, re', im, im').
+// group holds the pair b = rows 2 g, 2 g + 1 in (re, re', im, im').  Every lane takes
+// its own pair's 2 x 2 step each time, which is the step's result on lane t, and the
+// others take that by shuffle: the pair's factor stays in registers and no lane
+// has to keep its result from later steps.  1023 x 777, N = 15: 3.18 -> 2.99 ms;
+// N = 64: 9.7 -> 9.1 ms; STBAS 256 x 384, N = 45: 4.90 -> 4.47 ms.
 template <int G, int NL>
 __device__ __forceinline__ void tile_solve(const TileLane &L, int tp, float &b0r, float &b1r, float &b0i, float &b1i)
 {
     using M = Tile<G, NL>;
     constexpr int TW = M::TW;
     const int m = L.g;
-    const uint32_t dg = L.mem + M::dg;
+    f32x2 rm, vm;
+    lds4(L.mem + M::dg + 16u * (uint32_t)(m < tp ? m : 0), rm, vm);
+    const float r0 = lo2(rm), r1 = hi2(rm), vr = lo2(vm), vi = hi2(vm);
+    float s0r, s0i, s1r, s1i, y1r, y1i;
+    auto pair_fwd = [&]() {
+        s0r = r0 * b0r;
+        s0i = r0 * b0i;
+        y1r = fmaf(vi, s0i, fmaf(-vr, s0r, b1r));
+        y1i = fmaf(-vi, s0r, fmaf(-vr, s0i, b1i));
+        s1r = r1 * y1r;
+        s1i = r1 * y1i;
+    };
     // forward: y_i -= v_ik y_k / d_k
-#pragma unroll 1
-    for (int t = 0; t < tp; ++t) {
-        f32x2 rr, v10;
-        lds4(dg + 16u * (uint32_t)t, rr, v10);
-        const float r0 = lo2(rr), r1 = hi2(rr), vr = lo2(v10), vi = hi2(v10);
-        const float y0r = __shfl_sync(0xffffffffu, b0r, t, G), y0i = __shfl_sync(0xffffffffu, b0i, t, G);
-        float y1r = __shfl_sync(0xffffffffu, b1r, t, G), y1i = __shfl_sync(0xffffffffu, b1i, t, G);
-        const float s0r = r0 * y0r, s0i = r0 * y0i;
-        y1r = fmaf(vi, s0i, fmaf(-vr, s0r, y1r));
-        y1i = fmaf(-vi, s0r, fmaf(-vr, s0i, y1i));
-        const float s1r = r1 * y1r, s1i = r1 * y1i;
-        if (m == t) { b1r = y1r; b1i = y1i; }
-        const bool low = t < TW / 2;
-        const uint32_t a = L.mem + 16u * (uint32_t)((low ? t : TW - 1 - t) * (TW + 1) + (low ? m : TW - 1 - m));
+    auto fwd = [&](int t, uint32_t a) {
+        pair_fwd();
+        const float p0r = __shfl_sync(0xffffffffu, s0r, t, G), p0i = __shfl_sync(0xffffffffu, s0i, t, G);
+        const float p1r = __shfl_sync(0xffffffffu, s1r, t, G), p1i = __shfl_sync(0xffffffffu, s1i, t, G);
         if (m > t && (M::T == G || m < M::T)) {
             f32x2 ar, ai, cr, ci;
             lds4(a, ar, ai);
             lds4(a + M::PAR, cr, ci);
-            b0r = fmaf(lo2(ai), s0i, fmaf(-lo2(ar), s0r, b0r));
-            b1r = fmaf(hi2(ai), s0i, fmaf(-hi2(ar), s0r, b1r));
-            b0i = fmaf(-lo2(ai), s0r, fmaf(-lo2(ar), s0i, b0i));
-            b1i = fmaf(-hi2(ai), s0r, fmaf(-hi2(ar), s0i, b1i));
-            b0r = fmaf(lo2(ci), s1i, fmaf(-lo2(cr), s1r, b0r));
-            b1r = fmaf(hi2(ci), s1i, fmaf(-hi2(cr), s1r, b1r));
-            b0i = fmaf(-lo2(ci), s1r, fmaf(-lo2(cr), s1i, b0i));
-            b1i = fmaf(-hi2(ci), s1r, fmaf(-hi2(cr), s1i, b1i));
+            b0r = fmaf(lo2(ai), p0i, fmaf(-lo2(ar), p0r, b0r));
+            b1r = fmaf(hi2(ai), p0i, fmaf(-hi2(ar), p0r, b1r));
+            b0i = fmaf(-lo2(ai), p0r, fmaf(-lo2(ar), p0i, b0i));
+            b1i = fmaf(-hi2(ai), p0r, fmaf(-hi2(ar), p0i, b1i));
+            b0r = fmaf(lo2(ci), p1i, fmaf(-lo2(cr), p1r, b0r));
+            b1r = fmaf(hi2(ci), p1i, fmaf(-hi2(cr), p1r, b1r));
+            b0i = fmaf(-lo2(ci), p1r, fmaf(-lo2(cr), p1i, b0i));
+            b1i = fmaf(-hi2(ci), p1r, fmaf(-hi2(cr), p1i, b1i));
         }
-    }
+    };
+    int t = 0;
+    uint32_t a = L.mem + 16u * (uint32_t)m;
+#pragma unroll 1
+    for (; t < min(tp, TW / 2); ++t, a += 16u * (TW + 1)) fwd(t, a);
+    a = L.mem + 16u * (uint32_t)((TW / 2 - 1) * (TW + 1) + TW - 1 - m);
+#pragma unroll 1
+    for (; t < tp; ++t, a -= 16u * (TW + 1)) fwd(t, a);
+    pair_fwd();
+    b1r = y1r;
+    b1i = y1i;
     // backward: x_k = (y_k - sum_{j > k} conj(v_jk) x_j) / d_k, y kept undivided
+    float x0r, x0i, x1r, x1i;
+    auto pair_bwd = [&]() {
+        x1r = r1 * b1r;
+        x1i = r1 * b1i;
+        x0r = r0 * fmaf(-vi, x1i, fmaf(-vr, x1r, b0r));      // - conj(v10) x1
+        x0i = r0 * fmaf(vi, x1r, fmaf(-vr, x1i, b0i));
+    };
     const bool mlow = m < TW / 2;
     const uint32_t step = mlow ? 16u : (uint32_t)-16;
-    uint32_t a = L.mem + 16u * (uint32_t)((mlow ? m : TW - 1 - m) * (TW + 1) + (mlow ? 0 : TW - 1)) + step * (uint32_t)(tp - 1);
-    f32x2 rm, vm;
-    lds4(dg + 16u * (uint32_t)(m < tp ? m : 0), rm, vm);
+    a = L.mem + 16u * (uint32_t)((mlow ? m : TW - 1 - m) * (TW + 1) + (mlow ? 0 : TW - 1)) + step * (uint32_t)(tp - 1);
 #pragma unroll 1
-    for (int t = tp - 1; t >= 0; --t, a -= step) {
-        f32x2 rr, v10;
-        lds4(dg + 16u * (uint32_t)t, rr, v10);
-        const float r0 = lo2(rr), r1 = hi2(rr), vr = lo2(v10), vi = hi2(v10);
-        float x0r = __shfl_sync(0xffffffffu, b0r, t, G), x0i = __shfl_sync(0xffffffffu, b0i, t, G);
-        const float x1r = r1 * __shfl_sync(0xffffffffu, b1r, t, G), x1i = r1 * __shfl_sync(0xffffffffu, b1i, t, G);
-        x0r = fmaf(-vi, x1i, fmaf(-vr, x1r, x0r));           // - conj(v10) x1
-        x0i = fmaf(vi, x1r, fmaf(-vr, x1i, x0i));
-        if (m == t) { b0r = x0r; b0i = x0i; }
-        x0r *= r0;
-        x0i *= r0;
+    for (t = tp - 1; t >= 0; --t, a -= step) {
+        pair_bwd();
+        const float p0r = __shfl_sync(0xffffffffu, x0r, t, G), p0i = __shfl_sync(0xffffffffu, x0i, t, G);
+        const float p1r = __shfl_sync(0xffffffffu, x1r, t, G), p1i = __shfl_sync(0xffffffffu, x1i, t, G);
         if (m < t) {
             // columns 2 m and 2 m + 1 at row pair t
             f32x2 ar, ai, cr, ci;
             lds4(a, ar, ai);
             lds4(a + M::PAR, cr, ci);
-            b0r = fmaf(-lo2(ai), x0i, fmaf(-lo2(ar), x0r, b0r));
-            b0i = fmaf(lo2(ai), x0r, fmaf(-lo2(ar), x0i, b0i));
-            b0r = fmaf(-hi2(ai), x1i, fmaf(-hi2(ar), x1r, b0r));
-            b0i = fmaf(hi2(ai), x1r, fmaf(-hi2(ar), x1i, b0i));
-            b1r = fmaf(-lo2(ci), x0i, fmaf(-lo2(cr), x0r, b1r));
-            b1i = fmaf(lo2(ci), x0r, fmaf(-lo2(cr), x0i, b1i));
-            b1r = fmaf(-hi2(ci), x1i, fmaf(-hi2(cr), x1r, b1r));
-            b1i = fmaf(hi2(ci), x1r, fmaf(-hi2(cr), x1i, b1i));
+            b0r = fmaf(-lo2(ai), p0i, fmaf(-lo2(ar), p0r, b0r));
+            b0i = fmaf(lo2(ai), p0r, fmaf(-lo2(ar), p0i, b0i));
+            b0r = fmaf(-hi2(ai), p1i, fmaf(-hi2(ar), p1r, b0r));
+            b0i = fmaf(hi2(ai), p1r, fmaf(-hi2(ar), p1i, b0i));
+            b1r = fmaf(-lo2(ci), p0i, fmaf(-lo2(cr), p0r, b1r));
+            b1i = fmaf(lo2(ci), p0r, fmaf(-lo2(cr), p0i, b1i));
+            b1r = fmaf(-hi2(ci), p1i, fmaf(-hi2(cr), p1r, b1r));
+            b1i = fmaf(hi2(ci), p1r, fmaf(-hi2(cr), p1i, b1i));
         }
     }
-    const float r0 = m < tp ? lo2(rm) : 0.f, r1 = m < tp ? hi2(rm) : 0.f;
-    b0r *= r0;
-    b0i *= r0;
-    b1r *= r1;
-    b1i *= r1;
+    pair_bwd();
+    const bool in = m < tp;
+    b0r = in ? x0r : 0.f;
+    b0i = in ? x0i : 0.f;
+    b1r = in ? x1r : 0.f;
+    b1i = in ? x1i : 0.f;
 }
 
 // outcome of a group's pixel
@@ -629,7 +645,7 @@ __device__ __forceinline__ void tile_finish(const KParams &P, long long pp, cons
                                             bool stbas, float z0r, float z1r, float z0i, float z1i, const float2 (&own)[2])
 {
     using M = Tile<G, NL>;
-    constexpr int RT = M::RT, LRN = M::LRN, NLC = M::NLC;
+    constexpr int RT = M::RT, LRN = M::LRN;
     const int n = P.nb;
     // ---- phase referencing (evd.cpp:738-749) -----------------------------------------
     const int mref = P.mini - 1;
@@ -667,17 +683,18 @@ __device__ __forceinline__ void tile_finish(const KParams &P, long long pp, cons
     // conjugate of the reference's sum over the upper one -----------------------------
     float tr = 0.f, ti = 0.f;
     {
-        f32x2 pr[NLC], pi[NLC];
-#pragma unroll
-        for (int li = 0; li < NLC; ++li) lds4(L.mem + M::z + 16u * (uint32_t)(4 * li + L.lc), pr[li], pi[li]);
-#pragma unroll
+        // rolled: one block's code for all (1024^2, N = 30: 13.1 -> 12.2 ms by instruction fetch)
+        uint32_t ta = taddr;
+#pragma unroll 1
         for (int mi = 0; mi < NL; ++mi) {
             // w_i = sum_j exp(i arg C_ij) ph_j over j < i, rows i (lo) and i' (hi)
             float w0r = 0.f, w0i = 0.f, w1r = 0.f, w1i = 0.f;
-#pragma unroll
-            for (int li = 0; li < RT * (mi + 1); ++li) {
+#pragma unroll 1
+            for (int li = 0; li < RT * (mi + 1); ++li, ta += 8u) {
                 uint32_t w[8];
-                tmem_ld8(taddr + 8u * (uint32_t)M::blk(mi, li), w);
+                tmem_ld8(ta, w);
+                f32x2 pr, pi;
+                lds4(L.mem + M::z + 16u * (uint32_t)(4 * li + L.lc), pr, pi);
                 const int m = LRN * mi + L.lr, l = 4 * li + L.lc;
                 const bool all = li < RT * mi || m > l, some = all || m == l;
                 auto term = [&](int e, float pjr, float pji, bool on, float &ar, float &ai) {
@@ -689,7 +706,7 @@ __device__ __forceinline__ void tile_finish(const KParams &P, long long pp, cons
                         ai = fmaf(vr, pji, fmaf(vi, pjr, ai));
                     }
                 };
-                const float jr = lo2(pr[li]), ji = lo2(pi[li]), kr = hi2(pr[li]), ki = hi2(pi[li]);
+                const float jr = lo2(pr), ji = lo2(pi), kr = hi2(pr), ki = hi2(pi);
                 const int d = stbas ? P.bw - 2 * (m - l) : 1;        // pairs at most the bandwidth apart
                 term(0, jr, ji, all && d >= 0, w0r, w0i);            // (i, j)
                 term(1, kr, ki, all && d >= 0, w1r, w1i);            // (i', j')
@@ -763,17 +780,26 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
                 K[b].e = pk(a[2], a[3]);
             }
             tile_on_diag<G, NL>(L, [&](int, int b) { K[b].d = pk(1.f, 1.f); });
-            const float anorm = tile_inf_norm<G, NL>(K, L);
             bool ok = true;
-            tile_sweep_seg<G, NL, 0>(K, L, tp, ok);
-            // inv|C| = -K, its diagonal 2 - K
+            // norms of |C| and inv|C|; at 25 to 32 dates with one copy of the code, which
+            // the instruction cache just does not hold otherwise (1024^2, N = 30: 12.3 ->
+            // 11.95 ms; N = 15, where it fits: 3.00 -> 3.05 ms)
+            float anorm = 0.f, xnorm = 0.f;
+#pragma unroll(NL == 4 ? 1 : 2)
+            for (int rep = 0; rep < 2; ++rep) {
+                if (rep == 1) {
+                    tile_sweep_seg<G, NL, 0>(K, L, tp, ok);
+                    // inv|C| = -K, its diagonal 2 - K
 #pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                K[b].d ^= 0x8000000080000000ull;
-                K[b].e ^= 0x8000000080000000ull;
+                    for (int b = 0; b < NB; ++b) {
+                        K[b].d ^= 0x8000000080000000ull;
+                        K[b].e ^= 0x8000000080000000ull;
+                    }
+                    tile_on_diag<G, NL>(L, [&](int, int b) { K[b].d = add2(K[b].d, pk(2.f, 2.f)); });
+                }
+                anorm = xnorm;
+                xnorm = tile_inf_norm<G, NL>(K, L);
             }
-            tile_on_diag<G, NL>(L, [&](int, int b) { K[b].d = add2(K[b].d, pk(2.f, 2.f)); });
-            const float xnorm = tile_inf_norm<G, NL>(K, L);
             if (state == TILE_RUN && !ok) state = TILE_GENERAL;
             if (state == TILE_RUN && (!(anorm * xnorm <= P.cond_max) || (!plink && !(1.f / xnorm > thr + amb * (float)n)))) {
                 // condition too large for an FP32 inverse, or 1/||inv|C||| within the band of 1e-6

@@ -29,8 +29,8 @@
 // within the band of the 1e-6 test, |C| not positive definite, a shift above
 // lambda_1, slow convergence -- the pixel goes on a list for pixel_solve, which decides
 // as it always did.  Solve kernels on GB300: 2048^2, N = 30, 11 x 21, 91.9 ->
-// 47.8 ms; 384 x 320, N = 64, ill-conditioned, 37.7 -> 9.1 ms; 333 x 517, N = 23,
-// 2.77 -> 1.27 ms; 1023 x 777, N = 15, 4.29 -> 3.00 ms.  The FMA pipe bounds it (a
+// 47.2 ms; 384 x 320, N = 64, ill-conditioned, 37.7 -> 9.0 ms; 333 x 517, N = 23,
+// 2.77 -> 1.21 ms; 1023 x 777, N = 15, 4.29 -> 2.95 ms.  The FMA pipe bounds it (a
 // packed multiply-add holds it for 2.3 clocks), then instruction fetch: swaps and signs
 // are therefore moves and bit operations, not products (1024^2, N = 30, 13.75 -> 12.7 ms).
 // Tried and slower: one copy of an elimination or sweep step's code for both columns of a
@@ -47,6 +47,14 @@ __device__ __forceinline__ float rcp_fast(float a)
 {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+// rsqrtf of a normal number (the same result without its steps for subnormal ones)
+__device__ __forceinline__ float rsqrt_fast(float a)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
 
@@ -508,12 +516,19 @@ __device__ __forceinline__ int tile_begin(const KParams &P, long long pp, const 
     bool bad = false;
     const uint32_t yv = L.mem + M::v;
     tile_on_diag<G, NL>(L, [&](int x, int b) {
-        const int i = 2 * (LRN * x + L.lr);
-        const float p0 = lo2(A[b].dr), p1 = hi2(A[b].dr);
+        sts2(yv + 8u * (uint32_t)(LRN * x + L.lr), lo2(A[b].dr), hi2(A[b].dr));
+    });
+    __syncwarp();
+    // 1/sqrt(P), a pair per lane: on the diagonal lanes it is NL times the code and the
+    // work (N = 15: 3.00 -> 2.95 ms with rsqrt_fast in |C|, N = 23: 1.25 -> 1.21 ms)
+    if (L.g < M::T) {
+        const int i = 2 * L.g;
+        const f32x2 p = lds2(yv + 8u * (uint32_t)L.g);
+        const float p0 = lo2(p), p1 = hi2(p);
         bad |= i < n && (!(p0 > 0.f) || !isfinite(p0));
         bad |= i + 1 < n && (!(p1 > 0.f) || !isfinite(p1));
-        sts2(yv + 8u * (uint32_t)(LRN * x + L.lr), i < n ? 1.f / sqrtf(p0) : 0.f, i + 1 < n ? 1.f / sqrtf(p1) : 0.f);
-    });
+        sts2(yv + 8u * (uint32_t)L.g, i < n ? 1.f / sqrtf(p0) : 0.f, i + 1 < n ? 1.f / sqrtf(p1) : 0.f);
+    }
     __syncwarp();
     float fs = 0.f;
     {
@@ -774,7 +789,7 @@ __device__ __forceinline__ int tile_mle(const KParams &P, long long pp, const Ti
                     // entries: D lo, D hi, E lo, E hi
                     const float x = __uint_as_float(w[(e & 1) + 4 * (e >> 1)]), y = __uint_as_float(w[(e & 1) + 4 * (e >> 1) + 2]);
                     const float m2 = fmaf(x, x, y * y);
-                    a[e] = m2 * rsqrtf(fmaxf(m2, 1e-37f));
+                    a[e] = m2 * rsqrt_fast(fmaxf(m2, 1e-37f));
                 }
                 K[b].d = pk(a[0], a[1]);
                 K[b].e = pk(a[2], a[3]);

@@ -56,10 +56,10 @@ METRIC = "phase-linked px/s (N=30, 11x21)"
 # what the ncu captures under profiles/ show for each kernel
 # what the ncu captures under profiles/ show for each kernel
 BOUND_NOTES = {
-    "solve": "instruction issue (one warp per pixel; per-pixel FP32 factorisations, sweep inverse and "
-             "triangular solves); DRAM and tensor pipe idle",
-    "gram": "operand build on the CUDA cores with 8 warps/SM and a barrier per chunk; tensor pipe partly idle",
-    "fp32": "per-pixel FP32 gather, Gamma and eigen-solves: latency/issue-bound",
+    "solve": "instruction issue and the FMA pipe (two pixels per warp, matrices in registers; FP32 factorisations, "
+             "sweep inverse and triangular solves); DRAM and tensor pipe idle",
+    "gram": "operand build on the CUDA cores, two warp groups on alternate chunks; tensor pipe partly idle",
+    "fp32": "per-pixel FP32 gather, Gamma and eigen-solves (windows the Gamma kernel does not take)",
 }
 # FP32 flops of the MLE eigen-solves per pixel as implemented, for n dates and
 # `solves` pairs of triangular solves: the Cholesky test of C - 1e-6 I and the
@@ -724,14 +724,11 @@ def main():
     flops = float((4.0 * NB * (NB + 1) * shp[centre]).sum())     # Gamma, Hermitian half
     alg_bytes = npx * (16 * NB + 4 * nmap.shape[2] + 12)
     km = head["kernel_ms"]
-    if args.precision == "mixed":
-        # dominant kernel of the mixed form by device time
-        dom = "solve" if km["solve"] >= km["gram"] else "gram"
-    else:
-        dom = "fp32"
+    # dominant kernel by device time (the FP64 list apart)
+    dom = max(("solve", "gram", "fp32"), key=lambda k: km.get(k, 0.0))
     names = {"fp32": "k_pixels<float> (FP32 SIMT gather + Gamma + eigen-solves)",
-             "gram": "k_gram_box (tcgen05 bf16 hi/lo Gamma, TMEM accumulate)",
-             "solve": "k_solve (warp eigen-solves from the Gamma records)"}
+             "gram": "k_gram_box (tcgen05 Gamma of bf16 parts, TMEM accumulate)",
+             "solve": "k_solve (register eigen-solves from the Gamma records)"}
     k_ms = km[dom]
     kc = kernel_counters()
     ent = kc.get(dom) or {}

@@ -19,14 +19,14 @@
 //       form's results against 64 bits is that of the plain FP32 kernel or
 //       less (STBAS, N = 48: phases 2.9e-7 rad RMS from the oracle, plain kernel
 //       2.8e-7; EVD 9.3e-7 against 1.0e-6), and at 1024^2, N = 30, 11 x 21 its Gamma
-//       takes 6.7 ms (two parts: 4.6) of a 22.2 ms call; the plain kernel, 20 of
+//       takes 5.8 ms (two parts: 4.3) of an 18.7 ms call; the plain kernel, 20 of
 //       whose 32 lanes hold sums, took 52 of 54 ms.
 // Each outer product is formed once per tile instead of once for every pixel
 // that uses it.  One thread issues tcgen05.mma (M = 128 pixels, N <= 256
 // Gamma entries, K = 16 samples) into one of two tensor-memory accumulators;
 // the Gamma entries are processed in passes of 512 columns, each pass over
-// the tile's samples in chunks of 32 (two operand stages, one CTA barrier
-// per chunk).
+// the tile's samples in chunks of 32, which two warp groups build in turn, each
+// into its own operand stage.
 //
 // Column order (the Gamma record read by the eigen kernel): dates padded to an
 // even count and grouped in pairs; block (a, b), a <= b, row-major over the

@@ -2056,6 +2056,12 @@ __device__ bool pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
         if (!plink && lam < thr) { put_code(P, pp, lane, -7); return true; }
     }
 
+    if constexpr (std::is_same<T, ff>::value) {
+        // beyond FP32's exponent range on the way (FP64's is wider)
+        const bool fin = isfinite(lam) && isfinite(z0.x) && isfinite(z0.y) && isfinite(z1.x) && isfinite(z1.y);
+        if (!__all_sync(0xffffffffu, fin)) return open();
+    }
+
     // ---- phase referencing (evd.cpp:738-749) ------------------------------
     const int mref = P.mini - 1;
     C2<T> zr;

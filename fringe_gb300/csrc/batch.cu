@@ -274,6 +274,7 @@ struct MixedWave {
     int ent_first[3] = {0, 0, 0}, ent_count[3] = {0, 0, 0};
     long long ent_total[3] = {0, 0, 0};
     int ent_kinds[3] = {0, 0, 0};
+    std::vector<fpl::KParams> own;       // pieces with solve launches of their own
 };
 
 struct fpl_batch {
@@ -324,6 +325,8 @@ int batch_enqueue(fpl_batch *b, cudaStream_t st)
                                                           w.ent_total[c], w.ent_kinds[c], ctx->num_sms, st,
                                                           b->mixed_warps[c]) != cudaSuccess)
                 return FPL_ERR_CUDA;
+        for (const fpl::KParams &P : w.own)
+            if (fpl::launch_solve(P, ctx->num_sms, st) != cudaSuccess) return FPL_ERR_CUDA;
     }
     for (const BatchClass &k : b->classes)
         if (fpl::launch_batch64(k.np, b->d_table + k.first, k.count, ctx->num_sms, st) != cudaSuccess)
@@ -509,6 +512,10 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                     mw.ent_first[c] = (int)ments.size();
                     for (int i = 0; i < np_; ++i) {
                         if (wave_of[i] != (int)w || fpl::pick_np(pp[i].nb) != npd) continue;
+                        if (pp[i].npix >= fpl::kOwnSolvePx) {
+                            mw.own.push_back(pp[i]);
+                            continue;
+                        }
                         fpl::BatchEntry en;
                         en.P = pp[i];
                         en.px_offset = mw.ent_total[c];
@@ -548,6 +555,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 return FPL_ERR_CUDA;
             }
             // kernel attributes are set before any capture
+            if (fpl::prepare_solve() != cudaSuccess) { fpl_batch_destroy(b); return FPL_ERR_CUDA; }
             for (int c = 0; c < 3; ++c)
                 if (fpl::prepare_mixed_batch(16 << c) != cudaSuccess) { fpl_batch_destroy(b); return FPL_ERR_CUDA; }
         }

@@ -35,6 +35,16 @@ cudaError_t launch_gram_box(const KParams &P, int num_sms, cudaStream_t st);
 
 // eigen-solves and outputs from P.cbuf / P.cinfo
 cudaError_t launch_solve(const KParams &P, int num_sms, cudaStream_t st);
+// sets the attributes of its kernels (before a capture)
+cudaError_t prepare_solve();
+// Pieces of a batch or serving wave from this size on get solve launches of
+// their own: the kernel for their depth (the combined one has one shape for 17 to 32
+// and one for 33 to 64 dates) with its parameters in constant memory.  20 pieces of
+// 10 to 45 dates, combined -> own launches: 512^2 106 -> 81 ms, 256^2 30.0 -> 23.9 ms,
+// 180^2 17.1 -> 14.7 ms; of 30 dates all: 512^2 79.0 -> 71.1, 256^2 23.3 -> 22.0, but
+// 180^2 14.08 -> 14.14 and 128^2 9.5 -> 10.2 ms; of 10 dates: 256^2 6.23 -> 6.06,
+// 128^2 1.81 -> 2.09 ms.  From 2^16 pixels on every batch gains.
+constexpr long long kOwnSolvePx = 1ll << 16;
 
 // batched: a launch of the Gamma kernel covers gram_box_tiles(P)
 // tiles and needs gram_box_smem bytes of shared memory.

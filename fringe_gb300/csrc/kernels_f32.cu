@@ -57,6 +57,15 @@ int solve_max_warps(int np)
     return 1;
 }
 
+cudaError_t prepare_solve()
+{
+    const cudaError_t e[5] = {prepare_solve_t<16, 2>(), prepare_solve_t<16, 3>(), prepare_solve_t<16, 4>(),
+                              prepare_solve_t<32, 3>(), prepare_solve_t<32, 4>()};
+    for (cudaError_t r : e)
+        if (r != cudaSuccess) return r;
+    return cudaSuccess;
+}
+
 int solve_kind(const KParams &P) { return 1 << tile_kind(P); }
 
 cudaError_t launch_solve_batch(int np, const BatchEntry *ents, int nent, long long total, int kinds, int num_sms,

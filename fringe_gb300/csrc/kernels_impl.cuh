@@ -249,10 +249,22 @@ static long long solve_grid(long long items, int num_sms, int *warps)
 }
 
 template <int NP>
-static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
+static cudaError_t configure_rest()
 {
     static bool configured[64] = {false};
-    cudaError_t e = solve_configure(k_rest<NP>, configured);
+    return solve_configure(k_rest<NP>, configured);
+}
+template <int G, int NL, int KIND>
+static cudaError_t configure_solve_kind()
+{
+    static bool configured[64] = {false};
+    return solve_configure(k_solve<G, NL, KIND>, configured);
+}
+
+template <int NP>
+static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
+{
+    cudaError_t e = configure_rest<NP>();
     if (e != cudaSuccess) return e;
     int warps = rest_max_warps<NP>();
     const long long blocks = solve_grid(P.npix, num_sms, &warps);
@@ -263,8 +275,7 @@ static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
 template <int G, int NL, int KIND>
 static cudaError_t launch_solve_kind(const KParams &P, int num_sms, cudaStream_t st)
 {
-    static bool configured[64] = {false};
-    cudaError_t e = solve_configure(k_solve<G, NL, KIND>, configured);
+    cudaError_t e = configure_solve_kind<G, NL, KIND>();
     if (e != cudaSuccess) return e;
     int warps = solve_warps<G, NL>();
     const long long blocks = solve_grid(SolveShape<G, NL>::items(P.npix), num_sms, &warps);
@@ -280,6 +291,15 @@ static cudaError_t launch_solve_t(const KParams &P, int num_sms, cudaStream_t st
     if (tile_kind(P) == TK_MLE) e = launch_solve_kind<G, NL, TK_MLE>(P, num_sms, st);
     else if (tile_kind(P) == TK_EVD) e = launch_solve_kind<G, NL, TK_EVD>(P, num_sms, st);
     return e != cudaSuccess ? e : launch_rest_t<NP>(P, num_sms, st);
+}
+
+template <int G, int NL>
+static cudaError_t prepare_solve_t()
+{
+    constexpr int NP = G == 32 ? 64 : (NL == 2 ? 16 : 32);
+    cudaError_t e = configure_solve_kind<G, NL, TK_MLE>();
+    if (e == cudaSuccess) e = configure_solve_kind<G, NL, TK_EVD>();
+    return e != cudaSuccess ? e : configure_rest<NP>();
 }
 
 // attributes of the batch kernels, set once per device

@@ -199,7 +199,10 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
         const int ra = j->next_row, rb = std::min(j->r1, ra + rows);
         j->next_row = rb;
         if (!j->started) { j->started = true; j->t_first = clk::now(); }
-        const int tiled = fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x) ? 1 : 0;
+        // 0: plain kernel, 1: combined solve launch, 2: one of its own
+        const int tiled = !fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x) ? 0
+                          : (long long)(rb - ra) * j->host.cols >= fpl::kOwnSolvePx                               ? 2
+                                                                                                                   : 1;
         pieces.push_back({j, ra, rb, fpl::pick_np(j->host.nbands), tiled});
         total += (long long)(rb - ra) * j->host.cols;
     }
@@ -299,7 +302,10 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
             n_px += s->h_table[e++].P.npix;
         }
         if (fpl::configure_np(np) != cudaSuccess) return false;
-        if (tiled) {
+        if (tiled == 2) {
+            for (size_t k = first; k < e; ++k)
+                if (fpl::launch_solve(s->h_table[k].P, s->num_sms, s->s_compute) != cudaSuccess) return false;
+        } else if (tiled) {
             if (fpl::prepare_mixed_batch(np) != cudaSuccess) return false;
             if (fpl::launch_solve_batch(np, s->d_table + first, (int)(e - first), n_px, kinds, s->num_sms, s->s_compute) !=
                 cudaSuccess)

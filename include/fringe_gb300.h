@@ -127,7 +127,7 @@ typedef struct {
 /* statistics of the last fpl_run on a context */
 typedef struct {
     long long pixels;            /* pixels in the row range          */
-    long long fp64_pixels;       /* pixels settled by the FP64 path  */
+    long long fp64_pixels;       /* pixels FP32 left undecided (settled in float-float or FP64) */
     long long mixed_fp64_inverse;/* MLE pixels whose |G| inverse ran in FP64 */
     long long slow_path_pixels;  /* pixels that left the fast eigen path (second shift or Householder) */
     float kernel_ms;             /* device time of the compute kernels */
@@ -156,7 +156,7 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out);
 /* ---- batches of jobs ------------------------------------------------------
  * Many device-memory jobs -- scenes or ministacks of different size, stack
  * depth, window and method -- run as waves of persistent launches, followed by
- * one FP64 settle launch per padded depth (16 / 32 / 64 dates).  Replaces running the evd module once
+ * one launch over the undecided pixels per padded depth (16 / 32 / 64 dates).  Replaces running the evd module once
  * per ministack (src/sequential/sequential.py:193-254 calls evd_process in a
  * loop).  FPL_BATCH_GRAPH captures the launch sequence into a CUDA graph at
  * creation; fpl_batch_run replays it (buffers are fixed, their contents may
@@ -253,7 +253,7 @@ enum fpl_kernel_tag {
     FPL_KTAG_FP32 = 0,       /* plain FP32 pixel kernel (gather + Gamma + solve) */
     FPL_KTAG_GRAM = 1,       /* tensor-core Gamma records                        */
     FPL_KTAG_SOLVE = 2,      /* eigen-solves from the records                    */
-    FPL_KTAG_FP64 = 3,       /* FP64 settle pass                                 */
+    FPL_KTAG_FP64 = 3,       /* undecided pixels (float-float, then FP64)          */
     FPL_KTAG_COUNT = 4
 };
 int fpl_ctx_profile_kernels(const fpl_ctx *ctx, double *ms, int count);

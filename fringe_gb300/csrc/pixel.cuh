@@ -171,8 +171,10 @@ template <typename T, int NP> struct Lay {
     static constexpr int LD = NP + 1;        // matrix row stride (odd: conflict-free columns)
     static constexpr int XS = NP + 2;        // staging row stride in float2 (16-byte rows)
     static constexpr size_t mat = sizeof(C2<T>) * NP * LD;
+    static constexpr int SR = 32;                                     // samples staged at a time
     static constexpr size_t wm = 0;                                   // work: staging / Cholesky / M / tridiag
-    static constexpr size_t wm_bytes = align16(cmax(mat, sizeof(float2) * 32 * XS));
+    static constexpr size_t xs = wm;                                  // gather staging
+    static constexpr size_t wm_bytes = align16(cmax(mat, sizeof(float2) * SR * XS));
     static constexpr size_t xr = wm + align16(mat / 2);               // real sweep matrix: upper half of wm
     static constexpr size_t vv = wm + wm_bytes;                       // complex vector v
     static constexpr size_t ww = align16(vv + sizeof(C2<T>) * NP);    // complex vector w
@@ -190,22 +192,25 @@ template <typename T, int NP> struct Lay {
     static constexpr size_t bytes = cm + align16(mat);
 };
 
-// FP64 at 64 dates keeps C in tensor memory during the eigen-solve (see
-// CInTmem), so the coherence needs shared memory only while Gamma is summed
-// and normalised: it sits right after the gather staging, over the work
-// matrix (which the solve uses only after C has been copied out), and the
-// vectors follow it.  91.6 KB per warp instead of 141 KB: two warps per SM.
+// FP64 and float-float at 64 dates keep C in tensor memory during the
+// eigen-solve (see CInTmem), so the coherence needs shared memory only while Gamma is
+// summed and normalised: it takes the place of the work matrix (which the
+// solve uses only after C has been copied out).  The gather staging holds 16 samples
+// at a time and takes the place of the vectors (which are used only after
+// the gather).  75.0 KB per warp, three warps per SM; with the staging apart it was
+// 91.6 KB and two (384x320, 1451 entries: 9.2 -> 7.9 ms; 300x400, Voronoi: 22.3 ->
+// 15.9 ms).
 template <typename T> struct Lay64W {
     static constexpr int NP = 64;
     static constexpr int LD = NP + 1;
     static constexpr int XS = NP + 2;
+    static constexpr int SR = 16;                                     // samples staged at a time
     static constexpr size_t mat = sizeof(C2<T>) * NP * LD;
     static constexpr size_t wm = 0;
-    static constexpr size_t stage = align16(sizeof(float2) * 32 * XS);  // gather staging at wm
-    static constexpr size_t wm_bytes = align16(cmax(mat, stage));
     static constexpr size_t xr = wm + align16(mat / 2);
-    static constexpr size_t cm = stage;                               // Gamma / C while it is formed
-    static constexpr size_t vv = cmax(wm + wm_bytes, cm + align16(mat));
+    static constexpr size_t cm = wm;                                  // Gamma / C while it is formed
+    static constexpr size_t vv = align16(mat);
+    static constexpr size_t xs = vv;                                  // gather staging
     static constexpr size_t ww = align16(vv + sizeof(C2<T>) * NP);
     static constexpr size_t tu = align16(ww + sizeof(C2<T>) * NP);
     static constexpr size_t dd = align16(tu + sizeof(C2<T>) * NP);
@@ -214,19 +219,16 @@ template <typename T> struct Lay64W {
     static constexpr size_t yy = align16(e2 + sizeof(T) * NP);
     static constexpr size_t wk = align16(yy + sizeof(T) * NP);
     static constexpr size_t ph = align16(wk + sizeof(T) * 5 * NP);
-    static constexpr size_t bytes_noc = align16(ph + sizeof(float2) * NP);
+    static constexpr size_t bytes_noc = cmax(align16(ph + sizeof(float2) * NP), xs + align16(sizeof(float2) * SR * XS));
     static constexpr size_t bytes = bytes_noc;
 };
 template <> struct Lay<double, 64> : Lay64W<double> {};
 template <> struct Lay<ff, 64> : Lay64W<ff> {};
 
-// while Gamma is summed the gather staging, the coherence and the vectors
-// (1/sqrt(P) among them) are all live, so they must not overlap; the work
-// matrix may overlap the coherence (it is used only after C moved out)
-static_assert(Lay<double, 64>::cm >= Lay<double, 64>::wm + Lay<double, 64>::stage, "staging overlaps C");
-static_assert(Lay<double, 64>::vv >= Lay<double, 64>::cm + Lay<double, 64>::mat, "vectors overlap C");
-static_assert(Lay<double, 64>::vv >= Lay<double, 64>::wm + Lay<double, 64>::wm_bytes, "vectors overlap W");
-static_assert(2 * Lay<double, 64>::bytes <= 224 * 1024, "two warps per CTA");
+// while Gamma is summed the staging and the coherence are both live, so they
+// must not overlap; 1/sqrt(P), in the vectors, is formed after the last sample
+static_assert(Lay<double, 64>::xs >= Lay<double, 64>::cm + Lay<double, 64>::mat, "staging overlaps C");
+static_assert(3 * Lay<double, 64>::bytes <= 224 * 1024, "three warps per CTA");
 
 // kernels whose warps hold C in tensor memory in the FP64 and float-float forms
 template <typename T, int NP> struct CInTmem {
@@ -1558,12 +1560,7 @@ __device__ int pixel_coherence(const KParams &P, long long pp, unsigned char *sm
 
     static_assert(!CRowsTmemF<T, NP>::value || PASSES == 1, "C over the staging needs Gamma in registers");
     C2<T> *Cm = reinterpret_cast<C2<T> *>(sm + CmOffset<T, NP>::value);
-    C2<T> *Wm = reinterpret_cast<C2<T> *>(sm + L::wm);
-    float2 *Xs = reinterpret_cast<float2 *>(sm + L::wm);
-    T *Xr = reinterpret_cast<T *>(sm + L::xr);
-    T *yv = reinterpret_cast<T *>(sm + L::yy);
-    C2<T> *col = reinterpret_cast<C2<T> *>(sm + L::vv);
-    float2 *phs = reinterpret_cast<float2 *>(sm + L::ph);
+    float2 *Xs = reinterpret_cast<float2 *>(sm + L::xs);
 
     const int n = P.nb;
     const int cols = P.cols, rows = P.rows;
@@ -1626,57 +1623,60 @@ __device__ int pixel_coherence(const KParams &P, long long pp, unsigned char *sm
         const unsigned m = __ballot_sync(0xffffffffu, set);
         const int cnt = __popc(m);
         if (cnt == 0) continue;
-        __syncwarp();
-        if (set) {
-            const int rk = __popc(m & lt);
-            const float2 *src = P.stack + q;
-            float2 *dst = Xs + rk * XS;
-#pragma unroll 4
-            for (int t = 0; t < n; ++t) {
-                dst[t] = __ldg(src);
-                src += plane;
-            }
-        }
-        __syncwarp();
         npix += cnt;
-#pragma unroll
-        for (int ps = 0; ps < PASSES; ++ps) {
-            if (!bAct[ps]) continue;
-            const int r0 = BR * bR[ps], c0 = BC * bC[ps];
-            if (PASSES > 1) {
-#pragma unroll
-                for (int i = 0; i < BR; ++i)
-#pragma unroll
-                    for (int j = 0; j < BC; ++j) acc[i][j] = Cm[(r0 + i) * LD + c0 + j];
-            }
-            for (int s = 0; s < cnt; ++s) {
-                const float2 *xs = Xs + s * XS;
-                float2 xr[BR], xc[BC];
-#pragma unroll
-                for (int i = 0; i < BR; i += 2) {
-                    float4 v = *reinterpret_cast<const float4 *>(xs + r0 + i);
-                    xr[i] = make_float2(v.x, v.y);
-                    xr[i + 1] = make_float2(v.z, v.w);
+        const int rk = __popc(m & lt);
+        for (int h0 = 0; h0 < cnt; h0 += L::SR) {               // once where all 32 fit
+            const int take = min(cnt - h0, L::SR);
+            __syncwarp();
+            if (set && rk >= h0 && rk < h0 + L::SR) {
+                const float2 *src = P.stack + q;
+                float2 *dst = Xs + (rk - h0) * XS;
+#pragma unroll 4
+                for (int t = 0; t < n; ++t) {
+                    dst[t] = __ldg(src);
+                    src += plane;
                 }
+            }
+            __syncwarp();
 #pragma unroll
-                for (int j = 0; j < BC; j += 2) {
-                    float4 v = *reinterpret_cast<const float4 *>(xs + c0 + j);
-                    xc[j] = make_float2(v.x, v.y);
-                    xc[j + 1] = make_float2(v.z, v.w);
+            for (int ps = 0; ps < PASSES; ++ps) {
+                if (!bAct[ps]) continue;
+                const int r0 = BR * bR[ps], c0 = BC * bC[ps];
+                if (PASSES > 1) {
+#pragma unroll
+                    for (int i = 0; i < BR; ++i)
+#pragma unroll
+                        for (int j = 0; j < BC; ++j) acc[i][j] = Cm[(r0 + i) * LD + c0 + j];
                 }
+                for (int s = 0; s < take; ++s) {
+                    const float2 *xs = Xs + s * XS;
+                    float2 xr[BR], xc[BC];
 #pragma unroll
-                for (int i = 0; i < BR; ++i)
+                    for (int i = 0; i < BR; i += 2) {
+                        float4 v = *reinterpret_cast<const float4 *>(xs + r0 + i);
+                        xr[i] = make_float2(v.x, v.y);
+                        xr[i + 1] = make_float2(v.z, v.w);
+                    }
 #pragma unroll
-                    for (int j = 0; j < BC; ++j) acc_prod<T>(acc[i][j], xr[i], xc[j]);
+                    for (int j = 0; j < BC; j += 2) {
+                        float4 v = *reinterpret_cast<const float4 *>(xs + c0 + j);
+                        xc[j] = make_float2(v.x, v.y);
+                        xc[j + 1] = make_float2(v.z, v.w);
+                    }
+#pragma unroll
+                    for (int i = 0; i < BR; ++i)
+#pragma unroll
+                        for (int j = 0; j < BC; ++j) acc_prod<T>(acc[i][j], xr[i], xc[j]);
+                }
+                if (PASSES > 1) {
+#pragma unroll
+                    for (int i = 0; i < BR; ++i)
+#pragma unroll
+                        for (int j = 0; j < BC; ++j) Cm[(r0 + i) * LD + c0 + j] = acc[i][j];
+                }
             }
-            if (PASSES > 1) {
-#pragma unroll
-                for (int i = 0; i < BR; ++i)
-#pragma unroll
-                    for (int j = 0; j < BC; ++j) Cm[(r0 + i) * LD + c0 + j] = acc[i][j];
-            }
+            __syncwarp();
         }
-        __syncwarp();
     }
     if (PASSES == 1 && bAct[0]) {
         const int r0 = BR * bR[0], c0 = BC * bC[0];
@@ -2348,9 +2348,9 @@ __device__ bool process_pixel(const KParams &P, long long pp, unsigned char *sm,
 // A work-list entry: float-float, then FP64 where that leaves the pixel
 // open (out of line: 6 of 396 entries do at 333x517 with 23 dates, 5 of 1451 at
 // 384x320 with 64).  The FP64 pipe's two operations per SM and clock bound the
-// list before; float-float is bound by the latency of one pixel's chain (two
+// list before; float-float is bound by the latency of one pixel's chain (three
 // warps per SM at 64 dates, whose matrix takes 67 KB of shared memory).  List kernel
-// alone, FP64 -> float-float: 384x320, 64 dates 26.1 -> 9.7 ms (1451 entries);
+// alone, FP64 -> float-float: 384x320, 64 dates 26.1 -> 7.9 ms (1451 entries);
 // 1024x1024, 30 dates 1.6 -> 0.45 ms (788); 1023x777, 15 dates 0.44 -> 0.19 ms (15).
 // Against FP64 for every pixel (n 10..64) the codes are the same and the
 // phases differ by at most 1e-7 rad, FP32's rounding of the output.

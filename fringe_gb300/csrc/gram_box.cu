@@ -571,27 +571,33 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
             }
         }
         __syncwarp();
-        // the pass's MMAs: its last step and the one before
+        // The pass's MMAs: its last step but one, then the last.  A parity wait for step
+        // n tells phases n / 2 and n / 2 - 1 of its barrier apart only where step n - 2 is
+        // known to be done.  For step last - 1 both groups know that (one waited for
+        // last - 3 itself, the other for last - 2, which is issued after last - 3 is
+        // done); for step last it follows from last - 1, which is issued after
+        // last - 2 is done.
         {
             const unsigned last = st.base + (unsigned)((pass + 1) * nchunk - 1);
-            if (!late) late = box_wait(bars->empty, last, dead);
             if (!late && last >= 1) late = box_wait(bars->empty, last - 1, dead);
-        }
-        if (pass == 0 && tid < BX_M) {
-            // every sample of the tile has been stored (the last one before
-            // the last chunk's barrier): a pixel with an out-of-range SHP
-            // sample goes to the FP64 path
-            const int m = tid;
-            uint32_t hit = 0;
-            for (int w = 0; w < W; ++w) hit |= umask[m * W + w] & tbad[w];
-            pdefer[m] = hit != 0;
+            if (!late) late = box_wait(bars->empty, last, dead);
         }
         if (__syncthreads_or(late)) { st.timed_out = true; break; }
         fence_after_sync();
         if (pass == 0) {
+            // every sample of the tile has been checked and stored: both groups
+            // have passed the barrier above.  A pixel with an out-of-range SHP
+            // sample goes to the FP64 path.
+            if (tid < BX_M) {
+                const int m = tid;
+                uint32_t hit = 0;
+                for (int w = 0; w < W; ++w) hit |= umask[m * W + w] & tbad[w];
+                pdefer[m] = hit != 0;
+            }
             uint32_t any = 0;
             for (int w = 0; w < W; ++w) any |= tbad[w];
             clean = any == 0;
+            __syncthreads();
         }
         // ---- epilogue: warp w reads TMEM lanes 32(w%4).., every fourth 32 columns ----
         // A lane holds its own pixel's columns; they are written out through

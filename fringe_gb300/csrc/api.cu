@@ -56,6 +56,30 @@ int grow(fpl_ctx *ctx, void **p, size_t *cap, size_t need)
     return FPL_OK;
 }
 
+// Scratch that a run's kernels refer to.  A capture records its address in the
+// caller's graph, which may be replayed after the scratch has been outgrown, so from
+// then on it stays allocated until the context is destroyed.  While capturing
+// nothing is freed, and the allocation is allowed whatever the capture's mode.
+int grow_run(fpl_ctx *ctx, RunScratch &s, size_t need, bool capturing)
+{
+    if (s.cap < need) {
+        if (s.p && (s.captured || capturing)) ctx->retired.push_back(s.p);
+        else if (s.p) cudaFree(s.p);
+        s = RunScratch();
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaMalloc(&s.p, need);
+        if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            s.p = nullptr;
+            return cuda_fail(ctx, e, "cudaMalloc");
+        }
+        s.cap = need;
+    }
+    s.captured = s.captured || capturing;
+    return FPL_OK;
+}
+
 // wrapped datum adjustment (python/adjustMiniStacks.py:174-197: the "mul"
 // pixel function of a derived VRT band): out[d][p] = phase[d][p] * datum[p]
 __global__ void k_adjust_wrapped(const float2 *phase, const float2 *__restrict__ datum, float2 *out,
@@ -173,10 +197,11 @@ int fpl_ctx_destroy(fpl_ctx *ctx)
         if (ctx->s_in) cudaStreamDestroy(ctx->s_in);
         if (ctx->s_out) cudaStreamDestroy(ctx->s_out);
         void *bufs[] = {ctx->d_stack, ctx->d_nmap, ctx->d_phase, ctx->d_tcorr, ctx->d_comp,
-                        ctx->d_status, ctx->d_fb_list, ctx->d_small, ctx->d_cbuf, ctx->d_cinfo,
+                        ctx->d_status, ctx->fb_list.p, ctx->d_small, ctx->cbuf.p, ctx->cinfo.p,
                         ctx->d_nm, ctx->d_pack};
         for (void *b : bufs)
             if (b) cudaFree(b);
+        for (void *b : ctx->retired) cudaFree(b);
         if (ctx->ev_last) cudaEventDestroy(ctx->ev_last);
         if (ctx->ev0) cudaEventDestroy(ctx->ev0);
         if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -199,10 +224,11 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out)
 
 static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                             void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
-                            bool fp64_all, void *counters, bool count_run, int stages, long long list_cap);
+                            bool fp64_all, void *counters, bool count_run, int stages, long long list_cap,
+                            bool capturing);
 
 // Enqueues both passes on `st` for device buffers.  Scratch: the context's
-// work-list buffer (grown with cudaMalloc when too small) and d_small.
+// work list and records (grown with cudaMalloc when too small) and d_small.
 int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                 void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
                 bool fp64_all, void *counters, bool count_run, int stages, long long list_cap)
@@ -216,7 +242,7 @@ int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint3
     const bool order = (cap == cudaStreamCaptureStatusNone);
     if (order && ctx->last_used) FPL_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_last, 0));
     int rc_ = fpl_enqueue_body(ctx, job, stack, nmap, phase, tcorr, comp, status, st, fp64_all, counters,
-                               count_run, stages, list_cap);
+                               count_run, stages, list_cap, !order);
     if (rc_) return rc_;
     if (order) {
         FPL_CUDA(ctx, cudaEventRecord(ctx->ev_last, st));
@@ -227,7 +253,8 @@ int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint3
 
 static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                             void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
-                            bool fp64_all, void *counters, bool count_run, int stages, long long list_cap)
+                            bool fp64_all, void *counters, bool count_run, int stages, long long list_cap,
+                            bool capturing)
 {
     const int r0 = job->row_begin, r1 = job->row_end <= 0 ? job->rows : job->row_end;
     int rc = 0;
@@ -267,9 +294,9 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
     // work list: at most one entry per pixel of the range (or of the run)
     const long long cap = list_cap > 0 ? list_cap : P.npix;
     size_t need = sizeof(long long) * (size_t)(cap > 0 ? cap : 1);
-    rc = grow(ctx, &ctx->d_fb_list, &ctx->cap_fb_list, need);
+    rc = grow_run(ctx, ctx->fb_list, need, capturing);
     if (rc) return rc;
-    P.fb_list = static_cast<long long *>(ctx->d_fb_list);
+    P.fb_list = static_cast<long long *>(ctx->fb_list.p);
     P.fb_cap = (int)(cap < 0x7fffffff ? cap : 0x7fffffff);
     if (stages & ENQ_RESET) FPL_CUDA(ctx, cudaMemsetAsync(counters, 0, kCounterBlock, st));
     if (P.npix == 0) return FPL_OK;
@@ -312,9 +339,9 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
         rows_per_chunk = std::min(rows_per_chunk, r1 - r0);
         for (;;) {
             chunk_px = (long long)rows_per_chunk * P.cols;
-            rc = grow(ctx, &ctx->d_cbuf, &ctx->cap_cbuf, sizeof(float) * (size_t)rec * chunk_px);
+            rc = grow_run(ctx, ctx->cbuf, sizeof(float) * (size_t)rec * chunk_px, capturing);
             // tile information and rest list
-            if (!rc) rc = grow(ctx, &ctx->d_cinfo, &ctx->cap_cinfo, 2 * sizeof(int) * (size_t)chunk_px);
+            if (!rc) rc = grow_run(ctx, ctx->cinfo, 2 * sizeof(int) * (size_t)chunk_px, capturing);
             if (!rc) break;
             if (rc != FPL_ERR_NOMEM || job->precision == FPL_PREC_MIXED) return rc;
             cudaGetLastError();
@@ -331,8 +358,8 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
             Q.pix_begin = (long long)ra * P.cols;
             Q.npix = (long long)(rb - ra) * P.cols;
             Q.parts = job->precision == FPL_PREC_MIXED ? 2 : 3;
-            Q.cbuf = static_cast<float2 *>(ctx->d_cbuf);
-            Q.cinfo = static_cast<int *>(ctx->d_cinfo);
+            Q.cbuf = static_cast<float2 *>(ctx->cbuf.p);
+            Q.cinfo = static_cast<int *>(ctx->cinfo.p);
             Q.rest = Q.cinfo + chunk_px;
             Q.cbase = Q.pix_begin;
             Q.cstride = rec;
@@ -538,7 +565,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
                 const size_t slots = (size_t)nset * (nb + 3);
                 if ((rc = grow(ctx, &ctx->d_pack, &ctx->cap_pack, slots * sizeof(float2)))) return rc;
                 const unsigned blocks = (unsigned)std::min<size_t>((slots + 255) / 256, (size_t)ctx->num_sms * 8);
-                k_pack_settled<<<blocks, 256, 0, st>>>(static_cast<const long long *>(ctx->d_fb_list),
+                k_pack_settled<<<blocks, 256, 0, st>>>(static_cast<const long long *>(ctx->fb_list.p),
                                                        static_cast<const int *>(ctx->d_small), (int)nset,
                                                        reinterpret_cast<const float2 *>(d_phase), d_tcorr,
                                                        reinterpret_cast<const float2 *>(d_comp), d_status, (long long)plane,

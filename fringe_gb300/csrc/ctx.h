@@ -28,6 +28,14 @@ struct NmapAdPlan {
     float lo = 0.f, hi = 0.f, w[2 * FPL_MAX_BANDS] = {};
 };
 
+// device scratch that a run's kernels refer to; captured: a stream capture
+// has recorded its address
+struct RunScratch {
+    void *p = nullptr;
+    size_t cap = 0;
+    bool captured = false;
+};
+
 struct fpl_ctx {
     int device = 0;
     int num_sms = 0;
@@ -43,12 +51,12 @@ struct fpl_ctx {
     size_t cap_stack = 0, cap_nmap = 0, cap_phase = 0, cap_tcorr = 0, cap_comp = 0,
            cap_status = 0;
     // scratch: FP64 work list, and d_small = {count, .., err flags}
-    void *d_fb_list = nullptr;
-    size_t cap_fb_list = 0;
+    RunScratch fb_list;
     void *d_small = nullptr;
-    // mixed form: packed coherence matrices of one chunk of rows
-    void *d_cbuf = nullptr, *d_cinfo = nullptr;
-    size_t cap_cbuf = 0, cap_cinfo = 0;
+    // Gamma records of one chunk of rows; their tile information and rest list
+    RunScratch cbuf, cinfo;
+    // outgrown scratch that a captured graph may still refer to
+    std::vector<void *> retired;
     // nmap: sorted amplitudes, validity and staging of host jobs
     void *d_nm = nullptr;
     size_t cap_nm = 0;

@@ -148,7 +148,9 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job);
  * legacy default stream); device buffers only.  Runs sharing one context
  * share its scratch: each run waits on the GPU for the context's previous
  * run, on whatever stream that was enqueued (inside a stream capture the
- * caller's graph orders them instead).  Same replacement as fpl_run. */
+ * caller's graph orders them instead).  Scratch that a captured run refers to
+ * stays allocated until the context is destroyed, so its graph can be replayed
+ * whatever larger runs the context has made since.  Same replacement as fpl_run. */
 int fpl_run_async(fpl_ctx *ctx, const fpl_job *job, void *stream);
 
 int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out);

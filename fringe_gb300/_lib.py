@@ -121,6 +121,7 @@ _SIGS = {
     "fpl_server_destroy": (ctypes.c_int, [_P]),
     "fpl_ctx_set_tuning": (ctypes.c_int, [_P, ctypes.c_float, ctypes.c_int]),
     "fpl_ctx_set_shift": (ctypes.c_int, [_P, ctypes.c_float, ctypes.c_float]),
+    "fpl_ctx_set_record_limit": (ctypes.c_int, [_P, ctypes.c_longlong]),
     "fpl_adjust_wrapped": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int, ctypes.c_longlong, _P]),
     "fpl_ctx_last_error": (ctypes.c_char_p, [_P]),
     "fpl_ctx_set_profiling": (ctypes.c_int, [_P, ctypes.c_int]),
@@ -230,6 +231,10 @@ class Context:
     def set_shift(self, shift=0.999, backoff=0.97):
         """Shifts of the FP32 MLE inverse iteration (fpl_ctx_set_shift)."""
         check(load().fpl_ctx_set_shift(self.handle, float(shift), float(backoff)), self.handle)
+
+    def set_record_limit(self, nbytes=-1):
+        """Device bytes that FP32 runs keep for records (fpl_ctx_set_record_limit)."""
+        check(load().fpl_ctx_set_record_limit(self.handle, int(nbytes)), self.handle)
 
 
 _contexts = {}

@@ -227,6 +227,25 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
                             bool fp64_all, void *counters, bool count_run, int stages, long long list_cap,
                             bool capturing);
 
+// Rows of records that a run over `span` rows of the job takes at a time: 2^20
+// pixels at most, and in the FP32 form no more bytes than the context's limit.
+// Whole tile rows (8 rows) where there is more than one chunk; 0: records are not used.
+static int record_rows(const fpl_ctx *ctx, const fpl_job *job, int rec, int span)
+{
+    long long rows = std::max<long long>(1, (1ll << 20) / job->cols);
+    if (job->precision == FPL_PREC_FP32) {
+        const long long row_bytes = (long long)job->cols * (4ll * rec + 2 * (long long)sizeof(int));
+        const long long limit = ctx->record_limit >= 0 ? ctx->record_limit : std::max(kDefaultRecordLimit, 8 * row_bytes);
+        rows = std::min(std::max(rows, 8ll), limit / row_bytes);
+        if (rows < std::min(8, span)) return 0;
+    }
+    if (rows >= span) return span;
+    if (rows < 8) return (int)rows;
+    // chunks of about the same height: a short last one would leave SMs idle
+    const long long chunks = (span + rows / 8 * 8 - 1) / (rows / 8 * 8);
+    return (int)(((span + chunks - 1) / chunks + 7) / 8 * 8);
+}
+
 // Enqueues both passes on `st` for device buffers.  Scratch: the context's
 // work list and records (grown with cudaMalloc when too small) and d_small.
 int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
@@ -326,34 +345,37 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
         return cudaSuccess;
     };
     if (ctx->profile && count_run) ctx->prof_runs++;
-    bool tiled = fpl::gram_box_supported(P.nb, P.ny, P.nx);
+    const int rec = fpl::gram_box_record(P.nb);
     int rows_per_chunk = 0;
     long long chunk_px = 0;
-    const int rec = fpl::gram_box_record(P.nb);
+    bool tiled = fpl::gram_box_supported(P.nb, P.ny, P.nx);
     if ((stages & ENQ_KERNELS) && tiled) {
         // tensor-core Gamma records, then eigen-solves, chunk by chunk of rows
         // so the records stay within a bounded buffer.  A record's value does not
         // depend on the chunk, so the FP32 form, which needs no such buffer by itself,
-        // takes smaller chunks where the device memory is short.
-        rows_per_chunk = (int)std::max<long long>(1, std::max<long long>(P.cols, (1ll << 20)) / P.cols);
-        rows_per_chunk = std::min(rows_per_chunk, r1 - r0);
+        // takes smaller chunks where the device memory is short, and the plain
+        // kernel where not even a row of tiles fits.
+        const bool fp32 = job->precision == FPL_PREC_FP32;
+        rows_per_chunk = record_rows(ctx, job, rec, r1 - r0);
         for (;;) {
+            if (rows_per_chunk == 0) { tiled = false; break; }
             chunk_px = (long long)rows_per_chunk * P.cols;
             rc = grow_run(ctx, ctx->cbuf, sizeof(float) * (size_t)rec * chunk_px, capturing);
             // tile information and rest list
             if (!rc) rc = grow_run(ctx, ctx->cinfo, 2 * sizeof(int) * (size_t)chunk_px, capturing);
             if (!rc) break;
-            if (rc != FPL_ERR_NOMEM || job->precision == FPL_PREC_MIXED) return rc;
+            if (rc != FPL_ERR_NOMEM || !fp32) return rc;
             cudaGetLastError();
-            if (rows_per_chunk == 1) { tiled = false; break; }
-            rows_per_chunk = (rows_per_chunk + 1) / 2;
+            rows_per_chunk = rows_per_chunk >= 16 ? rows_per_chunk / 2 / 8 * 8 : 0;
         }
     }
     if (!(stages & ENQ_KERNELS)) {
         // settle only
     } else if (tiled) {
-        for (int ra = r0; ra < r1; ra += rows_per_chunk) {
-            const int rb = std::min(r1, ra + rows_per_chunk);
+        for (int ra = r0, rb; ra < r1; ra = rb) {
+            // several chunks end on the tile grid, so that no tile is computed twice
+            const bool grid = rows_per_chunk >= 8 && rows_per_chunk < r1 - r0;
+            rb = std::min(r1, (grid ? ra / 8 * 8 : ra) + rows_per_chunk);
             KParams Q = P;
             Q.pix_begin = (long long)ra * P.cols;
             Q.npix = (long long)(rb - ra) * P.cols;
@@ -664,6 +686,23 @@ int fpl_ctx_set_shift(fpl_ctx *ctx, float shift, float backoff)
         if (!(shift > 0.f) || !(backoff > 0.f)) return FPL_ERR_OPTIONS;
         ctx->shift = shift;
         ctx->shift_backoff = backoff;
+        return FPL_OK;
+    });
+}
+
+int fpl_ctx_set_record_limit(fpl_ctx *ctx, long long bytes)
+{
+    return fpl_guard([&]() -> int {
+        if (!ctx) return FPL_ERR_NULL;
+        FPL_CUDA(ctx, cudaSetDevice(ctx->device));
+        ctx->record_limit = bytes < 0 ? -1 : bytes;
+        const size_t limit = (size_t)(bytes < 0 ? kDefaultRecordLimit : bytes);
+        if (ctx->cbuf.cap + ctx->cinfo.cap > limit && !ctx->cbuf.captured && !ctx->cinfo.captured) {
+            if (ctx->last_used) FPL_CUDA(ctx, cudaEventSynchronize(ctx->ev_last));
+            if (ctx->cbuf.p) cudaFree(ctx->cbuf.p);
+            if (ctx->cinfo.p) cudaFree(ctx->cinfo.p);
+            ctx->cbuf = ctx->cinfo = RunScratch();
+        }
         return FPL_OK;
     });
 }

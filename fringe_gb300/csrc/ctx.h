@@ -19,6 +19,11 @@ constexpr float kDefaultAmbScale = 8.0f;    // FP32 rounding band, in units of n
 constexpr float kDefaultCondMax = 1000.0f;  // |C| inverted in FP32 up to this inf-norm condition
 constexpr float kDefaultShift = 0.999f;     // inverse-iteration shift, in units of min(1, rho)
 constexpr float kDefaultShiftBackoff = 0.97f;   // second shift when M - sigma I is not definite
+// Device bytes that FP32 runs keep for Gamma records (at least 8 rows of them).
+// 4 GiB hold a chunk of 2^20 pixels, beyond which nothing is gained, up to 30 dates.
+// 1024^2 without a limit and with 4, 2, 1 and 0.5 GiB: 30 dates 18.0, 18.0, 18.4, 18.9 and
+// 19.7 ms; 64 dates 132, 134, 136, 140 and 159 ms (the tails of every chunk's kernels).
+constexpr long long kDefaultRecordLimit = 4ll << 30;
 
 // decision boundary of the Anderson-Darling test (nmap.cu) for one stack
 // depth and threshold
@@ -55,6 +60,7 @@ struct fpl_ctx {
     void *d_small = nullptr;
     // Gamma records of one chunk of rows; their tile information and rest list
     RunScratch cbuf, cinfo;
+    long long record_limit = -1;     // bytes of them in the FP32 form; -1: the default
     // outgrown scratch that a captured graph may still refer to
     std::vector<void *> retired;
     // nmap: sorted amplitudes, validity and staging of host jobs

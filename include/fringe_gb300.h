@@ -243,6 +243,14 @@ int fpl_ctx_set_tuning(fpl_ctx *ctx, float amb_scale, int force_fp64);
  * the second attempt and the Householder path.  Runs and batches on this
  * context use them (servers and fpl_run_noalloc keep the defaults). */
 int fpl_ctx_set_shift(fpl_ctx *ctx, float shift, float backoff);
+/* Device memory for the coherence records of FP32 runs.  A context keeps the
+ * records of one chunk of rows between runs; by default FP32 runs let them
+ * take 4 GiB, or 8 rows if that is more.  bytes >= 0: no more than that; a run
+ * for which it does not hold 8 rows (or all its rows) uses the plain kernel, which
+ * needs none (0: every FP32 run).  < 0: the default.  Records held beyond the new
+ * limit are released, unless a captured run refers to them.  Mixed runs need
+ * records and take those of up to 2^20 pixels whatever the limit. */
+int fpl_ctx_set_record_limit(fpl_ctx *ctx, long long bytes);
 /* Per-kernel device timing of subsequent runs (CUDA events on the run's
  * stream); fpl_ctx_profile waits for them, returns the summed FP32 and FP64
  * kernel milliseconds and the run count, and resets the record. */

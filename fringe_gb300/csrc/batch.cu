@@ -375,51 +375,111 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
         fpl_batch *b = new fpl_batch();
         b->ctx = ctx;
         b->njobs = njobs;
-        auto is_tiled = [&](const fpl_job &jb) {
-            return fpl::gram_box_supported(jb.nbands, jb.half_window_y, jb.half_window_x);
-        };
-        // jobs whose windows the Gamma kernel does not take (plain FP32 kernel), grouped by padded depth
+        // Jobs whose windows the Gamma kernel takes are cut into row pieces, packed into
+        // waves of at most wave_px pixels; FP32 jobs, which need no records, take them
+        // within the context's limit.  Other jobs run the plain FP32 kernel, grouped by padded
+        // depth.  Where the device memory is short of the records the waves are made
+        // smaller, and at last FP32 jobs do without.
+        struct Piece { int job, ra, rb; long long px; int wave; size_t rec, info; };
         std::vector<int> order;
-        for (int j = 0; j < njobs; ++j)
-            if (!is_tiled(jobs[j])) order.push_back(j);
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int a, int c) { return fpl::pick_np(jobs[a].nbands) < fpl::pick_np(jobs[c].nbands); });
-        const int nf = (int)order.size();
-        // the others: row pieces of at most kWavePx pixels, packed into waves
-        struct Piece { int job, ra, rb; long long px; };
-        // smaller waves where the device memory is short of their records
-        long long kWavePx = 1ll << 20;
-        {
-            size_t free_b = 0, total_b = 0, rec_px = 0;
-            for (int j = 0; j < njobs; ++j)
-                if (is_tiled(jobs[j])) rec_px = std::max(rec_px, 4 * (size_t)fpl::gram_box_record(jobs[j].nbands));
-            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
-                while (kWavePx > 65536 && (size_t)kWavePx * rec_px > free_b / 2) kWavePx /= 2;
-        }
         std::vector<Piece> pieces;
-        for (int j = 0; j < njobs; ++j) {
-            if (!is_tiled(jobs[j])) continue;
-            const fpl_job &jb = jobs[j];
-            const int r0 = jb.row_begin, r1 = jb.row_end <= 0 ? jb.rows : jb.row_end;
-            const int step = (int)std::max<long long>(1, kWavePx / jb.cols);
-            for (int ra = r0; ra < r1; ra += step) {
-                const int rb = std::min(r1, ra + step);
-                pieces.push_back({j, ra, rb, (long long)(rb - ra) * jb.cols});
+        size_t rec_max = 0, info_max = 0;           // of a wave: record floats, pixels
+        int nwaves = 0;
+        bool fp32_tiled = false;
+        auto plan = [&](long long wave_px, size_t fp32_bytes, bool fp32_records) {
+            order.clear();
+            pieces.clear();
+            rec_max = info_max = 0;
+            nwaves = 0;
+            fp32_tiled = false;
+            long long wpx = 0;
+            size_t rec = 0, info = 0, wbytes = 0;   // of the present wave; wbytes: of FP32 records
+            for (int j = 0; j < njobs; ++j) {
+                const fpl_job &jb = jobs[j];
+                const int r0 = jb.row_begin, r1 = jb.row_end <= 0 ? jb.rows : jb.row_end;
+                const bool fp32 = jb.precision == FPL_PREC_FP32;
+                const size_t cstride = fpl::gram_box_record(jb.nbands), px_bytes = 4 * cstride + 2 * sizeof(int),
+                             row_bytes = px_bytes * jb.cols;
+                long long step = std::max<long long>(1, wave_px / jb.cols);
+                bool tiled = fpl::gram_box_supported(jb.nbands, jb.half_window_y, jb.half_window_x);
+                if (tiled && fp32) {
+                    // (8 rows by default even if they take more than the limit)
+                    const long long fit = fp32_bytes / row_bytes, least = std::min(8, std::max(1, r1 - r0));
+                    step = std::min(std::max(step, least), ctx->record_limit < 0 ? std::max(fit, least) : fit);
+                    tiled = fp32_records && step >= least;
+                    fp32_tiled = fp32_tiled || tiled;
+                }
+                if (!tiled) {
+                    order.push_back(j);
+                    continue;
+                }
+                for (int ra = r0; ra < r1;) {
+                    const int rb = (int)std::min<long long>(r1, step >= 8 ? (ra + step) / 8 * 8 : ra + step);
+                    const long long px = (long long)(rb - ra) * jb.cols;
+                    const size_t bytes = fp32 ? px_bytes * px : 0;
+                    if (nwaves == 0 || wpx + px > wave_px || (bytes && wbytes && wbytes + bytes > fp32_bytes)) {
+                        ++nwaves;
+                        wpx = 0;
+                        rec = info = wbytes = 0;
+                    }
+                    pieces.push_back({j, ra, rb, px, nwaves - 1, rec, info});
+                    wpx += px;
+                    rec += cstride * px;
+                    info += px;
+                    wbytes += bytes;
+                    rec_max = std::max(rec_max, rec);
+                    info_max = std::max(info_max, info);
+                    ra = rb;
+                }
             }
-        }
-        const int np_ = (int)pieces.size();
-        b->nent = nf + np_;
+            std::stable_sort(order.begin(), order.end(),
+                             [&](int a, int c) { return fpl::pick_np(jobs[a].nbands) < fpl::pick_np(jobs[c].nbands); });
+        };
         long long fb_total = 0;
+        size_t rec_px = 0;
         for (int j = 0; j < njobs; ++j) {
             const fpl_job &jb = jobs[j];
             const int r1 = jb.row_end <= 0 ? jb.rows : jb.row_end;
             fb_total += (long long)(r1 - jb.row_begin) * jb.cols;
+            if (fpl::gram_box_supported(jb.nbands, jb.half_window_y, jb.half_window_x))
+                rec_px = std::max(rec_px, 4 * (size_t)fpl::gram_box_record(jb.nbands));
         }
         b->pixels = fb_total;
-        // scratch: per-entry counters | work counters (one per class, <= 3) | FP64 lists
-        b->counter_bytes = kJobCounterBytes * b->nent + 64;
-        const size_t scratch = b->counter_bytes + sizeof(long long) * (size_t)std::max<long long>(fb_total, 1);
-        if (cudaMalloc(&b->d_scratch, scratch) != cudaSuccess) { fpl_batch_destroy(b); return FPL_ERR_NOMEM; }
+        long long wave_px = 1ll << 20;
+        size_t fp32_bytes = (size_t)(ctx->record_limit >= 0 ? ctx->record_limit : kDefaultRecordLimit);
+        bool fp32_records = true;
+        {
+            size_t free_b = 0, total_b = 0;
+            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
+                while (wave_px > 65536 && (size_t)wave_px * rec_px > free_b / 2) wave_px /= 2;
+        }
+        size_t rec_bytes = 0;
+        for (;;) {
+            plan(wave_px, fp32_bytes, fp32_records);
+            b->nent = (int)(order.size() + pieces.size());
+            // scratch: per-entry counters | work counters (one per class, <= 3) | FP64 lists
+            b->counter_bytes = kJobCounterBytes * b->nent + 64;
+            const size_t scratch = b->counter_bytes + sizeof(long long) * (size_t)std::max<long long>(fb_total, 1);
+            if (cudaMalloc(&b->d_scratch, scratch) != cudaSuccess) {
+                b->d_scratch = nullptr;
+                fpl_batch_destroy(b);
+                return FPL_ERR_NOMEM;
+            }
+            if (pieces.empty()) break;
+            rec_bytes = (sizeof(float) * rec_max + 255) & ~size_t(255);
+            if (cudaMalloc(&b->d_rec, rec_bytes + 2 * sizeof(int) * std::max<size_t>(info_max, 1)) == cudaSuccess) break;
+            cudaGetLastError();
+            b->d_rec = nullptr;
+            if (wave_px <= 65536 && !fp32_tiled) {
+                fpl_batch_destroy(b);
+                return FPL_ERR_NOMEM;
+            }
+            cudaFree(b->d_scratch);
+            b->d_scratch = nullptr;
+            if (wave_px > 65536) wave_px /= 2;
+            else fp32_records = false;
+        }
+        const int nf = (int)order.size(), np_ = (int)pieces.size();
         std::vector<fpl::BatchEntry> table(nf);
         long long fb_off = 0;
         char *cnt_base = static_cast<char *>(b->d_scratch);
@@ -443,37 +503,10 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
             set_counters(P, e);
             b->job_of_entry.push_back(j);
         }
-        // mixed pieces: parameters, waves, records buffer
+        // the pieces' parameters, wave by wave
         if (np_ > 0) {
             std::vector<fpl::KParams> pp(np_);
-            std::vector<int> wave_of(np_);
-            std::vector<long long> rec_off(np_), info_off(np_);
-            size_t rec_max = 0, info_max = 0;
-            {
-                long long wpx = 0;
-                size_t rec = 0, inf = 0;
-                int w = -1;
-                for (int i = 0; i < np_; ++i) {
-                    const Piece &pc = pieces[i];
-                    const fpl_job &jb = jobs[pc.job];
-                    if (w < 0 || wpx + pc.px > kWavePx) { ++w; wpx = 0; rec = 0; inf = 0; }
-                    wave_of[i] = w;
-                    wpx += pc.px;
-                    const int cstride = fpl::gram_box_record(jb.nbands);
-                    rec_off[i] = (long long)rec;
-                    info_off[i] = (long long)inf;
-                    rec += (size_t)pc.px * cstride;
-                    inf += (size_t)pc.px;
-                    rec_max = std::max(rec_max, rec);
-                    info_max = std::max(info_max, inf);
-                }
-                b->waves.resize(w + 1);
-            }
-            const size_t rec_bytes = (sizeof(float) * rec_max + 255) & ~size_t(255);
-            if (cudaMalloc(&b->d_rec, rec_bytes + 2 * sizeof(int) * std::max<size_t>(info_max, 1)) != cudaSuccess) {
-                fpl_batch_destroy(b);
-                return FPL_ERR_NOMEM;
-            }
+            b->waves.resize(nwaves);
             float *recs = static_cast<float *>(b->d_rec);
             int *infos = reinterpret_cast<int *>(static_cast<char *>(b->d_rec) + rec_bytes);
             for (int i = 0; i < np_; ++i) {
@@ -484,8 +517,8 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 P.shift = ctx->shift;
                 P.shift_backoff = ctx->shift_backoff;
                 set_counters(P, nf + i);
-                P.cbuf = reinterpret_cast<float2 *>(recs + rec_off[i]);
-                P.cinfo = infos + info_off[i];
+                P.cbuf = reinterpret_cast<float2 *>(recs + pc.rec);
+                P.cinfo = infos + pc.info;
                 P.rest = P.cinfo + info_max;
                 P.cbase = P.pix_begin;
                 P.cstride = fpl::gram_box_record(jb.nbands);
@@ -498,7 +531,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 MixedWave &mw = b->waves[w];
                 mw.seg_first = (int)segs.size();
                 for (int i = 0; i < np_; ++i) {
-                    if (wave_of[i] != (int)w) continue;
+                    if (pieces[i].wave != (int)w) continue;
                     fpl::BoxSeg sg;
                     sg.P = pp[i];
                     sg.tile_offset = mw.seg_tiles;
@@ -511,7 +544,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                     const int npd = 16 << c;
                     mw.ent_first[c] = (int)ments.size();
                     for (int i = 0; i < np_; ++i) {
-                        if (wave_of[i] != (int)w || fpl::pick_np(pp[i].nb) != npd) continue;
+                        if (pieces[i].wave != (int)w || fpl::pick_np(pp[i].nb) != npd) continue;
                         if (pp[i].npix >= fpl::kOwnSolvePx) {
                             mw.own.push_back(pp[i]);
                             continue;

@@ -168,7 +168,10 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out);
  * waves of <= 2^20 pixels (fewer where device memory is short), with one
  * tensor-core Gamma launch over the tiles and one solve launch per padded depth
  * and kind of method over the pixels of each wave.  Jobs whose window the Gamma
- * kernel does not take run one persistent plain FP32 launch per padded depth. */
+ * kernel does not take run one persistent plain FP32 launch per padded depth, and so
+ * do FP32 jobs for whose records there is no room on the device or within the
+ * context's limit (fpl_ctx_set_record_limit).  A batch holds its records until it
+ * is destroyed. */
 #define FPL_BATCH_GRAPH 1
 #define FPL_BATCH_AUTOTUNE 2
 typedef struct fpl_batch fpl_batch;
@@ -249,7 +252,8 @@ int fpl_ctx_set_shift(fpl_ctx *ctx, float shift, float backoff);
  * for which it does not hold 8 rows (or all its rows) uses the plain kernel, which
  * needs none (0: every FP32 run).  < 0: the default.  Records held beyond the new
  * limit are released, unless a captured run refers to them.  Mixed runs need
- * records and take those of up to 2^20 pixels whatever the limit. */
+ * records and take those of up to 2^20 pixels whatever the limit.  A wave of a batch
+ * made on the context keeps to it in the same way. */
 int fpl_ctx_set_record_limit(fpl_ctx *ctx, long long bytes);
 /* Per-kernel device timing of subsequent runs (CUDA events on the run's
  * stream); fpl_ctx_profile waits for them, returns the summed FP32 and FP64

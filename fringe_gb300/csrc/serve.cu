@@ -195,45 +195,62 @@ bool run_wave(fpl_server *s, std::vector<Piece> &pieces)
     long long total = 0;
     for (SJob *j : ready) {
         if ((int)pieces.size() >= s->max_pieces) break;
+        const bool supported = fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x);
         int rows = (int)std::max<long long>(1, share / j->host.cols);
+        if (supported && j->host.precision == FPL_PREC_FP32) {
+            // an equal share of the records' bytes too (8 rows even if they take more)
+            const long long row_bytes = (long long)j->host.cols * (4ll * fpl::gram_box_record(j->host.nbands) + 8);
+            rows = (int)std::min<long long>(rows, std::max<long long>(8, kDefaultRecordLimit / (long long)ready.size() / row_bytes));
+        }
         const int ra = j->next_row, rb = std::min(j->r1, ra + rows);
         j->next_row = rb;
         if (!j->started) { j->started = true; j->t_first = clk::now(); }
         // 0: plain kernel, 1: combined solve launch, 2: one of its own
-        const int tiled = !fpl::gram_box_supported(j->host.nbands, j->host.half_window_y, j->host.half_window_x) ? 0
-                          : (long long)(rb - ra) * j->host.cols >= fpl::kOwnSolvePx                               ? 2
-                                                                                                                   : 1;
+        const int tiled = !supported ? 0 : (long long)(rb - ra) * j->host.cols >= fpl::kOwnSolvePx ? 2 : 1;
         pieces.push_back({j, ra, rb, fpl::pick_np(j->host.nbands), tiled});
         total += (long long)(rb - ra) * j->host.cols;
     }
-    std::stable_sort(pieces.begin(), pieces.end(), [](const Piece &a, const Piece &b) {
-        return a.np != b.np ? a.np < b.np : a.tiled < b.tiled;
-    });
-    // Gamma records of the wave's tiled pieces
-    size_t rec_floats = 0, infos = 0;
-    for (const Piece &pc : pieces)
-        if (pc.tiled) {
-            const size_t px = (size_t)(pc.rb - pc.ra) * pc.job->host.cols;
-            rec_floats += px * fpl::gram_box_record(pc.job->host.nbands);
-            infos += px;
-        }
-    const size_t rec_bytes = (sizeof(float) * rec_floats + 255) & ~size_t(255);
-    const size_t rec_need = rec_bytes + 2 * sizeof(int) * infos;
-    if (rec_floats && rec_need > s->rec_cap) {
+    // Gamma records of the wave's tiled pieces.  Where the device has no room for them:
+    // smaller waves from here on, then the plain kernel for the FP32 pieces, which need none
+    size_t infos = 0, rec_bytes = 0;
+    for (;;) {
+        std::stable_sort(pieces.begin(), pieces.end(), [](const Piece &a, const Piece &b) {
+            return a.np != b.np ? a.np < b.np : a.tiled < b.tiled;
+        });
+        size_t rec_floats = 0;
+        infos = 0;
+        for (const Piece &pc : pieces)
+            if (pc.tiled) {
+                const size_t px = (size_t)(pc.rb - pc.ra) * pc.job->host.cols;
+                rec_floats += px * fpl::gram_box_record(pc.job->host.nbands);
+                infos += px;
+            }
+        rec_bytes = (sizeof(float) * rec_floats + 255) & ~size_t(255);
+        const size_t rec_need = rec_bytes + 2 * sizeof(int) * infos;
+        if (!rec_floats || rec_need <= s->rec_cap) break;
         // the previous wave has finished (its event was waited for)
         if (s->d_rec) cudaFree(s->d_rec);
         s->d_rec = nullptr;
         s->rec_cap = 0;
-        if (cudaMalloc(&s->d_rec, rec_need) != cudaSuccess) {
-            if (s->cfg.wave_pixels <= 65536) return false;
-            // short of device memory: smaller waves from here on
-            cudaGetLastError();
+        if (cudaMalloc(&s->d_rec, rec_need) == cudaSuccess) {
+            s->rec_cap = rec_need;
+            break;
+        }
+        s->d_rec = nullptr;
+        cudaGetLastError();
+        if (s->cfg.wave_pixels > 65536) {
             s->cfg.wave_pixels /= 2;
             for (Piece &pc : pieces) pc.job->next_row = pc.ra;
             pieces.clear();
             return true;
         }
-        s->rec_cap = rec_need;
+        bool fewer = false;
+        for (Piece &pc : pieces)
+            if (pc.tiled && pc.job->host.precision == FPL_PREC_FP32) {
+                pc.tiled = 0;
+                fewer = true;
+            }
+        if (!fewer) return false;
     }
     float *recs = static_cast<float *>(s->d_rec);
     int *rinfo = reinterpret_cast<int *>(static_cast<char *>(s->d_rec) + rec_bytes);

@@ -190,7 +190,11 @@ int fpl_batch_destroy(fpl_batch *batch);
  * and runs waves of at most wave_pixels pixels in which every resident job
  * gets a slice of rows -- jobs arriving during a wave join the next one
  * (continuous batching).  Results are copied back as each job finishes.  A
- * job's result does not depend on the other jobs in flight. */
+ * job's result does not depend on the other jobs in flight.  The coherence records
+ * of a wave come on top of memory_budget: for FP32 jobs 4 GiB, or 8 rows of every
+ * job if that is more; for mixed jobs those of the wave's pixels.  Where the
+ * device has no room for them the waves are made smaller, and at last FP32 jobs run
+ * the plain kernel, whose results differ in the last bits. */
 typedef struct fpl_server fpl_server;
 typedef struct {
     size_t memory_budget;      /* device bytes for resident jobs (default 80 GB) */

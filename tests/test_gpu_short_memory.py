@@ -1,5 +1,5 @@
-"""FP32 jobs need no Gamma records: where the device has no room for them, runs
-and batches fall back to the plain FP32 kernel, and only jobs of the mixed form
+"""FP32 jobs need no Gamma records: where the device has no room for them, runs,
+batches and servers fall back to the plain FP32 kernel, and only jobs of the mixed form
 are refused.  A preloaded cudaMalloc that refuses large requests stands in for
 the full device."""
 import os
@@ -31,6 +31,7 @@ import ctypes, os, sys
 import numpy as np
 from fringe_gb300 import _lib, synth
 from fringe_gb300.linker import _make_job, phase_link
+from fringe_gb300.serve import Server
 from tests.parity import assert_parity, compare
 
 MAX = str(16 << 20)                  # the records below take 22 to 80 MB, every other buffer less than 16
@@ -81,12 +82,22 @@ def batch(precision):
         lib.fpl_batch_destroy(h)
 
 
+def serve(wave_pixels):
+    srv = Server(wave_pixels=wave_pixels)
+    os.environ["TEST_MALLOC_MAX"] = MAX
+    tickets = [srv.submit(stack, nmap, W) for _ in range(3)]
+    for t in tickets:
+        srv.wait(t)
+        check(srv.result(t))
+    srv.close()
+
+
 eval(sys.argv[1])
 print("short memory ok")
 """
 
 
-@pytest.mark.parametrize("call", ["run()", "batch('fp32')", "batch('mixed')"])
+@pytest.mark.parametrize("call", ["run()", "batch('fp32')", "batch('mixed')", "serve(1 << 20)", "serve(8192)"])
 def test_without_room_for_records(gpu_lib, tmp_path, call):
     src, so = tmp_path / "shim.c", tmp_path / "shim.so"
     src.write_text(SHIM)

@@ -39,9 +39,10 @@
 //
 // Samples whose value is non-finite, or whose components lie outside
 // [2^-50, 2^50] in magnitude (other than 0), are outside the range of the
-// split: they are zeroed in the tile and every pixel that has one among its
-// SHPs is handed to the FP64 path (CI_DEFER), which follows the reference
-// exactly.  Every wait on the tensor core is bounded; on timeout the CTA
+// split and zeroed in the tile.  A pixel with a non-finite one among its SHPs has
+// a non-finite power at that date, so its outcome is known: the failure code
+// of the first eigen call (CI_BAD).  A pixel with a finite one is handed to the FP64 path
+// (CI_DEFER), which follows the reference exactly.  Every wait on the tensor core is bounded; on timeout the CTA
 // records an error flag, stops, and frees its tensor memory after a second
 // bounded wait.
 #include <cuda_bf16.h>
@@ -288,9 +289,10 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     BoxBars *bars = reinterpret_cast<BoxBars *>(misc);
     volatile int *dead = &bars->dead;
     int *pinfo = reinterpret_cast<int *>(misc + 64);                     // 128
-    int *pdefer = reinterpret_cast<int *>(misc + 64 + 512);              // 128
+    int *pdefer = reinterpret_cast<int *>(misc + 64 + 512);              // 128: 0, CI_DEFER or CI_BAD
     short2 *blk = reinterpret_cast<short2 *>(misc + 64 + 1024);          // <= 528 blocks
     uint32_t *tbad = reinterpret_cast<uint32_t *>(misc + 3200);          // [W] out-of-range samples
+    uint32_t *tinf = tbad + BX_MAXW;                                     // [W] non-finite ones
     uint32_t *umask = reinterpret_cast<uint32_t *>(smem + L::OFF_U);     // [128][W]
     const uint4 *lut = reinterpret_cast<const uint4 *>(smem + L::OFF_LUT);
     uint32_t *nm = reinterpret_cast<uint32_t *>(stages + L::STAGE);      // nmap words (stage 1, mask build only)
@@ -372,7 +374,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     }
     // ---- per-pixel SHP masks over the union samples ----------------
     for (int e = tid; e < BX_M * W; e += BX_THREADS) umask[e] = 0;
-    for (int e = tid; e < W; e += BX_THREADS) tbad[e] = 0;
+    for (int e = tid; e < W; e += BX_THREADS) tbad[e] = tinf[e] = 0;
     for (int e = tid; e < BX_M * nul; e += BX_THREADS) {
         const int m = e / nul, w = e - m * nul;
         const int r = R0 + m / BX_TC, c = C0 + m % BX_TC;
@@ -420,7 +422,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     // first found an out-of-range sample in the tile (clean: it found none)
     bool clean = false;
     auto put = [&](unsigned char *xd, int k0) {
-        bool xbad = false;
+        bool xbad = false, xinf = false;
 #pragma unroll
         for (int q = 0; q < BX_XPT; ++q) {
             const int d = d0 + q * (BX_GRP / KC);
@@ -428,6 +430,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
             float2 x = xv[q];
             if (!clean && (!split_range(x.x) || !split_range(x.y))) {
                 xbad = true;
+                xinf = xinf || !isfinite(x.x) || !isfinite(x.y);
                 x = make_float2(0.f, 0.f);
             }
             // per date pair: Re and Im of the first date, then of the second,
@@ -437,6 +440,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
             xp[KC] = x.y;
         }
         if (xbad) atomicOr(tbad + ((k0 + sidx) >> 5), 1u << ((k0 + sidx) & 31));
+        if (xinf) atomicOr(tinf + ((k0 + sidx) >> 5), 1u << ((k0 + sidx) & 31));
     };
     __syncthreads();
 
@@ -586,13 +590,15 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         fence_after_sync();
         if (pass == 0) {
             // every sample of the tile has been checked and stored: both groups
-            // have passed the barrier above.  A pixel with an out-of-range SHP
-            // sample goes to the FP64 path.
+            // have passed the barrier above
             if (tid < BX_M) {
                 const int m = tid;
-                uint32_t hit = 0;
-                for (int w = 0; w < W; ++w) hit |= umask[m * W + w] & tbad[w];
-                pdefer[m] = hit != 0;
+                uint32_t hit = 0, inf = 0;
+                for (int w = 0; w < W; ++w) {
+                    hit |= umask[m * W + w] & tbad[w];
+                    inf |= umask[m * W + w] & tinf[w];
+                }
+                pdefer[m] = inf ? CI_BAD : hit ? CI_DEFER : 0;
             }
             uint32_t any = 0;
             for (int w = 0; w < W; ++w) any |= tbad[w];
@@ -647,7 +653,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         const int m = tid, info = pinfo[m];
         if (info != CI_SKIP) {
             const long long loc = (long long)(R0 + m / BX_TC) * cols + (C0 + m % BX_TC) - P.cbase;
-            P.cinfo[loc] = (info >= 0 && pdefer[m]) ? CI_DEFER : info;
+            P.cinfo[loc] = (info >= 0 && pdefer[m]) ? pdefer[m] : info;
         }
     }
     __syncthreads();

@@ -68,7 +68,7 @@ struct KParams {
     int *rest;                          // pixels (- cbase) that the register solve hands to pixel_solve
 };
 
-enum { CI_CENTRE = -1, CI_FEW = -2, CI_DEFER = -3 };
+enum { CI_CENTRE = -1, CI_FEW = -2, CI_DEFER = -3, CI_BAD = -4 };
 
 // one launch's share of a batched launch: the Gamma kernel's segment
 // (tiles [tile_offset, next segment's tile_offset)) and the solve and FP64
@@ -2198,6 +2198,10 @@ __device__ int pixel_load_gamma(const KParams &P, long long pp, unsigned char *s
     }
     if (info == CI_DEFER) {
         defer_fp64(P, pp, lane, true);
+        return -1;
+    }
+    if (info == CI_BAD) {
+        put_code(P, pp, lane, (P.semantics != SEM_PL && P.method != M_MLE) ? -6 : -1);
         return -1;
     }
     const float4 *rec4 =

@@ -1,0 +1,44 @@
+"""Samples that are not finite do not take their pixels to the FP64 list: a
+window that holds one has a known outcome."""
+import numpy as np
+import pytest
+
+from fringe_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+RUNS = [dict(method="MLE"), dict(method="EVD"), dict(method="MLE", semantics="phase_link"),
+        dict(method="STBAS", band_width=1), dict(method="STBAS", band_width=4)]
+
+
+def _listed(stack, nmap, half, **kw):
+    from fringe_gb300 import _lib, phase_link
+    ctx = _lib.Context(0)
+    out = phase_link(stack, nmap, half, ctx=ctx, want_status=True, **kw)
+    n = ctx.stats()["fp64_pixels"]
+    ctx.close()
+    return out, n
+
+
+@pytest.mark.parametrize("n", [9, 30, 45])
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+def test_non_finite_samples_are_coded(gpu_lib, n, precision):
+    from fringe_gb300 import _lib, phase_link
+    stack, nmap = synth.scene("voronoi", 41, 53, n, 3, 5, seed=n)
+    hurt = stack.copy()
+    hurt[:, :, :9] = np.nan                           # a border
+    hurt[2, 20, 30] = np.inf
+    hurt[n - 1, 33, 44] = -np.inf * 1j
+    ctx = _lib.Context(0)
+    ctx.set_tuning(force_fp64=True)
+    for kw in RUNS:
+        ref = phase_link(hurt, nmap, (3, 5), ctx=ctx, want_status=True, **kw)
+        assert (ref["status"] < 0).sum() > 400
+        _, clean = _listed(stack, nmap, (3, 5), precision=precision, **kw)
+        got, listed = _listed(hurt, nmap, (3, 5), precision=precision, **kw)
+        assert np.array_equal(got["status"], ref["status"]), kw
+        assert listed <= clean, (kw, listed, clean)
+        off = (ref["status"] != 0) & (ref["status"] != 3)      # 3: solved by EVD
+        assert np.array_equal(got["tcorr"][off], ref["tcorr"][off])
+        assert not got["phase"][:, off].any() and not got["comp"][off].any()
+    ctx.close()

@@ -155,7 +155,18 @@ __global__ void __launch_bounds__(32 * SolveShape<G, NL>::max_warps, 1) k_solve_
     });
 }
 
-// the pixels of entry P that k_solve left: every one, or those of its rest list
+// coherence of a pixel from its samples, in FP32 (out of line: few pixels have
+// samples that the records cannot hold)
+template <int NP>
+__device__ __noinline__ int rest_coherence(const KParams &P, long long pp, unsigned char *sm, int lane)
+{
+    return pixel_coherence<float, NP, RestLay<NP>, RestLay<NP>::cm>(P, pp, sm, lane);
+}
+
+// the pixels of entry P that k_solve left: every one, or those of its rest
+// list.  FP32 form: a pixel with a finite sample outside the range of the bf16 parts
+// has no record; its coherence is formed from the samples as the plain kernel forms it.  (1024^2,
+// N = 30, every 64th row at 1e-17 of the others' amplitude: 437 ms by the FP64 list, 26.5 ms.)
 template <int NP>
 __device__ __forceinline__ void rest_loop(const KParams &P, unsigned char *sm, int lane, const CRowsTmem<NP> &cp)
 {
@@ -163,20 +174,33 @@ __device__ __forceinline__ void rest_loop(const KParams &P, unsigned char *sm, i
     const bool listed = tile_kind(P) != TK_REST;
     const long long cnt = listed ? *((volatile int *)(P.fb_count + 1)) : P.npix;
     for (long long q = list_first(); q < cnt; q = rest_next(P, lane)) {
-        const long long pp = P.cbase + (listed ? (long long)P.rest[q] : q);
-        if constexpr (NP <= 32) {
-            const int npix = pixel_load_gamma<NP, false>(P, pp, sm, lane, A);
-            float cfro = -1.f;
-            if (npix >= 0 && rows_coherence<NP>(P, pp, A, sm, cp, lane, &cfro))
-                pixel_solve<float, NP>(P, pp, sm, lane, npix, cp, cfro);
+        long long loc = q;
+        bool plain;
+        if (listed) {
+            const int e = P.rest[q];
+            plain = e < 0;
+            loc = plain ? ~e : e;
+        } else {
+            plain = P.parts == 3 && P.cinfo[q] == CI_DEFER;
+        }
+        const long long pp = P.cbase + loc;
+        int npix;
+        float cfro = -1.f;
+        bool go;
+        if (plain) {
+            npix = rest_coherence<NP>(P, pp, sm, lane);
+            go = npix >= 0;
+            if (go) rows_from_smem<NP>(cp, A, lane);
+        } else if constexpr (NP <= 32) {
+            npix = pixel_load_gamma<NP, false>(P, pp, sm, lane, A);
+            go = npix >= 0 && rows_coherence<NP>(P, pp, A, sm, cp, lane, &cfro);
         } else {
             // two rows per lane: normalise in the slab, then copy the rows over
-            const int npix = pixel_load_gamma<NP>(P, pp, sm, lane, A);
-            if (npix >= 0) {
-                rows_from_smem<NP>(cp, A, lane);
-                pixel_solve<float, NP>(P, pp, sm, lane, npix, cp);
-            }
+            npix = pixel_load_gamma<NP>(P, pp, sm, lane, A);
+            go = npix >= 0;
+            if (go) rows_from_smem<NP>(cp, A, lane);
         }
+        if (go) pixel_solve<float, NP>(P, pp, sm, lane, npix, cp, cfro);
         __syncwarp();
     }
 }
@@ -194,7 +218,7 @@ __global__ void __launch_bounds__(32 * rest_max_warps<NP>(), 1) k_rest(const __g
     const uint32_t tbase = tmem_alloc_cta(&tslot, warp, tcols);
     const CRowsTmem<NP> cp{tbase + ((uint32_t)(32 * (warp & 3)) << 16) +
                            (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp};
-    rest_loop<NP>(P, smem + (size_t)warp * Lay<float, NP>::bytes_noc, lane, cp);
+    rest_loop<NP>(P, smem + (size_t)warp * RestLay<NP>::bytes_noc, lane, cp);
     tmem_free_cta(tbase, warp, tcols);
 }
 
@@ -208,7 +232,7 @@ __global__ void __launch_bounds__(32 * rest_max_warps<NP>(), 1) k_rest_batch(con
     const uint32_t tbase = tmem_alloc_cta(&tslot, warp, tcols);
     const CRowsTmem<NP> cp{tbase + ((uint32_t)(32 * (warp & 3)) << 16) +
                            (uint32_t)(warp >> 2) * CRowsTmem<NP>::kColsPerWarp};
-    for (int e = 0; e < nent; ++e) rest_loop<NP>(ents[e].P, smem + (size_t)warp * Lay<float, NP>::bytes_noc, lane, cp);
+    for (int e = 0; e < nent; ++e) rest_loop<NP>(ents[e].P, smem + (size_t)warp * RestLay<NP>::bytes_noc, lane, cp);
     tmem_free_cta(tbase, warp, tcols);
 }
 
@@ -268,7 +292,7 @@ static cudaError_t launch_rest_t(const KParams &P, int num_sms, cudaStream_t st)
     if (e != cudaSuccess) return e;
     int warps = rest_max_warps<NP>();
     const long long blocks = solve_grid(P.npix, num_sms, &warps);
-    k_rest<NP><<<(unsigned)blocks, warps * 32, solve_smem(Lay<float, NP>::bytes_noc, warps), st>>>(P);
+    k_rest<NP><<<(unsigned)blocks, warps * 32, solve_smem(RestLay<NP>::bytes_noc, warps), st>>>(P);
     return cudaGetLastError();
 }
 
@@ -332,7 +356,7 @@ static cudaError_t launch_solve_batch_t(const BatchEntry *ents, int nent, long l
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int rw = rest_max_warps<NP>();
     const long long rb = solve_grid(total, num_sms, &rw);
-    k_rest_batch<NP><<<(unsigned)rb, rw * 32, solve_smem(Lay<float, NP>::bytes_noc, rw), st>>>(ents, nent);
+    k_rest_batch<NP><<<(unsigned)rb, rw * 32, solve_smem(RestLay<NP>::bytes_noc, rw), st>>>(ents, nent);
     return cudaGetLastError();
 }
 

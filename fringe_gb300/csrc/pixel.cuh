@@ -225,6 +225,15 @@ template <typename T> struct Lay64W {
 template <> struct Lay<double, 64> : Lay64W<double> {};
 template <> struct Lay<ff, 64> : Lay64W<ff> {};
 
+// k_rest holds C in tensor memory at every depth; where it forms a pixel's C
+// from the samples at 64 dates, C and the staging lie as in Lay64W (whose vectors have
+// the same places as Lay<float, 64>'s)
+template <int NP> struct RestLay : Lay<float, NP> {
+    static constexpr size_t cm = Lay<float, NP>::wm;
+};
+template <> struct RestLay<64> : Lay64W<float> {};
+static_assert(RestLay<64>::vv == Lay<float, 64>::vv && RestLay<64>::ph == Lay<float, 64>::ph, "the same vectors");
+
 // while Gamma is summed the staging and the coherence are both live, so they
 // must not overlap; 1/sqrt(P), in the vectors, is formed after the last sample
 static_assert(Lay<double, 64>::xs >= Lay<double, 64>::cm + Lay<double, 64>::mat, "staging overlaps C");
@@ -1465,10 +1474,12 @@ __device__ __forceinline__ void put_code(const KParams &P, long long pp, int lan
     }
 }
 
-// the rest list of a chunk: appended to by the register solve, read by k_rest
-__device__ __forceinline__ void rest_put(const KParams &P, long long pp)
+// the rest list of a chunk: appended to by the register solve, read by k_rest;
+// plain: the pixel has no record (FP32 form), marked by the complement
+__device__ __forceinline__ void rest_put(const KParams &P, long long pp, bool plain = false)
 {
-    P.rest[atomicAdd(P.fb_count + 1, 1)] = int(pp - P.cbase);
+    const int loc = int(pp - P.cbase);
+    P.rest[atomicAdd(P.fb_count + 1, 1)] = plain ? ~loc : loc;
 }
 __device__ __forceinline__ long long rest_next(const KParams &P, int lane) { return list_next(P.fb_count + 13, lane); }
 
@@ -1546,10 +1557,10 @@ __device__ bool gamma_to_coherence(const KParams &P, long long pp, C2<T> *Cm, un
     return true;
 }
 
-template <typename T, int NP>
+// L: the slab; CM: where C is formed in it
+template <typename T, int NP, typename L = Lay<T, NP>, size_t CM = CmOffset<T, NP>::value>
 __device__ int pixel_coherence(const KParams &P, long long pp, unsigned char *sm, int lane)
 {
-    using L = Lay<T, NP>;
     constexpr int LD = L::LD;
     constexpr int XS = L::XS;
     constexpr int BR = BlockShape<T, NP>::BR, BC = BlockShape<T, NP>::BC;
@@ -1559,7 +1570,7 @@ __device__ int pixel_coherence(const KParams &P, long long pp, unsigned char *sm
     constexpr int PASSES = (NBLK + 31) / 32;
 
     static_assert(!CRowsTmemF<T, NP>::value || PASSES == 1, "C over the staging needs Gamma in registers");
-    C2<T> *Cm = reinterpret_cast<C2<T> *>(sm + CmOffset<T, NP>::value);
+    C2<T> *Cm = reinterpret_cast<C2<T> *>(sm + CM);
     float2 *Xs = reinterpret_cast<float2 *>(sm + L::xs);
 
     const int n = P.nb;

@@ -481,7 +481,10 @@ __device__ __forceinline__ int tile_begin(const KParams &P, long long pp, const 
         const int info = P.cinfo[loc];
         if (info < 0) {
             tile_zero<G>(P, pp, L.g);
-            if (info == CI_DEFER) defer_fp64(P, pp, L.g, true);
+            if (info == CI_DEFER) {
+                if (P.parts == 2) defer_fp64(P, pp, L.g, true);
+                else if (L.g == 0) rest_put(P, pp, true);
+            }
             else if (info == CI_BAD) put_code(P, pp, L.g, MLE ? -1 : -6);
             else if (P.status && L.g == 0) P.status[pp] = (info == CI_CENTRE) ? 1 : 2;
             state = TILE_DONE;

@@ -1,9 +1,13 @@
-"""Samples that are not finite do not take their pixels to the FP64 list: a
-window that holds one has a known outcome."""
+"""Samples that are not finite, or lie outside the range of the bf16 parts, do
+not take their pixels to the FP64 list where FP32 settles them: a window with a non-finite
+sample has a known outcome, and the FP32 form solves windows of very small or large
+samples in FP32."""
 import numpy as np
 import pytest
 
+import oracle
 from fringe_gb300 import synth
+from tests.parity import assert_parity, compare
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +46,22 @@ def test_non_finite_samples_are_coded(gpu_lib, n, precision):
         assert np.array_equal(got["tcorr"][off], ref["tcorr"][off])
         assert not got["phase"][:, off].any() and not got["comp"][off].any()
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [5, 16, 30, 45, 64])
+def test_amplitudes_outside_the_split_stay_in_fp32(gpu_lib, n):
+    """Dates scaled by powers of two that the split cannot hold: the coherence
+    is the unscaled scene's."""
+    stack, nmap = synth.scene("uniform", 37, 43, n, 4, 6, seed=n)
+    scaled = stack.copy()
+    scaled[1] *= np.float32(2.0 ** 52)
+    scaled[n - 2] *= np.float32(2.0 ** -56)
+    for kw in [r for r in RUNS if r.get("band_width", 0) < n - 1]:
+        _, clean = _listed(stack, nmap, (4, 6), precision="fp32", **kw)
+        got, listed = _listed(scaled, nmap, (4, 6), precision="fp32", **kw)
+        assert listed <= clean + stack.shape[1] * stack.shape[2] // 50, (kw, listed, clean)
+        o = oracle.run(scaled, nmap, 4, 6, **kw)
+        got["comp"] = o["comp"]                       # dominated by the scaled date
+        m = compare(got, o)
+        assert m["valid_both"] > 1000, (kw, m)
+        assert_parity(m)

@@ -289,7 +289,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
     BoxBars *bars = reinterpret_cast<BoxBars *>(misc);
     volatile int *dead = &bars->dead;
     int *pinfo = reinterpret_cast<int *>(misc + 64);                     // 128
-    int *pdefer = reinterpret_cast<int *>(misc + 64 + 512);              // 128: 0, CI_DEFER or CI_BAD
+    int *pdefer = reinterpret_cast<int *>(misc + 64 + 512);              // 128: 0, CI_DEFER or CI_BAD (tiles that are not clean)
     short2 *blk = reinterpret_cast<short2 *>(misc + 64 + 1024);          // <= 528 blocks
     uint32_t *tbad = reinterpret_cast<uint32_t *>(misc + 3200);          // [W] out-of-range samples
     uint32_t *tinf = tbad + BX_MAXW;                                     // [W] non-finite ones
@@ -591,19 +591,21 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         if (pass == 0) {
             // every sample of the tile has been checked and stored: both groups
             // have passed the barrier above
-            if (tid < BX_M) {
-                const int m = tid;
-                uint32_t hit = 0, inf = 0;
-                for (int w = 0; w < W; ++w) {
-                    hit |= umask[m * W + w] & tbad[w];
-                    inf |= umask[m * W + w] & tinf[w];
-                }
-                pdefer[m] = inf ? CI_BAD : hit ? CI_DEFER : 0;
-            }
             uint32_t any = 0;
             for (int w = 0; w < W; ++w) any |= tbad[w];
             clean = any == 0;
-            __syncthreads();
+            if (!clean) {
+                if (tid < BX_M) {
+                    const int m = tid;
+                    uint32_t hit = 0, inf = 0;
+                    for (int w = 0; w < W; ++w) {
+                        hit |= umask[m * W + w] & tbad[w];
+                        inf |= umask[m * W + w] & tinf[w];
+                    }
+                    pdefer[m] = inf ? CI_BAD : hit ? CI_DEFER : 0;
+                }
+                __syncthreads();
+            }
         }
         // ---- epilogue: warp w reads TMEM lanes 32(w%4).., every fourth 32 columns ----
         // A lane holds its own pixel's columns; they are written out through
@@ -635,7 +637,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
                 for (int i = 0; i < 8; ++i) {
                     const int pl = 4 * i + (lane >> 3);          // pixel of the warp's 32
                     const int m = 32 * q + pl;
-                    if (j < lim && pinfo[m] >= 0 && !pdefer[m]) {
+                    if (j < lim && pinfo[m] >= 0 && (clean || !pdefer[m])) {
                         const long long loc = (long long)(R0 + m / BX_TC) * cols + (C0 + m % BX_TC) - P.cbase;
                         *reinterpret_cast<float4 *>(rec + loc * P.cstride + cb + col0 + j) =
                             *reinterpret_cast<const float4 *>(stg + pl * SROW + j);
@@ -653,7 +655,7 @@ __device__ __forceinline__ void box_tile(const KParams &P, long long t, unsigned
         const int m = tid, info = pinfo[m];
         if (info != CI_SKIP) {
             const long long loc = (long long)(R0 + m / BX_TC) * cols + (C0 + m % BX_TC) - P.cbase;
-            P.cinfo[loc] = (info >= 0 && pdefer[m]) ? pdefer[m] : info;
+            P.cinfo[loc] = (info >= 0 && !clean && pdefer[m]) ? pdefer[m] : info;
         }
     }
     __syncthreads();

@@ -225,7 +225,7 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out)
 static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                             void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
                             bool fp64_all, void *counters, bool count_run, int stages, long long list_cap,
-                            bool capturing);
+                            bool capturing, int grid0);
 
 // Rows of records that a run over `span` rows of the job takes at a time: 2^20
 // pixels at most, and in the FP32 form no more bytes than the context's limit.
@@ -250,7 +250,7 @@ static int record_rows(const fpl_ctx *ctx, const fpl_job *job, int rec, int span
 // work list and records (grown with cudaMalloc when too small) and d_small.
 int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                 void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
-                bool fp64_all, void *counters, bool count_run, int stages, long long list_cap)
+                bool fp64_all, void *counters, bool count_run, int stages, long long list_cap, int grid0)
 {
     if (!counters) counters = ctx->d_small;
     // runs sharing this context share its scratch: a run waits for the
@@ -261,7 +261,7 @@ int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint3
     const bool order = (cap == cudaStreamCaptureStatusNone);
     if (order && ctx->last_used) FPL_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_last, 0));
     int rc_ = fpl_enqueue_body(ctx, job, stack, nmap, phase, tcorr, comp, status, st, fp64_all, counters,
-                               count_run, stages, list_cap, !order);
+                               count_run, stages, list_cap, !order, grid0);
     if (rc_) return rc_;
     if (order) {
         FPL_CUDA(ctx, cudaEventRecord(ctx->ev_last, st));
@@ -273,7 +273,7 @@ int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint3
 static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                             void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
                             bool fp64_all, void *counters, bool count_run, int stages, long long list_cap,
-                            bool capturing)
+                            bool capturing, int grid0)
 {
     const int r0 = job->row_begin, r1 = job->row_end <= 0 ? job->rows : job->row_end;
     int rc = 0;
@@ -296,6 +296,7 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
     P.plane = (long long)job->rows * job->cols;
     P.pix_begin = (long long)r0 * job->cols;
     P.npix = (long long)(r1 - r0) * job->cols;
+    P.grid0 = grid0;
     P.method = job->method;
     P.semantics = job->semantics;
     P.mini = job->mini_stack_count;
@@ -375,7 +376,7 @@ static int fpl_enqueue_body(fpl_ctx *ctx, const fpl_job *job, const void *stack,
         for (int ra = r0, rb; ra < r1; ra = rb) {
             // several chunks end on the tile grid, so that no tile is computed twice
             const bool grid = rows_per_chunk >= 8 && rows_per_chunk < r1 - r0;
-            rb = std::min(r1, (grid ? ra / 8 * 8 : ra) + rows_per_chunk);
+            rb = std::min(r1, (grid ? (ra + grid0) / 8 * 8 - grid0 : ra) + rows_per_chunk);
             KParams Q = P;
             Q.pix_begin = (long long)ra * P.cols;
             Q.npix = (long long)(rb - ra) * P.cols;
@@ -462,12 +463,15 @@ constexpr int kScatterThreads = 8;
 // computed on the context's stream once they have arrived, and its outputs
 // come back on a third stream while the next chunk computes.  Each chunk has
 // its own block of counters so the statistics add up over the run.
-int fpl_run(fpl_ctx *ctx, const fpl_job *job)
+int fpl_run(fpl_ctx *ctx, const fpl_job *job) { return fpl_run_at(ctx, job, 0); }
+
+int fpl_run_at(fpl_ctx *ctx, const fpl_job *job, int row0)
 {
     return fpl_guard([&]() -> int {
         if (!ctx) return FPL_ERR_NULL;
         int rc = fpl_validate_job(job);
         if (rc) return rc;
+        const int grid0 = row0 % 8;
         auto t0 = std::chrono::steady_clock::now();
         FPL_CUDA(ctx, cudaSetDevice(ctx->device));
         cudaStream_t st = ctx->stream;
@@ -481,7 +485,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
         if (job->memory == FPL_MEM_DEVICE) {
             FPL_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
             rc = fpl_enqueue(ctx, job, job->stack, job->nmap, job->phase, job->tcorr, job->comp, job->status, st,
-                             ctx->force_fp64, ctx->d_small, true);
+                             ctx->force_fp64, ctx->d_small, true, ENQ_ALL, 0, grid0);
             if (rc) return rc;
             FPL_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
         } else {
@@ -528,7 +532,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
                 nchunks = std::max(nchunks, 1);
                 if (span <= 0) cb[1] = r1;
             }
-            int copied = std::max(0, r0 / 8 * 8 - ny);     // first stack row on the device
+            int copied = std::max(0, (r0 + grid0) / 8 * 8 - grid0 - ny);     // first stack row on the device
             // One work list for the whole run: the chunks append to it and its
             // FP64 settle runs once, after the last chunk (a settle per chunk
             // costs a round of the slow FP64 pixels each time); the settled
@@ -540,7 +544,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
                 const int a = cb[c], b = cb[c + 1];
                 if (b <= a) continue;
                 // stack rows every computed pixel's window (and the chunk's tiles) read
-                const int need = std::min(rows, (b + 7) / 8 * 8 + ny);
+                const int need = std::min(rows, (b + grid0 + 7) / 8 * 8 - grid0 + ny);
                 if (need > copied) {
                     const size_t off = (size_t)copied * cols * 8;
                     FPL_CUDA(ctx, cudaMemcpy2DAsync(d_stack + off, plane * 8, h_stack + off, plane * 8,
@@ -557,7 +561,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
                 cj.row_begin = a;
                 cj.row_end = b;
                 rc = fpl_enqueue(ctx, &cj, d_stack, d_nmap, d_phase, d_tcorr, d_comp, d_status, st, ctx->force_fp64,
-                                 ctx->d_small, first, ENQ_KERNELS | (first ? ENQ_RESET : 0), run_px);
+                                 ctx->d_small, first, ENQ_KERNELS | (first ? ENQ_RESET : 0), run_px, grid0);
                 if (rc) return rc;
                 first = false;
                 FPL_CUDA(ctx, cudaEventRecord(ev_done, st));
@@ -576,7 +580,7 @@ int fpl_run(fpl_ctx *ctx, const fpl_job *job)
             // the FP64 settle of every chunk's list, on the whole range (an empty
             // range only clears the counters)
             rc = fpl_enqueue(ctx, job, d_stack, d_nmap, d_phase, d_tcorr, d_comp, d_status, st, ctx->force_fp64,
-                             ctx->d_small, false, first ? ENQ_RESET : ENQ_SETTLE, run_px);
+                             ctx->d_small, false, first ? ENQ_RESET : ENQ_SETTLE, run_px, grid0);
             if (rc) return rc;
             FPL_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
             int head[16];

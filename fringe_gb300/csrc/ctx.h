@@ -100,8 +100,12 @@ enum { ENQ_KERNELS = 1, ENQ_SETTLE = 2, ENQ_RESET = 4, ENQ_ALL = 7 };
 // context's first block); count_run: count it as a run for the profiler;
 // list_cap: entries of the work list (0: the pixels of the row range; a
 // run enqueued as several row ranges with one settle at the end passes the
-// pixels of the whole run).
+// pixels of the whole run); grid0: row 0 of the buffers is a row r of its scene with
+// r % 8 == grid0.
 int fpl_enqueue(fpl_ctx *ctx, const fpl_job *job, const void *stack, const uint32_t *nmap,
                 void *phase, float *tcorr, void *comp, int32_t *status, cudaStream_t st,
                 bool fp64_all, void *counters = nullptr, bool count_run = true, int stages = ENQ_ALL,
-                long long list_cap = 0);
+                long long list_cap = 0, int grid0 = 0);
+// fpl_run for rows cut from a scene (row 0 of the job is row row0 of it): on the scene's
+// tile grid, so that a pixel's results are the same bits however the scene is cut.
+extern "C" int fpl_run_at(fpl_ctx *ctx, const fpl_job *job, int row0);

@@ -266,15 +266,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *mbar)
 }
 
 // tiles of the rows [ra, rb) of a launch: 8-row tiles on the absolute grid
-// (rows 8t .. 8t+7 of the scene) so that a pixel's Gamma, and its order of
-// accumulation, do not depend on how the rows were split into launches
-__device__ __forceinline__ int box_first_row(const KParams &P) { return int(P.pix_begin / P.cols) / BX_TR * BX_TR; }
+// (rows 8t .. 8t+7 of the scene, whose first row is row -grid0 of the array) so that a pixel's
+// Gamma, and its order of accumulation, do not depend on how the rows were split into
+// launches or the scene into arrays
+__host__ __device__ __forceinline__ int box_first_row(const KParams &P)
+{
+    return (int(P.pix_begin / P.cols) + P.grid0) / BX_TR * BX_TR - P.grid0;
+}
 __host__ __device__ __forceinline__ long long box_tiles(const KParams &P)
 {
     const int ra = int(P.pix_begin / P.cols), rb = ra + int(P.npix / P.cols);
     if (rb <= ra) return 0;
-    const int r0 = ra / BX_TR * BX_TR;
-    return (long long)((P.cols + BX_TC - 1) / BX_TC) * ((rb - r0 + BX_TR - 1) / BX_TR);
+    return (long long)((P.cols + BX_TC - 1) / BX_TC) * ((rb - box_first_row(P) + BX_TR - 1) / BX_TR);
 }
 
 // Gamma records of tile t of the launch described by P (all threads of the

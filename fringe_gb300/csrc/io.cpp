@@ -13,8 +13,8 @@
 // CFloat32 file per date named <date>.slc, tcorr.bin (Float32) and the
 // compressed SLC (CFloat32), each with a "<name>.hdr" header.
 // Rows are processed in blocks with the reference's block / halo logic
-// (src/evd/evd.cpp:169-187,399-443,861-870); each block runs on the GPU via
-// fpl_run.  Return codes are the reference's (101-121).
+// (src/evd/evd.cpp:169-187,399-443,861-870); each block runs on the GPU on
+// the file's tile grid (fpl_run_at), so its size does not change the results.  Return codes are the reference's (101-121).
 #include <sys/stat.h>
 #include <sys/types.h>
 
@@ -29,6 +29,7 @@
 #include <string>
 #include <vector>
 
+#include "ctx.h"
 #include "fringe_gb300.h"
 #include "guard.h"
 
@@ -622,7 +623,7 @@ int fpl_process(const fpl_options *opts)
             job.tcorr = tcorr.data();
             job.comp = compv.data();
             if (linestowrite > 0) {
-                rc = fpl_run(ctx, &job);
+                rc = fpl_run_at(ctx, &job, yoff);
                 if (rc) return rc;
                 const size_t off = (size_t)firstlinetowrite * cols;
                 for (int b = 0; b < nbands; ++b)

@@ -65,6 +65,7 @@ struct KParams {
     int *cinfo;                         // [pixel - cbase]: SHP count, or CI_* below
     long long cbase;                    // first pixel of the buffers
     int cstride;                        // floats per record
+    int grid0;                          // the Gamma kernel's tiles start at rows r with (r + grid0) % 8 == 0
     int *rest;                          // pixels (- cbase) that the register solve hands to pixel_solve
 };
 

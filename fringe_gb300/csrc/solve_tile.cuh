@@ -1049,7 +1049,7 @@ __device__ __forceinline__ int tile_evd(const KParams &P, long long pp, const Ti
     float z0r = lo2(vr), z1r = hi2(vr), z0i = lo2(vi), z1i = hi2(vi);
     if (L.g >= dp) z0r = z1r = z0i = z1i = 0.f;
     if (__any_sync(0xffffffffu, slow)) {
-        if (slow && L.g == 0) atomicAdd(P.slow, 1);
+        const bool left = slow;
         const int tp = G == 32 ? dp : max(__shfl_sync(0xffffffffu, dp, 0), __shfl_sync(0xffffffffu, dp, 16));
         // mu above rho by three times the estimate r^2 / gap of lambda_max - rho,
         // at most by the residual; the gap from the contraction, dl (1 / c - 1)
@@ -1117,6 +1117,8 @@ __device__ __forceinline__ int tile_evd(const KParams &P, long long pp, const Ti
             }
         }
         if (state == TILE_RUN && (slow || hard)) state = TILE_GENERAL;
+        // (pixel_solve counts those that it takes over)
+        if (left && state == TILE_RUN && L.g == 0) atomicAdd(P.slow, 1);
     }
     tile_finish<G, NL>(P, pp, L, taddr, state == TILE_RUN, P.method == M_STBAS, z0r, z1r, z0i, z1i, own);
     return state == TILE_RUN ? (int)TILE_DONE : state;

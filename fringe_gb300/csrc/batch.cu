@@ -630,7 +630,10 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
             cudaEventCreate(&e1);
             // one untimed run first: the candidates' times then exclude one-time
             // costs (module loading, kernel attributes, first-touch of buffers)
-            if (batch_enqueue(b, b->cap_stream) != FPL_OK || cudaStreamSynchronize(b->cap_stream) != cudaSuccess) {
+            bool any = !b->classes.empty();
+            for (const MixedWave &w : b->waves) any = any || w.ent_count[0] || w.ent_count[1] || w.ent_count[2];
+            if (any && (batch_enqueue(b, b->cap_stream) != FPL_OK ||
+                        cudaStreamSynchronize(b->cap_stream) != cudaSuccess)) {
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
                 cudaFree(d_sum);
@@ -677,16 +680,23 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                 k.warps = best_w;
                 ctx->tuned_warps[key] = best_w;
             }
-            // mixed form: warps per CTA of the solve launches of each padded depth,
-            // keyed like the FP32 classes with a bit for the form
+            // Combined solve launches: warps per CTA of each padded depth, keyed like the
+            // plain classes with the kinds of methods and a bit of their own.  Pieces
+            // with launches of their own take no shape from here.
             for (int c = 0; c < 3; ++c) {
-                if (!b->m64_count[c]) continue;
+                std::vector<fpl::BatchEntry> pcs;
+                int kinds = 0;
+                for (const MixedWave &w : b->waves) {
+                    const size_t at = pcs.size();
+                    pcs.resize(at + w.ent_count[c]);
+                    kinds |= w.ent_kinds[c];
+                    cudaMemcpy(pcs.data() + at, b->d_ments + w.ent_first[c], sizeof(fpl::BatchEntry) * w.ent_count[c],
+                               cudaMemcpyDeviceToHost);
+                }
+                if (pcs.empty()) continue;
                 const int np = 16 << c;
                 unsigned long long shp = 0, px = 0;
                 int taps = 0;
-                std::vector<fpl::BatchEntry> pcs(b->m64_count[c]);
-                cudaMemcpy(pcs.data(), b->d_m64 + b->m64_first[c], sizeof(fpl::BatchEntry) * pcs.size(),
-                           cudaMemcpyDeviceToHost);
                 for (const fpl::BatchEntry &en : pcs) {
                     const fpl::KParams &P = en.P;
                     taps = std::max(taps, P.K);
@@ -699,7 +709,7 @@ int fpl_batch_create(fpl_ctx *ctx, const fpl_job *jobs, int njobs, int flags, fp
                     shp += sum;
                     px += (unsigned long long)P.npix;
                 }
-                const long long key = (1ll << 62) | ((long long)np << 40) | ((long long)taps << 16) |
+                const long long key = (1ll << 62) | ((long long)kinds << 50) | ((long long)np << 40) | ((long long)taps << 16) |
                                       (long long)(px ? shp / px / 16 : 0);
                 auto it = ctx->tuned_warps.find(key);
                 if (it != ctx->tuned_warps.end()) {

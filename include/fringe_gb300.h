@@ -163,8 +163,9 @@ int fpl_last_stats(const fpl_ctx *ctx, fpl_stats *out);
  * loop).  FPL_BATCH_GRAPH captures the launch sequence into a CUDA graph at
  * creation; fpl_batch_run replays it (buffers are fixed, their contents may
  * change between runs).  FPL_BATCH_AUTOTUNE times candidate CTA shapes on
- * the batch at creation and caches the fastest per (form, depth, window,
- * mean SHP count) in the context.  Jobs are cut into row pieces, packed into
+ * the batch at creation and caches the fastest per (kinds of methods, depth, window,
+ * mean SHP count) in the context (pieces of 65,536 pixels and more, whose launches are
+ * their own, have one shape).  Jobs are cut into row pieces, packed into
  * waves of <= 2^20 pixels (fewer where device memory is short), with one
  * tensor-core Gamma launch over the tiles and one solve launch per padded depth
  * and kind of method over the pixels of each wave.  Jobs whose window the Gamma

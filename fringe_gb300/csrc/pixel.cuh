@@ -2169,20 +2169,6 @@ __device__ bool pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
 }
 
 
-// Mixed form: pulls the Gamma record and tile information of pixel pp of P
-// into L2 (one 128-byte line per lane), so the load of the next pixel of a
-// warp finds them there.
-__device__ __forceinline__ void prefetch_record(const KParams &P, long long pp, int lane)
-{
-    const long long loc = pp - P.cbase;
-    const char *rec = reinterpret_cast<const char *>(P.cbuf) + loc * (long long)P.cstride * 4;
-    const uintptr_t lo = reinterpret_cast<uintptr_t>(rec) & ~uintptr_t(127);
-    const uintptr_t hi = reinterpret_cast<uintptr_t>(rec) + (size_t)P.cstride * 4;
-    for (uintptr_t a = lo + 128u * (unsigned)lane; a < hi; a += 32u * 128u)
-        asm volatile("prefetch.L2 [%0];" :: "l"(a));
-    if (lane == 31) asm volatile("prefetch.L2 [%0];" :: "l"(P.cinfo + loc));
-}
-
 // Mixed form: Gamma of pixel pp was accumulated on the tensor cores
 // (gram_box.cu) into a record of P.cstride floats; load it into the shared-
 // memory matrix Cm of the warp and normalise it to coherence.  Record layout: dates padded to an even

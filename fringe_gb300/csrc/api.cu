@@ -659,7 +659,7 @@ int fpl_run_at(fpl_ctx *ctx, const fpl_job *job, int row0)
         const unsigned err = static_cast<unsigned>(small[4]);
         ctx->stats.pixels = (long long)(r1 - r0) * cols;
         ctx->stats.fp64_pixels = ctx->force_fp64 ? ctx->stats.pixels : fp64;
-        ctx->stats.mixed_fp64_inverse = 0;
+        ctx->stats.mixed_fp64_inverse = small[9];
         ctx->stats.slow_path_pixels = slow;
         ctx->stats.kernel_ms = ms;
         ctx->stats.total_ms =

@@ -781,6 +781,7 @@ int fpl_batch_stats(const fpl_batch *b, fpl_stats *out)
             out->fp64_pixels += c[(kJobCounterBytes / sizeof(int)) * e];
             err |= (unsigned)c[(kJobCounterBytes / sizeof(int)) * e + 4];
             out->slow_path_pixels += c[(kJobCounterBytes / sizeof(int)) * e + 8];
+            out->mixed_fp64_inverse += c[(kJobCounterBytes / sizeof(int)) * e + 9];
         }
         return err ? FPL_ERR_DEVICE_CHECK : FPL_OK;
     });

@@ -53,12 +53,13 @@ struct KParams {
     float cond_max;                     // largest inf-norm condition of |C| inverted in FP32
     float shift, shift_backoff;         // inverse-iteration shifts, in units of min(1, rho)
     int *fb_count;                      // FP64 work list (scratch): the 64-byte counter block of the
-                                        // run: +0 list length, +16 err, +32 slow, +48 work cursor;
+                                        // run: +0 list length, +16 err, +32 slow, +36 entries left to FP64, +48 work cursor;
                                         // of the chunk: +4 rest list length, +52 its work cursor
     long long *fb_list;
     int fb_cap;
     unsigned *err;                      // error flags (scratch)
-    int *slow;                          // pixels that left the fast eigen path (scratch)
+    int *slow;                          // pixels that left the fast eigen path (scratch); next to it: list
+                                        // entries that went on to FP64
     // Gamma records from the tensor-core kernel
     int parts;                          // bf16 parts per product: 2 mixed form, 3 FP32 form
     float2 *cbuf;                       // [pixel - cbase][cstride floats] (pixel_load_gamma)
@@ -2366,6 +2367,7 @@ __device__ __forceinline__ void settle_pixel(const KParams &P, long long entry, 
 {
     const long long pp = entry < 0 ? ~entry : entry;
     if (entry >= 0 && process_pixel<ff, NP>(P, pp, sm, lane, taddr)) return;
+    if (lane == 0) atomicAdd(P.slow + 1, 1);
     __syncwarp();
     fp64_pixel<NP>(P, pp, sm, lane, taddr);
 }

@@ -128,7 +128,7 @@ typedef struct {
 typedef struct {
     long long pixels;            /* pixels in the row range          */
     long long fp64_pixels;       /* pixels FP32 left undecided (settled in float-float or FP64) */
-    long long mixed_fp64_inverse;/* MLE pixels whose |G| inverse ran in FP64 */
+    long long mixed_fp64_inverse;/* of those, pixels that float-float left to FP64 */
     long long slow_path_pixels;  /* pixels that left the fast eigen path (second shift or Householder) */
     float kernel_ms;             /* device time of the compute kernels */
     float total_ms;              /* wall time of the call             */

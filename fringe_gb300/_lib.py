@@ -220,7 +220,7 @@ class Context:
     def profile_kernels(self):
         """Per-kernel milliseconds of the runs read by the last profile():
         {"fp32": plain pixel kernel, "gram": tensor-core Gamma, "solve":
-        eigen-solves of the mixed form, "fp64": undecided pixels}."""
+        eigen-solves from the records, "fp64": undecided pixels}."""
         ms = (ctypes.c_double * 4)()
         check(load().fpl_ctx_profile_kernels(self.handle, ms, 4), self.handle)
         return dict(zip(("fp32", "gram", "solve", "fp64"), list(ms)))

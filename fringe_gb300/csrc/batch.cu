@@ -265,7 +265,7 @@ struct BatchClass {
     int warps = 0;                  // CTA shape
 };
 
-// one wave of the mixed-form pieces: its Gamma segments and its solve
+// one wave of pieces: its Gamma segments and its solve
 // entries per padded depth (16/32/64)
 struct MixedWave {
     int seg_first = 0, seg_count = 0;
@@ -280,14 +280,14 @@ struct MixedWave {
 struct fpl_batch {
     fpl_ctx *ctx = nullptr;
     int njobs = 0;
-    int nent = 0;                    // counter blocks: FP32 jobs, then mixed pieces
+    int nent = 0;                    // counter blocks: plain jobs, then pieces
     std::vector<MixedWave> waves;
-    fpl::BoxSeg *d_segs = nullptr;   // mixed: Gamma segments of every wave
-    fpl::BatchEntry *d_ments = nullptr;   // mixed: solve entries of every wave
-    fpl::BatchEntry *d_m64 = nullptr;     // mixed: every piece, by padded depth (FP64 settle)
+    fpl::BoxSeg *d_segs = nullptr;   // Gamma segments of every wave
+    fpl::BatchEntry *d_ments = nullptr;   // solve entries of every wave
+    fpl::BatchEntry *d_m64 = nullptr;     // every piece, by padded depth (FP64 settle)
     int m64_first[3] = {0, 0, 0}, m64_count[3] = {0, 0, 0};
-    int mixed_warps[3] = {0, 0, 0};  // warps per CTA of the mixed solve launches (0: the most that fit)
-    void *d_rec = nullptr;           // mixed: Gamma records, tile infos and rest lists of one wave
+    int mixed_warps[3] = {0, 0, 0};  // warps per CTA of the combined solve launches (0: the most that fit)
+    void *d_rec = nullptr;           // Gamma records, tile infos and rest lists of one wave
     std::vector<BatchClass> classes;
     fpl::BatchEntry *d_table = nullptr;
     void *d_scratch = nullptr;       // per-job counters, work counters, FP64 lists

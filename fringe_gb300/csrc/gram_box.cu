@@ -41,8 +41,9 @@
 // [2^-50, 2^50] in magnitude (other than 0), are outside the range of the
 // split and zeroed in the tile.  A pixel with a non-finite one among its SHPs has
 // a non-finite power at that date, so its outcome is known: the failure code
-// of the first eigen call (CI_BAD).  A pixel with a finite one is handed to the FP64 path
-// (CI_DEFER), which follows the reference exactly.  Every wait on the tensor core is bounded; on timeout the CTA
+// of the first eigen call (CI_BAD).  A pixel with a finite one is marked CI_DEFER: the
+// mixed form settles it in FP64, the FP32 form from its samples in k_rest.  Every wait on the tensor
+// core is bounded; on timeout the CTA
 // records an error flag, stops, and frees its tensor memory after a second
 // bounded wait.
 #include <cuda_bf16.h>

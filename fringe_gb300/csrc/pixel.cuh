@@ -247,7 +247,7 @@ template <typename T, int NP> struct CInTmem {
 };
 
 // The plain FP32 form at <= 32 dates keeps C in tensor memory as well (rows
-// as CRowsTmem, as the mixed form's solve does), which halves the slab and
+// as CRowsTmem, as k_rest does), which halves the slab and
 // raises the warps per SM: Gamma is accumulated in registers in one pass,
 // so C is formed over the gather staging (no longer read by then) and moved
 // to tensor memory before the solve reuses that memory.
@@ -2170,7 +2170,7 @@ __device__ bool pixel_solve(const KParams &P, long long pp, unsigned char *sm, i
 }
 
 
-// Mixed form: Gamma of pixel pp was accumulated on the tensor cores
+// Gamma of pixel pp was accumulated on the tensor cores
 // (gram_box.cu) into a record of P.cstride floats; load it into the shared-
 // memory matrix Cm of the warp and normalise it to coherence.  Record layout: dates padded to an even
 // count and grouped in pairs; block (a, b), a <= b < DP, row-major over the

@@ -4,7 +4,7 @@ Pixels are independent given their windows, so a scene splits into bands of
 rows with no data-path collective: rank k computes rows [r0, r1) from the
 stack rows [s0, s1), its band plus an apron of at least Ny rows on each side
 (the reference's block overlap, src/evd/evd.cpp:419-443).  s0 is rounded
-down to the 8-row tile grid of the mixed form, so a band's results are the
+down to the 8-row tile grid of the Gamma kernel, so a band's results are the
 same bits as the whole scene's rows.  Gathering the bands (if a caller wants
 one array) is the caller's business: the outputs of the ranks are disjoint.
 """
